@@ -102,7 +102,7 @@ struct ewg_context {
   cudaEvent_t fork = nullptr, join = nullptr;
   DevBuf buf[B_COUNT];
   std::map<int, FftEntry> ffts;
-  std::map<std::tuple<int, int, int>, CorrEntry> corrs;
+  std::map<std::tuple<int, int, int>, CorrEntry> corrs;  // (n, H, half-width or -1)
   long long launches = 0;
   ewg_params last{};
   // TCoulomb state
@@ -117,6 +117,7 @@ struct ewg_context {
     int nb[3] = {0, 0, 0};
     int ng[3] = {0, 0, 0};
     int m = -1;
+    int kb = -1;
     int mixed = -1;
     int ad = -1;
   } resident;
@@ -272,17 +273,23 @@ int get_fft(ewg_context* c, int n, FftPlan& out, int sched = 1) {
   return EWG_OK;
 }
 
-// Squared deconvolution factors f(k)^2, f(k) = exp(b (pi k / n)^2)
-// (nfft/nfft.f90:163-189), for k in [-H, H].
-int get_corr(ewg_context* c, int n, int H, int m, const double** out) {
-  auto key = std::make_tuple(n, H, m);
+// Squared deconvolution factors f(k)^2 for k in [-H, H]: f(k) = exp(b (pi k / n)^2)
+// for the Gaussian (nfft/nfft.f90:163-189), the inverse of the window's
+// transform at k / n for the Kaiser-Bessel window.
+int get_corr(ewg_context* c, const MeshGeom& g, int d, const double** out) {
+  const int n = g.n[d], H = g.M[d] - g.M[d] / 2;
+  auto key = std::make_tuple(n, H, g.kb ? -1 : g.m);
   auto it = c->corrs.find(key);
   if (it == c->corrs.end()) {
-    const double b = window_shape(m);
     std::vector<double> host(2 * H + 1);
     for (int k = -H; k <= H; ++k) {
-      const double x = kPi * static_cast<double>(k) / static_cast<double>(n);
-      const double f = std::exp(b * (x * x));
+      double f;
+      if (g.kb) {
+        f = 1.0 / kb_transform(static_cast<double>(k) / static_cast<double>(n));
+      } else {
+        const double x = kPi * static_cast<double>(k) / static_cast<double>(n);
+        f = std::exp(g.b * (x * x));
+      }
       host[k + H] = f * f;
     }
     CorrEntry e;
@@ -340,7 +347,7 @@ ewg_kernel_shape resolve_shape(ewg_kernel_shape s) {
 std::array<int, 7> shape_bucket(int precision, int grids, int n, const MeshGeom& g) {
   int oct = 0;
   while (oct < 30 && (2L << oct) <= n) ++oct;
-  return {precision, grids, oct, g.n[0], g.n[1], g.n[2], g.m};
+  return {precision, grids, oct, g.n[0], g.n[1], g.n[2], g.kb ? -g.m : g.m};
 }
 
 ewg_kernel_shape shape_for(const ewg_context* c, const std::array<int, 7>& bucket) {
@@ -349,11 +356,18 @@ ewg_kernel_shape shape_for(const ewg_context* c, const std::array<int, 7>& bucke
   return resolve_shape(it == c->shapes.end() ? ewg_kernel_shape{} : it->second);
 }
 
-int mesh_geometry(const Cell& cell, const ewg_params& p, MeshGeom& g) {
-  for (int d = 0; d < 3; ++d) {
+int mesh_geometry(const Cell& cell, const ewg_params& p, bool mixed, MeshGeom& g) {
+  for (int d = 0; d < 3; ++d)
     if (p.n_modes[d] < 2) return EWG_ERR_ARG;
+  g.kb = mesh_window(cell, p, mixed) ? 1 : 0;
+  for (int d = 0; d < 3; ++d) {
     g.M[d] = p.n_modes[d];
     g.n[d] = kOversampling * p.n_modes[d];
+    if (!g.kb) continue;
+    // The mode counts that are accepted do not depend on the window.
+    FftPlan twice;
+    if (g.n[d] > kMaxFftLength || !factor_length(g.n[d], twice)) return EWG_ERR_GRID_TOO_LARGE;
+    g.n[d] = kb_length(p.n_modes[d]);
   }
   if (p.window_cutoff < 0) return EWG_ERR_ARG;
   // Closed box |k| <= H covering the mode set S = [M/2 - M, M/2 - 1] and -S.
@@ -363,7 +377,8 @@ int mesh_geometry(const Cell& cell, const ewg_params& p, MeshGeom& g) {
   g.K2 = 2 * H[1] + 1;
   g.K3 = 2 * H[2] + 1;
   g.m = p.window_cutoff;
-  g.W = 2 * g.m + 1;
+  g.lo = g.kb ? kKbLow : -g.m;
+  g.W = g.kb ? kKbWidth : 2 * g.m + 1;
   g.b = window_shape(g.m);
   g.pref = 1.0 / std::sqrt(kPi * g.b);
   for (int i = 0; i < 3; ++i)
@@ -384,13 +399,13 @@ void stencil_dims(const MeshGeom& g, bool ad, StencilDims& sd) {
     sd.T[d] = T;
     sd.ntiles[d] = nt;
     int most = nt;
-    if (2 * g.m + 1 < n) {
+    if (g.W < n) {
       // Walk each start point's stencil through the tiles, as the weights kernel does.
       most = 1;
       for (int c = 0; c < n; ++c) {
-        const int p0 = ((c - g.m) % n + n) % n;
+        const int p0 = ((c + g.lo) % n + n) % n;
         int t = p0 / T, covered = std::min((t + 1) * T, n) - p0, count = 1;
-        while (covered < 2 * g.m + 1) {
+        while (covered < g.W) {
           t = t + 1 == nt ? 0 : t + 1;
           ++count;
           covered += std::min((t + 1) * T, n) - t * T;
@@ -407,7 +422,9 @@ void stencil_dims(const MeshGeom& g, bool ad, StencilDims& sd) {
   sd.ad = ad ? 1 : 0;
   sd.dwoff = off;
   if (ad) sd.wstride = 2 * off;  // derivative rows follow the weight rows
-  sd.m = g.m;
+  sd.lo = g.lo;
+  sd.W = g.W;
+  sd.kb = g.kb;
   sd.b = g.b;
   sd.pref = g.pref;
 }
@@ -430,7 +447,7 @@ int evaluate(ewg_context* c, int n, const double* pos, long sa, long sd, const d
   const int nc = want_force && !ad ? 4 : 1;
   const int nparts = want_force ? 4 : 1;
   MeshPlan mp;
-  rc = mesh_geometry(cell, p, mp.g);
+  rc = mesh_geometry(cell, p, mixed, mp.g);
   if (rc) return rc;
   const ewg_kernel_shape ks =
       shape_for(c, shape_bucket(c->precision, want_force ? (ad ? 2 : 1) : 0, n, mp.g));
@@ -443,8 +460,7 @@ int evaluate(ewg_context* c, int n, const double* pos, long sa, long sd, const d
   mp.stencil = ks.stencil;
   for (int d = 0; d < 3; ++d) {
     if ((rc = get_fft(c, mp.g.n[d], mp.fft[d], ks.fft_sched))) return rc;
-    const int H = mp.g.M[d] - mp.g.M[d] / 2;
-    if ((rc = get_corr(c, mp.g.n[d], H, mp.g.m, &mp.corr2[d]))) return rc;
+    if ((rc = get_corr(c, mp.g, d, &mp.corr2[d]))) return rc;
   }
   if ((rc = mesh_check_lengths(mp.g, mixed))) return rc;
   stencil_dims(mp.g, ad, mp.sd);
@@ -489,7 +505,8 @@ int evaluate(ewg_context* c, int n, const double* pos, long sa, long sd, const d
                      c->resident.nb[0] == rg.nb[0] && c->resident.nb[1] == rg.nb[1] &&
                      c->resident.nb[2] == rg.nb[2] && c->resident.ng[0] == mp.g.n[0] &&
                      c->resident.ng[1] == mp.g.n[1] && c->resident.ng[2] == mp.g.n[2] &&
-                     c->resident.m == mp.g.m && c->resident.mixed == mixed &&
+                     c->resident.m == mp.g.m && c->resident.kb == mp.g.kb &&
+                     c->resident.mixed == mixed &&
                      c->resident.ad == mp.sd.ad;
   double* p6 = nullptr;
   double* zpart = nullptr;
@@ -618,6 +635,7 @@ int evaluate(ewg_context* c, int n, const double* pos, long sa, long sd, const d
       c->resident.ng[d] = mp.g.n[d];
     }
     c->resident.m = mp.g.m;
+    c->resident.kb = mp.g.kb;
     c->resident.mixed = mixed;
     c->resident.ad = mp.sd.ad;
   }
@@ -730,18 +748,18 @@ int seg_plan(ewg_context* c, int n_cells, const int* offsets, const std::vector<
     bc.cut2 = p.r_cut * p.r_cut;
     bc.pre2 = real_prefilter_bound(bc.rg, p.r_cut);
     bc.self_coef = -2.0 * p.alpha / std::sqrt(kPi);
-    int rc = mesh_geometry(cells[ci], p, bc.g);
+    int rc = mesh_geometry(cells[ci], p, mixed, bc.g);
     if (rc) return rc;
     if ((rc = mesh_check_lengths(bc.g, mixed))) return rc;
     for (int d = 0; d < 3; ++d) {
       FftPlan fp;
       if ((rc = get_fft(c, bc.g.n[d], fp))) return rc;
       bc.fft[d] = fp;
-      const int H = bc.g.M[d] - bc.g.M[d] / 2;
-      if ((rc = get_corr(c, bc.g.n[d], H, bc.g.m, &bc.corr2[d]))) return rc;
+      if ((rc = get_corr(c, bc.g, d, &bc.corr2[d]))) return rc;
       nmax[d] = std::max(nmax[d], bc.g.n[d]);
     }
     stencil_dims(bc.g, ad, bc.sd);
+    (bc.g.kb ? sp.b.any_kb : sp.b.any_gauss) = 1;
     sp.wstride = std::max<size_t>(sp.wstride, bc.sd.wstride);
     sp.pstride = std::max(sp.pstride, bc.sd.pstride);
     if (bc.sd.pstride > 32) lpa = 32;
@@ -811,6 +829,7 @@ int seg_plan(ewg_context* c, int n_cells, const int* offsets, const std::vector<
     for (int ci = 1; ci < n_cells; ++ci) b.uniform[d] &= sp.cells[ci].g.n[d] == sp.cells[0].g.n[d];
     b.plan[d] = sp.cells[0].fft[d];
   }
+  b.wstride = static_cast<int>(sp.wstride);
   for (int d = 0; d < 3; ++d) b.smem[d] = mesh_pass_smem(nmax[d], L, mixed, 0);
   b.smem_z = smz;
   b.n_atoms = pre(SP_ATOMS)[n_cells];
@@ -1143,7 +1162,7 @@ int ewg_device_memory(int n, const double* charges, const double* lat_rows, doub
   Cell cell;
   cell_from_rows(lat_rows, cell);
   MeshGeom g;
-  rc = mesh_geometry(cell, p, g);
+  rc = mesh_geometry(cell, p, precision == EWG_PRECISION_MIXED, g);
   if (rc) return rc;
   // The larger of the two force schemes: i k keeps four transform channels,
   // window derivatives one channel and twice the weight rows.
@@ -1401,7 +1420,7 @@ int tune_shapes(ewg_context* c, int n, const double* dpos, const double* dq, con
                 const ewg_params& p, double* dpot, double* dforce, double shift,
                 ewg_kernel_shape* out, double* ms_out) {
   MeshGeom g;
-  int rc = mesh_geometry(cell, p, g);
+  int rc = mesh_geometry(cell, p, c->precision == EWG_PRECISION_MIXED, g);
   if (rc) return rc;
   const bool want_force = dforce != nullptr;
   const bool ad = want_force && c->force_scheme == EWG_FORCE_AD;
@@ -2119,13 +2138,12 @@ int points_mesh(ewg_context* c, const Cell& cell, double tol, int nt, const doub
   real_geometry(cell, r_pair, ns, rg);
   const bool want_grad = dgrad != nullptr;
   MeshPlan src, tgt;
-  if ((rc = mesh_geometry(cell, p, src.g))) return rc;
+  if ((rc = mesh_geometry(cell, p, false, src.g))) return rc;
   src.mixed = 0;
   src.prof = nullptr;
   for (int d = 0; d < 3; ++d) {
     if ((rc = get_fft(c, src.g.n[d], src.fft[d]))) return rc;
-    const int H = src.g.M[d] - src.g.M[d] / 2;
-    if ((rc = get_corr(c, src.g.n[d], H, src.g.m, &src.corr2[d]))) return rc;
+    if ((rc = get_corr(c, src.g, d, &src.corr2[d]))) return rc;
   }
   if ((rc = mesh_check_lengths(src.g, false))) return rc;
   stencil_dims(src.g, false, src.sd);

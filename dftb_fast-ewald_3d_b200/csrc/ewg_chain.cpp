@@ -117,6 +117,105 @@ double window_shape(int m) {
   return (2.0 * s / (2.0 * s - 1.0)) * (static_cast<double>(m) / kPi);
 }
 
+// ---- Kaiser-Bessel window ---------------------------------------------------
+// The reference's Gaussian at m = 11 or 12 (tolerances of about 1e-9 and 1e-10)
+// spends 23 or 25 points per axis on a twice oversampled grid.  The
+// Kaiser-Bessel window (Kaiser 1974; as an NFFT window: Jackson, Meyer,
+// Nishimura and Macovski 1991; Potts and Steidl 2003) concentrates better: with
+// 14 points on 1.28 points per mode the reciprocal sum of a one-dimensional
+// model with the same mode weights (150 random charges, modes damped to 1e-9 .. 1e-7
+// at the edge of the box as the parameter chain leaves them) is off by
+//   potential   2e-14 .. 7e-14   (Gaussian 1.1e-13 at m = 12, 8e-13 at m = 11)
+//   i k force   4e-14 .. 7e-13   (Gaussian 8e-14, 8e-13)
+//   window-derivative force 7e-12 .. 1e-11   (Gaussian 9e-12, 8e-11)
+// so the results keep the accuracy of the Gaussian's while the grid has 0.26 of
+// its points at best and the stencil 0.18 (m = 12).  beta above pi W (1 - 1/(2 sigma)),
+// the value for unweighted modes, trades error at the edge of the mode box,
+// where the Ewald factor has damped the modes, for error at its centre.
+namespace {
+long double bessel_i0(long double x) {  // power series; x <= beta
+  const long double h = 0.25L * x * x;
+  long double t = 1.0L, s = 1.0L;
+  for (int k = 1; k < 300 && t > 1e-22L * s; ++k) {
+    t *= h / (static_cast<long double>(k) * k);
+    s += t;
+  }
+  return s;
+}
+}  // namespace
+
+void kb_polynomials(double* coef) {
+  constexpr int N = kKbDegree + 1;
+  const long double pi = 3.141592653589793238462643383279502884L;
+  const long double norm = bessel_i0(kKbBeta);
+  for (int j = 0; j < kKbWidth; ++j) {
+    // Chebyshev interpolation of the piece on t in [-1, 1] (error 3e-18 of the
+    // window's peak at degree 15), then its monomial coefficients.
+    long double f[N], c[N], mono[N] = {0.0L}, t0[N] = {0.0L}, t1[N] = {0.0L};
+    for (int i = 0; i < N; ++i) {
+      const long double t = cosl(pi * (i + 0.5L) / N);
+      const long double u = (kKbLow + j) - 0.5L * (t + 1.0L);
+      const long double r = 2.0L * u / kKbWidth;
+      f[i] = bessel_i0(kKbBeta * sqrtl(std::max(0.0L, 1.0L - r * r))) / norm;
+    }
+    for (int k = 0; k < N; ++k) {
+      c[k] = 0.0L;
+      for (int i = 0; i < N; ++i) c[k] += f[i] * cosl(pi * k * (i + 0.5L) / N);
+      c[k] *= (k == 0 ? 1.0L : 2.0L) / N;
+    }
+    t0[0] = 1.0L;  // T_0
+    t1[1] = 1.0L;  // T_1
+    mono[0] = c[0];
+    for (int k = 1; k < N; ++k) {
+      for (int i = 0; i < N; ++i) mono[i] += c[k] * t1[i];
+      long double t2[N];
+      for (int i = 0; i < N; ++i) t2[i] = (i > 0 ? 2.0L * t1[i - 1] : 0.0L) - t0[i];
+      for (int i = 0; i < N; ++i) {
+        t0[i] = t1[i];
+        t1[i] = t2[i];
+      }
+    }
+    for (int k = 0; k < N; ++k) coef[j * N + k] = static_cast<double>(mono[k]);
+  }
+}
+
+double kb_transform(double x) {
+  // Integral of w(u) exp(-2 pi i u x) du; |pi W x| < beta for every retained
+  // mode (|x| <= 1/2.56).
+  const long double y = 3.141592653589793238462643383279502884L * kKbWidth * x;
+  const long double a = sqrtl(static_cast<long double>(kKbBeta) * kKbBeta - y * y);
+  return static_cast<double>(kKbWidth * (sinhl(a) / a) / bessel_i0(kKbBeta));
+}
+
+int kb_length(int modes) {
+  // At least 1.28 points per mode and more points than the window is wide (every
+  // grid point then meets one image of a stencil), in whole tiles of 8: with a
+  // part tile at the end of the axis a stencil would cross four tiles there
+  // instead of three and every per-atom table would grow by a third per axis.
+  int n = std::max((32 * modes + 24) / 25, kKbWidth + 2);
+  for (n = (n + 7) / 8 * 8;; n += 8) {
+    int r = n;
+    for (int p : {2, 3, 5, 7})
+      while (r % p == 0) r /= p;
+    if (r == 1) return n;
+  }
+}
+
+bool mesh_window(const Cell& cell, const ewg_params& p, bool mixed) {
+  // Only where the Gaussian is as accurate as the Kaiser-Bessel window: half-widths
+  // 11 and 12 in the plain form.  Narrower Gaussians are the caller's choice of a
+  // looser result, wider ones of a tighter one, and the mixed form's FP32 weights
+  // keep their values.  The modes at the edge of the box must be damped to
+  // 2e-7 (the chain leaves 1e-10 .. 1e-7): overrides of alpha, k_cut or the modes
+  // that leave them undamped keep the Gaussian, whose error there is smaller.
+  if (mixed || p.window_cutoff < 11 || p.window_cutoff > 12) return false;
+  for (int d = 0; d < 3; ++d) {
+    const double edge = kPi * p.n_modes[d] / cell.latLen[d];
+    if (!(std::exp(-edge * edge / (4.0 * p.alpha * p.alpha)) <= 2.0e-7)) return false;
+  }
+  return true;
+}
+
 int box_count(double r_cut, double recLen) { return floor_int(1.0 / (r_cut * recLen)); }
 
 int choose_parameters(const Cell& cell, double q2sum, int n, double tol, const ewg_overrides* ov,

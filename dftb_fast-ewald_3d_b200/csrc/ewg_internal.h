@@ -44,6 +44,22 @@ int choose_parameters(const Cell& cell, double q2sum, int n, double tol, const e
 double grid_memory_gigabytes(const ewg_params& p);
 int next_fast_length(int n);      // nfft/fft_backend.f90:73-91
 double window_shape(int m);       // nfft/nfft.f90:82-92
+
+// The Kaiser-Bessel window that stands in for the reference's Gaussian in the
+// plain form (see mesh_window in ewg_chain.cpp for the rule and the errors):
+// w(u) = I0(beta sqrt(1 - (2u/W)^2)) / I0(beta) on |u| <= W/2, u in grid units,
+// on a fine grid of at least 1.28 points per retained mode instead of two.
+constexpr int kKbWidth = 14;     // W: grid points per axis
+constexpr int kKbDegree = 15;    // polynomial degree of the evaluated window
+constexpr double kKbBeta = 32.0;
+// w at the W points o = kb_low + j - frac, j = 0..W-1, as polynomials in
+// t = 2 frac - 1: coef[j * (kKbDegree + 1) + k] multiplies t^k.
+constexpr int kKbLow = -(kKbWidth / 2 - 1);
+void kb_polynomials(double* coef);
+double kb_transform(double x);   // Fourier transform of w at x cycles per grid unit
+int kb_length(int modes);        // fine grid length for that many modes
+// True when the Kaiser-Bessel window serves these parameters.
+bool mesh_window(const Cell& cell, const ewg_params& p, bool mixed);
 int box_count(double r_cut, double recLen);  // common/ewald_cell_list.f90:56-73
 
 // Balanced splitting of the direct engine (direct/ewald_direct_3d.f90:319-347).
@@ -78,11 +94,13 @@ struct FftPlan {
 
 // Everything the mesh kernels need about one evaluation.
 struct MeshGeom {
-  int n[3];        // fine grid = 2 * modes
+  int n[3];        // fine grid: 2 * modes (Gaussian), kb_length(modes) (Kaiser-Bessel)
   int M[3];        // retained modes
   int K1, K2, K3;  // compact spectrum extents: M1/2+1, M2+1, M3+1
-  int m;           // window half-width
-  int W;           // 2m+1
+  int m;           // window half-width of the parameter set
+  int kb;          // 1: Kaiser-Bessel window
+  int lo;          // lowest stencil offset from the lowest grid point: -m, or kKbLow
+  int W;           // stencil points per axis: 2m+1, or kKbWidth
   double b;        // window shape
   double pref;     // 1/sqrt(pi b)
   double rec[3][3];

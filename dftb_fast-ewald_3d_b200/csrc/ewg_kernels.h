@@ -135,8 +135,10 @@ struct StencilDims {
   int S[3];        // most tiles one stencil touches per axis
   int woff[3];     // per-atom weight offsets per axis
   int wstride;     // per-atom weight count: sum S_d T_d
-  int m;           // window half-width
-  double b;        // window shape
+  int lo;          // lowest stencil offset from the atom's lowest grid point
+  int W;           // stencil points per axis
+  int kb;          // 1: Kaiser-Bessel window
+  double b;        // Gaussian window shape
   double pref;     // 1/sqrt(pi b)
   int ad;          // 1: window derivatives stored after the weights (forces by
                    // analytic differentiation of the window)
@@ -203,6 +205,8 @@ struct BatchLaunch {
   const BatchCell* cells = nullptr;
   int ncells = 0;
   int mixed = 0, nc = 1, nparts = 1, ad = 0;
+  int any_kb = 0, any_gauss = 0;  // windows that occur among the cells
+  int wstride = 0;                // weight values per atom, common to the cells
   int L = 1;           // FFT lines per CTA, one value for every cell
   int uniform[3] = {0, 0, 0};  // every cell has the same length along this axis
   FftPlan plan[3];             // that length's plan (when uniform)

@@ -89,21 +89,21 @@ __device__ __forceinline__ void weights_row(const int4* __restrict__ mc,
   const int c = d == 0 ? c4.x : (d == 1 ? c4.y : c4.z);
   const double frac = d == 0 ? f4.x : (d == 1 ? f4.y : f4.z);
   const int nd = sd.n[d], T = sd.T[d], nt = sd.ntiles[d];
-  const int m = sd.m;
-  // Tiles the stencil [c - m, c + m] (mod n) runs through, starting at `first`;
+  const int lo = sd.lo, hi = sd.lo + sd.W - 1, W = sd.W;
+  // Tiles the stencil [c + lo, c + hi] (mod n) runs through, starting at `first`;
   // a stencil that comes back into its first tile, or covers the whole axis,
   // touches every tile once (repeated points are folded into the weights).
   int first, count;
-  if (2 * m + 1 >= nd) {
+  if (W >= nd) {
     first = 0;
     count = nt;
   } else {
-    const int p0 = pmod(c - m, nd);
+    const int p0 = pmod(c + lo, nd);
     int t = p0 / T;
     first = t;
     int covered = min((t + 1) * T, nd) - p0;
     count = 1;
-    while (covered < 2 * m + 1) {
+    while (covered < W) {
       t = t + 1 == nt ? 0 : t + 1;
       ++count;
       covered += min((t + 1) * T, nd) - t * T;
@@ -118,16 +118,16 @@ __device__ __forceinline__ void weights_row(const int4* __restrict__ mc,
   const int origin = ((first + s) % nt) * T;
   R wv[TX], dv[TX];
   static_assert(TX == TY && TY == TZ, "one row length for all axes");
-  if (2 * m + 1 < nd) {
-    // Every point has at most one image in [-m, m]: the offsets of the row are
+  if (W < nd) {
+    // Every point has at most one image in [lo, hi]: the offsets of the row are
     // consecutive (one wrap at most) and the eight terms are independent.
     const int o0 = pmod(origin - c, nd);
 #pragma unroll
     for (int p = 0; p < TX; ++p) {
       int o = o0 + p;
       if (o >= nd) o -= nd;
-      if (o > m) o -= nd;  // largest offset <= m congruent to P - c
-      const bool live = s < count && origin + p < nd && o >= -m;
+      if (o > hi) o -= nd;  // largest offset <= hi congruent to P - c
+      const bool live = s < count && origin + p < nd && o >= lo;
       const double dd = frac - static_cast<double>(o);
       const double e = sd.pref * exp(-(dd * dd) / sd.b);
       wv[p] = static_cast<R>(live ? e : 0.0);
@@ -139,10 +139,10 @@ __device__ __forceinline__ void weights_row(const int4* __restrict__ mc,
       const int P = origin + p;
       double w = 0.0, dw = 0.0;
       if (s < count && P < nd) {
-        int o = pmod(P - c, nd);  // largest offset <= m congruent to P - c
-        while (o > m) o -= nd;
-        while (o + nd <= m) o += nd;
-        for (; o >= -m; o -= nd) {
+        int o = pmod(P - c, nd);  // largest offset <= hi congruent to P - c
+        while (o > hi) o -= nd;
+        while (o + nd <= hi) o += nd;
+        for (; o >= lo; o -= nd) {
           const double dd = frac - static_cast<double>(o);
           const double e = sd.pref * exp(-(dd * dd) / sd.b);
           w += e;
@@ -193,10 +193,136 @@ __global__ void k_weights_seg(const BatchCell* __restrict__ cells, const int* __
   const int c = seg_cell(prefix, ncells, idx);
   const BatchCell& bc = cells[c];
   const StencilDims sd = bc.sd;
+  if (sd.kb) return;  // k_weights_kb_seg
   const int SS = sd.S[0] + sd.S[1] + sd.S[2];
   const int local = static_cast<int>(idx - prefix[c]);
   const int kl = local / SS;
   weights_row<R>(mc, fr, perm, bc.atom0 + kl, local - kl * SS, sd, wtab, qk, slot);
+}
+
+// ---------------------------------------------------------------------------
+// Kaiser-Bessel weights (plain form).  A warp takes one axis of 32 atoms, a lane
+// one atom: the W = 14 weights are polynomials in the atom's fraction with the
+// same coefficients for every lane, read as constant operands, so the 14 x 15
+// multiply-adds of a lane need no memory access.  (Evaluated row by row in the
+// layout above, neighbouring lanes would need different polynomials and so
+// gather their coefficients.)  The values go to the tiled rows through shared
+// memory, from where the CTA writes the rows of its 32 atoms, a contiguous piece
+// of the table, with full 16-byte stores.  Bounded by those stores (576 B per
+// atom): at 32,769 atoms 18.9 MB.
+// ---------------------------------------------------------------------------
+constexpr int kKbCoefs = kKbDegree + 1;
+constexpr int kKbAtoms = 32;              // atoms per CTA, one warp per axis
+constexpr int kKbRow = 3 * 3 * kTileX;    // most values of an atom's three axes
+__constant__ double c_kb[kKbWidth * kKbCoefs];
+
+// Shared values per atom: the rows (and, for ad, derivative rows) plus padding
+// that spreads the lanes over the banks and keeps rows 16-byte aligned.
+__host__ __device__ constexpr int kb_pitch(int ad) { return (ad ? 2 : 1) * kKbRow + 2; }
+
+// The weights of sorted atom k along axis d into its shared row w (derivative
+// rows dw, null without them), and its slot record.
+__device__ __forceinline__ void kb_axis(const int4* __restrict__ mc,
+                                        const double4* __restrict__ fr,
+                                        const int* __restrict__ perm, int k, int d,
+                                        const StencilDims& sd, double* __restrict__ w,
+                                        double* __restrict__ dw, double* __restrict__ qk,
+                                        int4* __restrict__ slot) {
+  const int i = perm[k];
+  const int4 c4 = mc[i];
+  const double4 f4 = fr[i];
+  const int c = d == 0 ? c4.x : (d == 1 ? c4.y : c4.z);
+  const double frac = d == 0 ? f4.x : (d == 1 ? f4.y : f4.z);
+  const int nd = sd.n[d], nt = sd.ntiles[d];
+  int p0 = c + kKbLow;
+  if (p0 < 0) p0 += nd;
+  const int first = p0 / kTileX;
+  // Whole tiles of 8 points: the stencil covers (p0 mod 8) + 14 row points.
+  const int row0 = p0 - first * kTileX;
+  const int count = min((row0 + kKbWidth + kTileX - 1) / kTileX, nt);
+  const double t = 2.0 * frac - 1.0;
+  const double dscale = 2.0 * static_cast<double>(nd);  // dt/ds_d
+  const int span = nt * kTileX;
+  double* out = w + sd.woff[d];
+#pragma unroll
+  for (int j = 0; j < kKbWidth; ++j) {
+    const double* cf = c_kb + j * kKbCoefs;
+    double v = cf[kKbDegree], dv = 0.0;
+#pragma unroll
+    for (int e = kKbDegree - 1; e >= 0; --e) {
+      if (dw) dv = fma(dv, t, v);
+      v = fma(v, t, cf[e]);
+    }
+    int r = row0 + j;
+    if (r >= span) r -= span;  // back in the first tile (nt = 2)
+    out[r] = v;
+    if (dw) dw[sd.woff[d] + r] = dscale * dv;
+  }
+  int* sp = reinterpret_cast<int*>(&slot[k]);
+  sp[d] = first | (count << 16);
+  if (d == 0) {
+    sp[3] = 0;
+    qk[k] = f4.w;
+  }
+}
+
+// Zeroes the CTA's shared rows, fills them and writes each row's first
+// rowlen(k) values (0: not a row of this window) to the table.
+template <class Fill, class RowLen>
+__device__ __forceinline__ void kb_rows(double* sm, int pitch, int k0, int n, int wstride,
+                                        double* __restrict__ wtab, Fill fill, RowLen rowlen) {
+  __shared__ int len[kKbAtoms];
+  const int lane = threadIdx.x & 31, d = threadIdx.x >> 5;
+  for (int e = threadIdx.x; e < kKbAtoms * pitch; e += 3 * 32) sm[e] = 0.0;
+  if (threadIdx.x < kKbAtoms) len[threadIdx.x] = k0 + lane < n ? rowlen(k0 + lane) : 0;
+  __syncthreads();
+  if (len[lane]) fill(k0 + lane, d, sm + lane * pitch);
+  __syncthreads();
+  const int half = pitch / 2;
+  for (int e = threadIdx.x; e < kKbAtoms * half; e += 3 * 32) {
+    const int a = e / half, v = 2 * (e - a * half);
+    if (v < len[a])
+      *reinterpret_cast<double2*>(wtab + static_cast<size_t>(k0 + a) * wstride + v) =
+          *reinterpret_cast<const double2*>(sm + a * pitch + v);
+  }
+}
+
+template <bool AD>
+__global__ void __launch_bounds__(96) k_weights_kb(const int4* __restrict__ mc,
+                                                   const double4* __restrict__ fr,
+                                                   const int* __restrict__ perm, int n,
+                                                   StencilDims sd, double* __restrict__ wtab,
+                                                   double* __restrict__ qk,
+                                                   int4* __restrict__ slot) {
+  chain_enter();
+  __shared__ __align__(16) double sm[kKbAtoms * kb_pitch(AD)];
+  kb_rows(
+      sm, kb_pitch(AD), blockIdx.x * kKbAtoms, n, sd.wstride, wtab,
+      [&](int k, int d, double* row) {
+        kb_axis(mc, fr, perm, k, d, sd, row, AD ? row + sd.dwoff : nullptr, qk, slot);
+      },
+      [&](int) { return sd.wstride; });
+}
+
+// Every cell of a batch; rows of cells with a Gaussian window are k_weights_seg's.
+template <bool AD>
+__global__ void __launch_bounds__(96) k_weights_kb_seg(
+    const BatchCell* __restrict__ cells, const int* __restrict__ atom_prefix, int ncells, int n,
+    int wstride, const int4* __restrict__ mc, const double4* __restrict__ fr,
+    const int* __restrict__ perm, double* __restrict__ wtab, double* __restrict__ qk,
+    int4* __restrict__ slot) {
+  chain_enter();
+  __shared__ __align__(16) double sm[kKbAtoms * kb_pitch(AD)];
+  kb_rows(
+      sm, kb_pitch(AD), blockIdx.x * kKbAtoms, n, wstride, wtab,
+      [&](int k, int d, double* row) {
+        const StencilDims sd = cells[seg_cell(atom_prefix, ncells, k)].sd;
+        kb_axis(mc, fr, perm, k, d, sd, row, AD ? row + sd.dwoff : nullptr, qk, slot);
+      },
+      [&](int k) {
+        const StencilDims& sd = cells[seg_cell(atom_prefix, ncells, k)].sd;
+        return sd.kb ? (AD ? 2 : 1) * sd.dwoff : 0;
+      });
 }
 
 // ---------------------------------------------------------------------------
@@ -1347,7 +1473,11 @@ void launch_weights(const MeshPlan& mp, const int4* mc, const double4* fr, const
                     void* wtab, void* qk, int4* slot, cudaStream_t st) {
   if (n == 0) return;
   const long threads = static_cast<long>(mp.sd.S[0] + mp.sd.S[1] + mp.sd.S[2]) * n;
-  if (mp.mixed)
+  if (mp.sd.kb)
+    launch_chained(mp.sd.ad ? k_weights_kb<true> : k_weights_kb<false>, blocks_for(n, kKbAtoms),
+                   96, 0, st, mc, fr, perm, n, mp.sd, static_cast<double*>(wtab),
+                   static_cast<double*>(qk), slot);
+  else if (mp.mixed)
     launch_chained(k_weights_tiled<float>, blocks_for(threads, 128), 128, 0, st,
         mc, fr, perm, n, mp.sd, static_cast<float*>(wtab), static_cast<float*>(qk), slot);
   else
@@ -1498,6 +1628,14 @@ void launch_gather_final(const MeshPlan& mp, const int4* slot, const int* perm, 
 void launch_weights_seg(const BatchLaunch& b, const int4* mc, const double4* fr, const int* perm,
                         void* wtab, void* qk, int4* slot, cudaStream_t st) {
   if (b.n_weights == 0) return;
+  if (b.any_kb) {
+    launch_chained(b.ad ? k_weights_kb_seg<true> : k_weights_kb_seg<false>,
+                   blocks_for(b.n_atoms, kKbAtoms), 96, 0, st, b.cells, b.p_atoms, b.ncells,
+                   b.n_atoms, b.wstride, mc, fr, perm, static_cast<double*>(wtab),
+                   static_cast<double*>(qk), slot);
+    ++g_launches;
+    if (!b.any_gauss) return;
+  }
   if (b.mixed)
     launch_chained(k_weights_seg<float>, blocks_for(b.n_weights, 128), 128, 0, st, b.cells,
                    b.p_weights, b.ncells, b.n_weights, mc, fr, perm, static_cast<float*>(wtab),
@@ -1605,7 +1743,15 @@ void launch_gather_final_seg(const BatchLaunch& b, const int4* slot, const int* 
   ++g_launches;
 }
 
-int stencil_configure_kernels() { return EWG_OK; }
+int stencil_configure_kernels() {
+  // The window's polynomials, computed once (0.5 ms) and put on the context's device.
+  struct Table {
+    double coef[kKbWidth * kKbCoefs];
+    Table() { kb_polynomials(coef); }
+  };
+  static const Table t;
+  return cudaMemcpyToSymbol(c_kb, t.coef, sizeof(t.coef)) == cudaSuccess ? EWG_OK : EWG_ERR_CUDA;
+}
 
 int measure_dmma_peak(cudaStream_t st, double* tflops) {
   int dev = 0, nsm = 0;
