@@ -15,6 +15,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -23,8 +24,10 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libewald_b200.so")
 
 SOURCES = ["ewg_chain.cpp", "ewg_real.cu", "ewg_mesh.cu", "ewg_stencil.cu", "ewg_api.cu",
-           "ewg_static.cu", "ewg_external.cu", "ewg_points.cu"]
-HEADERS = ["ewg_internal.h", "ewg_kernels.h", "ewg_fft.cuh"]
+           "ewg_static.cu", "ewg_external.cu", "ewg_points.cu", "ewg_fft64.cu"]
+# The transform passes of many lengths, in several files so that they build in parallel.
+SOURCES += [f"ewg_fft64_{part}.cu" for part in ("a", "b", "c", "d", "e", "f", "g", "s0", "s1", "s2", "s3")]
+HEADERS = ["ewg_internal.h", "ewg_kernels.h", "ewg_fft.cuh", "ewg_dft.cuh", "ewg_fft64.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -50,7 +53,7 @@ def _stale(obj: str, deps: list[str]) -> bool:
 def build(force: bool = False, verbose: bool = False, ptxas_verbose: bool = False) -> str:
     os.makedirs(BUILD, exist_ok=True)
     headers = [os.path.join(CSRC, h) for h in HEADERS] + [os.path.join(ROOT, "include", "ewald_b200.h")]
-    objs = []
+    objs, todo = [], []
     common = ["-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-ccbin", host_cxx(),
               "-I", os.path.join(ROOT, "include")]
     for src in SOURCES:
@@ -66,9 +69,15 @@ def build(force: bool = False, verbose: bool = False, ptxas_verbose: bool = Fals
         else:
             cmd = [host_cxx(), "-O3", "-std=c++17", "-fPIC", "-I", os.path.join(ROOT, "include"),
                    "-I", "/usr/local/cuda/include", "-c", path, "-o", obj]
+        todo.append(cmd)
+
+    def compile_one(cmd):
         if verbose:
             print(" ".join(cmd), flush=True)
         subprocess.run(cmd, check=True)
+
+    with ThreadPoolExecutor(max_workers=max(1, os.cpu_count() or 1)) as pool:
+        list(pool.map(compile_one, todo))
     if force or _stale(LIB, objs):
         cmd = [nvcc(), "-shared", "-ccbin", host_cxx()] + ARCH + objs + ["-o", LIB, "-lcudart"]
         if verbose:

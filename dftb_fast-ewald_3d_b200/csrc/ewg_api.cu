@@ -456,6 +456,7 @@ int evaluate(ewg_context* c, int n, const double* pos, long sa, long sd, const d
   mp.mixed = mixed;
   mp.prof = &c->prof;
   mp.lines_cap = ks.fft_lines;
+  mp.two_pass = ks.fft_sched != 2;
   mp.gather_warps = ks.gather_warps;
   mp.stencil = ks.stencil;
   for (int d = 0; d < 3; ++d) {
@@ -707,14 +708,14 @@ int validate_host(const ewg_context* c, int n, const double* pos, const double* 
 struct SegPlan {
   BatchLaunch b;
   std::vector<BatchCell> cells;
-  std::vector<int> prefix;  // 11 arrays of ncells + 1
+  std::vector<int> prefix;  // SP_COUNT arrays of ncells + 1, then the pass groups' tables
   size_t wstride = 0;       // common weight stride (values per atom)
   int pstride = 0;          // common partial slots per atom
   size_t pairs_max = 0;
   size_t grid = 0, A1 = 0, A2 = 0, B2 = 0, B1 = 0, out = 0;  // total bytes
 };
 
-// Offsets of the 11 prefix arrays inside SegPlan::prefix.
+// Offsets of the prefix arrays inside SegPlan::prefix.
 enum { SP_ATOMS, SP_WEIGHTS, SP_SLOTS, SP_TILES, SP_R2C, SP_YFWD, SP_Z, SP_YINV, SP_C2R, SP_BOXES,
        SP_COUNT };
 
@@ -730,6 +731,9 @@ int seg_plan(ewg_context* c, int n_cells, const int* offsets, const std::vector<
   const int nparts = want_force ? 4 : 1;
   const size_t rs = mixed ? 4 : 8;
   sp.cells.assign(n_cells, BatchCell{});
+  // Axes whose length has a register-radix kernel run in groups by length class;
+  // the launch shapes below are the other cells'.
+  auto grouped = [&](const MeshGeom& g, int d) { return !mixed && fft64_class(g.n[d]) >= 0; };
   int L = 8, nmax[3] = {0, 0, 0}, lpa = 8;
   std::vector<int> nboxes(n_cells);
   for (int ci = 0; ci < n_cells; ++ci) {
@@ -756,16 +760,16 @@ int seg_plan(ewg_context* c, int n_cells, const int* offsets, const std::vector<
       if ((rc = get_fft(c, bc.g.n[d], fp))) return rc;
       bc.fft[d] = fp;
       if ((rc = get_corr(c, bc.g, d, &bc.corr2[d]))) return rc;
-      nmax[d] = std::max(nmax[d], bc.g.n[d]);
+      if (!grouped(bc.g, d)) nmax[d] = std::max(nmax[d], bc.g.n[d]);
     }
     stencil_dims(bc.g, ad, bc.sd);
     (bc.g.kb ? sp.b.any_kb : sp.b.any_gauss) = 1;
     sp.wstride = std::max<size_t>(sp.wstride, bc.sd.wstride);
     sp.pstride = std::max(sp.pstride, bc.sd.pstride);
     if (bc.sd.pstride > 32) lpa = 32;
-    L = std::min(L, mesh_batch_lines(bc.g.n[0], mixed, 0));
-    L = std::min(L, mesh_batch_lines(bc.g.n[1], mixed, 0));
-    L = std::min(L, mesh_batch_lines(bc.g.n[2], mixed, bc.g.K3));
+    for (int d = 0; d < 3; ++d)
+      if (!grouped(bc.g, d))
+        L = std::min(L, mesh_batch_lines(bc.g.n[d], mixed, d == 2 ? bc.g.K3 : 0));
     nboxes[ci] = bc.rg.nb[0] * bc.rg.nb[1] * bc.rg.nb[2];
   }
   if (L < 1) return EWG_ERR_GRID_TOO_LARGE;
@@ -786,6 +790,9 @@ int seg_plan(ewg_context* c, int n_cells, const int* offsets, const std::vector<
     const int SS = sd.S[0] + sd.S[1] + sd.S[2], S3 = sd.S[0] * sd.S[1] * sd.S[2];
     int blk[5];
     mesh_pass_blocks(g, L, nc, blk);
+    if (grouped(g, 0)) blk[0] = blk[4] = 0;
+    if (grouped(g, 1)) blk[1] = blk[3] = 0;
+    if (grouped(g, 2)) blk[2] = 0;
     bc.box0 = pre(SP_BOXES)[ci];
     bc.tile0 = pre(SP_TILES)[ci];
     pre(SP_ATOMS)[ci + 1] = pre(SP_ATOMS)[ci] + na;
@@ -813,7 +820,7 @@ int seg_plan(ewg_context* c, int n_cells, const int* offsets, const std::vector<
     oB2 += align256(nz * static_cast<size_t>(g.n[2]) * g.K2 * g.K1 * cb);
     oB1 += align256(ny * static_cast<size_t>(g.n[2]) * g.n[1] * g.K1 * cb);
     oout += align256(nc * G * rs);
-    smz = std::max(smz, mesh_pass_smem(g.n[2], L, mixed, g.K3));
+    if (!grouped(g, 2)) smz = std::max(smz, mesh_pass_smem(g.n[2], L, mixed, g.K3));
   }
   sp.grid = og, sp.A1 = oA1, sp.A2 = oA2, sp.B2 = oB2, sp.B1 = oB1, sp.out = oout;
   BatchLaunch& b = sp.b;
@@ -826,9 +833,45 @@ int seg_plan(ewg_context* c, int n_cells, const int* offsets, const std::vector<
   b.lpa = lpa;
   for (int d = 0; d < 3; ++d) {
     b.uniform[d] = 1;
-    for (int ci = 1; ci < n_cells; ++ci) b.uniform[d] &= sp.cells[ci].g.n[d] == sp.cells[0].g.n[d];
-    b.plan[d] = sp.cells[0].fft[d];
+    const BatchCell* first = nullptr;
+    for (const BatchCell& bc : sp.cells) {
+      if (grouped(bc.g, d)) continue;
+      if (!first) first = &bc;
+      b.uniform[d] &= bc.g.n[d] == first->g.n[d];
+    }
+    if (first) b.plan[d] = first->fft[d];
   }
+  for (int d = 0; d < 3; ++d)
+    for (int k = 0; k < kClass64; ++k) {
+      std::vector<int> member;
+      for (int ci = 0; ci < n_cells; ++ci)
+        if (grouped(sp.cells[ci].g, d) && fft64_class(sp.cells[ci].g.n[d]) == k) member.push_back(ci);
+      if (member.empty()) continue;
+      // Longest lines first: the last wave is made of the short ones.
+      std::stable_sort(member.begin(), member.end(), [&](int a, int c2) {
+        return sp.cells[a].g.n[d] > sp.cells[c2].g.n[d];
+      });
+      BatchGroup gr;
+      gr.axis = d;
+      gr.klass = k;
+      gr.fwd.n = gr.inv.n = static_cast<int>(member.size());
+      gr.nmax = sp.cells[member[0]].g.n[d];
+      gr.off = sp.prefix.size();
+      std::vector<int> pf(1, 0), pi(1, 0);
+      for (int ci : member) {
+        int blk[5];
+        mesh_pass_blocks(sp.cells[ci].g, 8, nc, blk);
+        gr.K3 = std::max(gr.K3, sp.cells[ci].g.K3);
+        pf.push_back(pf.back() + (d == 0 ? blk[0] : d == 1 ? blk[1] : blk[2]));
+        pi.push_back(pi.back() + (d == 0 ? blk[4] : d == 1 ? blk[3] : 0));
+      }
+      gr.blocks_fwd = pf.back();
+      gr.blocks_inv = pi.back();
+      sp.prefix.insert(sp.prefix.end(), member.begin(), member.end());
+      sp.prefix.insert(sp.prefix.end(), pf.begin(), pf.end());
+      sp.prefix.insert(sp.prefix.end(), pi.begin(), pi.end());
+      b.groups.push_back(gr);
+    }
   b.wstride = static_cast<int>(sp.wstride);
   for (int d = 0; d < 3; ++d) b.smem[d] = mesh_pass_smem(nmax[d], L, mixed, 0);
   b.smem_z = smz;
@@ -922,6 +965,11 @@ int seg_prepare(ewg_context* c, SegPlan& sp, SegBufs& sb) {
   bl.p_yinv = dpre + SP_YINV * n1;
   bl.p_c2r = dpre + SP_C2R * n1;
   bl.p_final = bl.p_atoms;
+  for (BatchGroup& gr : bl.groups) {
+    gr.fwd.cell = gr.inv.cell = dpre + gr.off;
+    gr.fwd.prefix = dpre + gr.off + gr.fwd.n;
+    gr.inv.prefix = gr.fwd.prefix + gr.fwd.n + 1;
+  }
   return EWG_OK;
 }
 

@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "ewg_internal.h"
 
 namespace ewg {
@@ -154,6 +156,7 @@ struct MeshPlan {
   FftPlan fft[3];
   int mixed;                      // 0: FP64, 1: FP32 storage/products
   int lines_cap = 0;              // most FFT lines per CTA (0: the most that fit)
+  int two_pass = 1;               // FP64 passes of fft64_class lengths (radix schedule 1)
   int gather_warps = 4;           // FP64 i k gather CTA: 2, 4 or 8 warps
   int stencil = 1;                // mixed form's spread and gather: 1 FP64 tensor
                                   // cores on FP32 data, 2 FP32 CUDA cores
@@ -170,7 +173,14 @@ struct MeshPlan {
 // its cell through the launch's prefix array (prefix[c] = first index of cell
 // c, prefix[ncells] = total), and the cell's parameters come from the device
 // table below.
-struct BatchCell {
+// What the transform passes need of one cell.
+struct PassCell {
+  MeshGeom g;
+  FftPlan fft[3];
+  const double* corr2[3];
+  void *grid, *A1, *A2, *B2, *B1, *out;
+};
+struct BatchCell : PassCell {
   int atom0, natoms;  // global atom range
   int box0, tile0;    // first key of the cell in the global box and tile sorts
   double lat[3][3], rec[3][3];
@@ -178,11 +188,7 @@ struct BatchCell {
   double alpha, cut2;
   float pre2;
   double self_coef;
-  MeshGeom g;
   StencilDims sd;
-  FftPlan fft[3];
-  const double* corr2[3];
-  void *grid, *A1, *A2, *B2, *B1, *out;
 };
 
 // The cell holding global index idx: the last c with prefix[c] <= idx (cells
@@ -198,6 +204,41 @@ __device__ __forceinline__ int seg_cell(const int* __restrict__ prefix, int ncel
   }
   return lo;
 }
+
+// ---- FP64 transform passes with register radices (ewg_fft64.cuh) -----------
+// Lengths they exist for, by class; a batch launches one kernel per class.
+constexpr int kClass64 = 4;
+int fft64_class(int n);  // 0 .. kClass64 - 1, or -1: another length
+enum Pass64 { P64_R2C, P64_YFWD, P64_Z, P64_YINV, P64_C2R };
+// The cells of a batch in one class launch, longest lines first, end to end.
+struct PassGroup {
+  const int* cell = nullptr;    // cell of the batch table, per member
+  const int* prefix = nullptr;  // first block of each member; [n] = total
+  int n = 0;
+};
+struct Launch64 {
+  int pass = 0;
+  const PassCell* one = nullptr;     // a single cell, or
+  const BatchCell* cells = nullptr;  // a batch's table with the group of this launch
+  PassGroup group;
+  int blocks = 0;
+  int nmax = 0;  // batch: longest line of the group
+  int K3 = 0;    // z: most modes along z among the cells
+  int nz = 1;    // z: spectra out
+  int nc = 1;    // x C2R: components
+  double* stress = nullptr;
+  cudaStream_t st = nullptr;
+};
+void fft64_launch(int n, const Launch64& l);           // a single cell at length n
+void fft64_launch_seg(int klass, const Launch64& l);   // a batch's group of a class
+
+// One class's launches of a batch along one axis (two passes along x and y).
+struct BatchGroup {
+  int axis = 0, klass = 0, nmax = 0, K3 = 0;
+  PassGroup fwd, inv;  // r2c / y forward / z; c2r / y inverse
+  int blocks_fwd = 0, blocks_inv = 0;
+  size_t off = 0;      // members, then the two prefixes, in SegPlan::prefix
+};
 
 // Host description of one segmented batch: the device table, the prefix
 // array of every launch (device) and the totals (host).
@@ -225,6 +266,8 @@ struct BatchLaunch {
   const int* p_c2r = nullptr;     int n_c2r = 0;
   const int* p_final = nullptr;   long n_final = 0;    // natoms lpa
   int n_boxes = 0;
+  std::vector<BatchGroup> groups;  // passes by length class; the prefixes above
+                                   // cover the other cells
 };
 
 // Segmented counterparts of the single-cell launchers (same work per cell).

@@ -562,11 +562,7 @@ bool is_schedule(const FftPlan& p) {
 template <typename R, int L, typename F>
 void with_shape(const FftPlan& p, F&& f) {
   if constexpr (sizeof(R) == 8 && L == 4) {
-    if (is_schedule<280, 7, 5, 8>(p)) return f(StatShape<280, 7, 5, 8, 40>{});
     if (is_schedule<512, 8, 8, 8>(p)) return f(StatShape<512, 8, 8, 8, 64>{});
-  }
-  if constexpr (sizeof(R) == 8 && L == 8) {
-    if (is_schedule<128, 8, 8, 2>(p)) return f(StatShape<128, 8, 8, 2>{});
   }
   if constexpr (sizeof(R) == 4 && L == 8) {
     if (is_schedule<140, 7, 5, 4>(p)) return f(StatShape<140, 7, 5, 4, 36>{});
@@ -574,6 +570,39 @@ void with_shape(const FftPlan& p, F&& f) {
     if (is_schedule<280, 7, 5, 8>(p)) return f(StatShape<280, 7, 5, 8, 40>{});
   }
   f(DynShape{});
+}
+
+// A single cell's pass along axis d with the register-radix kernels of
+// ewg_fft64.cuh; false when the form or the length has none.
+template <typename R>
+bool pass64(const MeshPlan& mp, int pass, int d, const void* grid, const void* A1, const void* A2,
+            const void* B2, const void* B1, void* out, int nc, double* stress, cudaStream_t st) {
+  if (sizeof(R) != 8 || !mp.two_pass || fft64_class(mp.g.n[d]) < 0) return false;
+  PassCell pc{};
+  pc.g = mp.g;
+  for (int e = 0; e < 3; ++e) {
+    pc.fft[e] = mp.fft[e];
+    pc.corr2[e] = mp.corr2[e];
+  }
+  pc.grid = const_cast<void*>(grid);
+  pc.A1 = const_cast<void*>(A1);
+  pc.A2 = const_cast<void*>(A2);
+  pc.B2 = const_cast<void*>(B2);
+  pc.B1 = const_cast<void*>(B1);
+  pc.out = out;
+  int blk[5];
+  pass_blocks(mp.g, 8, nc, blk);
+  Launch64 l;
+  l.pass = pass;
+  l.one = &pc;
+  l.blocks = blk[pass];
+  l.K3 = mp.g.K3;
+  l.nz = nc == 4 ? 2 : 1;
+  l.nc = nc;
+  l.stress = stress;
+  l.st = st;
+  fft64_launch(mp.g.n[d], l);
+  return true;
 }
 
 template <typename R>
@@ -587,6 +616,7 @@ void forward_impl(const MeshPlan& mp, const void* grid, void* A1v, void* A2v, vo
   const size_t cb = cbytes<R>();
   {  // x, real to complex
     prof_mark(mp.prof, st, ST_FFT_X_R2C);
+    if (!pass64<R>(mp, P64_R2C, 0, grid, A1, A2, B2, nullptr, nullptr, nc, nullptr, st)) {
     const int npairs = n2 * n3 / 2;
     const int L = plan_lines(mp, n1, cb);
     const size_t sm = pass_smem(n1, L, cb, 0);
@@ -599,9 +629,11 @@ void forward_impl(const MeshPlan& mp, const void* grid, void* A1v, void* A2v, vo
       });
     });
     ++g_launches;
+    }
   }
   {  // y forward
     prof_mark(mp.prof, st, ST_FFT_Y_FWD);
+    if (!pass64<R>(mp, P64_YFWD, 1, grid, A1, A2, B2, nullptr, nullptr, nc, nullptr, st)) {
     const int L = plan_lines(mp, n2, cb);
     const size_t sm = pass_smem(n2, L, cb, 0);
     dim3 grd((g.K1 + L - 1) / L, n3);
@@ -614,9 +646,11 @@ void forward_impl(const MeshPlan& mp, const void* grid, void* A1v, void* A2v, vo
       });
     });
     ++g_launches;
+    }
   }
   {  // z forward + influence + z inverse
     prof_mark(mp.prof, st, ST_FFT_Z_INFL);
+    if (pass64<R>(mp, P64_Z, 2, grid, A1, A2, B2, nullptr, nullptr, nc, stress_part, st)) return;
     const int nz = nc == 4 ? 2 : 1;
     InfluenceArgs ia;
     for (int d = 0; d < 3; ++d) {
@@ -659,6 +693,7 @@ void inverse_impl(const MeshPlan& mp, const void* B2v, void* B1v, void* out, int
   const size_t cb = cbytes<R>();
   {
     prof_mark(mp.prof, st, ST_FFT_Y_INV);
+    if (!pass64<R>(mp, P64_YINV, 1, nullptr, nullptr, nullptr, B2, B1, out, nc, nullptr, st)) {
     const int L = plan_lines(mp, n2, cb);
     const size_t sm = pass_smem(n2, L, cb, 0);
     dim3 grd((g.K1 + L - 1) / L, n3, nc == 4 ? 3 : 1);
@@ -671,9 +706,11 @@ void inverse_impl(const MeshPlan& mp, const void* B2v, void* B1v, void* out, int
       });
     });
     ++g_launches;
+    }
   }
   {
     prof_mark(mp.prof, st, ST_FFT_X_C2R);
+    if (pass64<R>(mp, P64_C2R, 0, nullptr, nullptr, nullptr, B2, B1, out, nc, nullptr, st)) return;
     const int nrows = n2 * n3;
     const int L = plan_lines(mp, n1, cb);
     const size_t sm = pass_smem(n1, L, cb, 0);
@@ -731,9 +768,7 @@ void allow_shape() {
 template <typename R>
 void allow_all() {
   if constexpr (sizeof(R) == 8) {
-    allow_shape<R, 4, StatShape<280, 7, 5, 8, 40>>();
     allow_shape<R, 4, StatShape<512, 8, 8, 8, 64>>();
-    allow_shape<R, 8, StatShape<128, 8, 8, 2>>();
   } else {
     allow_shape<R, 8, StatShape<140, 7, 5, 4, 36>>();
     allow_shape<R, 8, StatShape<160, 5, 8, 4, 40>>();
@@ -759,46 +794,73 @@ void with_seg_shape(const BatchLaunch& b, int d, F&& f) {
     f(DynShape{});
 }
 
+// A pass's launches by length class.
+void groups64(const BatchLaunch& b, int pass, int axis, bool inverse, cudaStream_t st) {
+  for (const BatchGroup& gr : b.groups) {
+    if (gr.axis != axis) continue;
+    Launch64 l;
+    l.pass = pass;
+    l.cells = b.cells;
+    l.group = inverse ? gr.inv : gr.fwd;
+    l.blocks = inverse ? gr.blocks_inv : gr.blocks_fwd;
+    l.nmax = gr.nmax;
+    l.K3 = gr.K3;
+    l.nz = b.nc == 4 ? 2 : 1;
+    l.nc = b.nc;
+    l.st = st;
+    fft64_launch_seg(gr.klass, l);
+  }
+}
+
 template <typename R>
 void forward_seg_impl(const BatchLaunch& b, cudaStream_t st) {
   const int nz = b.nc == 4 ? 2 : 1;
   with_lines(b.L, [&](auto lc) {
     constexpr int LL = decltype(lc)::value;
+    groups64(b, P64_R2C, 0, false, st);
     if (b.n_r2c)
       with_seg_shape<R, LL>(b, 0, [&](auto sh) {
         using SH = decltype(sh);
         launch_chained(k_fft_x_r2c_seg<R, LL, SH>, b.n_r2c, SH::template threads<LL>(), b.smem[0],
                        st, b.cells, b.p_r2c, b.ncells);
+        ++g_launches;
       });
+    groups64(b, P64_YFWD, 1, false, st);
     if (b.n_yfwd)
       with_seg_shape<R, LL>(b, 1, [&](auto sh) {
         using SH = decltype(sh);
         launch_chained(k_fft_y_fwd_seg<R, LL, SH>, b.n_yfwd, SH::template threads<LL>(), b.smem[1],
                        st, b.cells, b.p_yfwd, b.ncells);
+        ++g_launches;
       });
+    groups64(b, P64_Z, 2, false, st);
     if (b.n_z)
       with_seg_shape<R, LL>(b, 2, [&](auto sh) {
         using SH = decltype(sh);
         launch_chained(k_fft_z_influence_seg<R, LL, SH>, b.n_z, SH::template threads<LL>(),
                        b.smem_z, st, b.cells, b.p_z, b.ncells, nz);
+        ++g_launches;
       });
   });
-  g_launches += 3;
 }
 
 template <typename R>
 void inverse_seg_impl(const BatchLaunch& b, cudaStream_t st) {
   with_lines(b.L, [&](auto lc) {
     constexpr int LL = decltype(lc)::value;
+    groups64(b, P64_YINV, 1, true, st);
     if (b.n_yinv)
       with_seg_shape<R, LL>(b, 1, [&](auto sh) {
         using SH = decltype(sh);
         launch_chained(k_fft_y_inv_seg<R, LL, SH>, b.n_yinv, SH::template threads<LL>(), b.smem[1],
                        st, b.cells, b.p_yinv, b.ncells);
+        ++g_launches;
       });
+    groups64(b, P64_C2R, 0, true, st);
     if (b.n_c2r)
       with_seg_shape<R, LL>(b, 0, [&](auto sh) {
         using SH = decltype(sh);
+        ++g_launches;
         if constexpr (LL >= 4) {
           if (b.nc == 4) {
             launch_chained(k_fft_x_c2r_seg<R, LL, 4, SH>, b.n_c2r, SH::template threads<LL>(),
@@ -810,7 +872,6 @@ void inverse_seg_impl(const BatchLaunch& b, cudaStream_t st) {
                        b.smem[0], st, b.cells, b.p_c2r, b.ncells, b.nc);
       });
   });
-  g_launches += 2;
 }
 
 }  // namespace
