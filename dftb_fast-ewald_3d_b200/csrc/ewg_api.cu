@@ -22,17 +22,17 @@ constexpr int kTiles[3] = {kTileX, kTileY, kTileZ};
 
 // Device buffers owned by a context, grown on demand and reused across calls.
 enum BufId {
-  B_POS, B_Q, B_POT, B_FORCE, B_POT_SR, B_F_SR, B_S4, B_S4S, B_BOXKEY, B_MC, B_FR,
-  B_COUNTS, B_CURSOR, B_BOXSTART, B_TMP, B_PERMBOX, B_WTAB,
+  B_POS, B_Q, B_POT, B_FORCE, B_POT_SR, B_F_SR, B_S4, B_S4S, B_BOXKEY,
+  B_COUNTS, B_ARRIVAL, B_BOXSTART, B_TMP, B_PERMBOX, B_WTAB,
   B_QK, B_GRID, B_A1, B_A2, B_B2, B_B1, B_OUT, B_ERR, B_SUMS, B_PARTIAL, B_KVEC, B_SK, B_WK,
   B_P6, B_O6, B_COORDS, B_SLOT, B_PART, B_PAIRTMP, B_PAIRS, B_PAIRSTART, B_CELLERR, B_ZPART,
-  B_BCOUNTS, B_BCURSOR, B_BTMP, B_EXT_T, B_EXT_S, B_EXT_SQ, B_EXT_TQ, B_EXT_BLUR, B_EXT_R,
+  B_BCOUNTS, B_BTMP, B_EXT_T, B_EXT_S, B_EXT_SQ, B_EXT_TQ, B_EXT_BLUR, B_EXT_R,
   B_EXT_G, B_EXT_SF, B_EXT_SF2, B_EXT_OUT, B_EXT_OUT2, B_X32S, B_TUNE_POT, B_TUNE_FORCE,
   // mesh-based point potentials: source (S) and target (T) tables
-  B_PT_S4, B_PT_S4S, B_PT_X32, B_PT_SKEY, B_PT_SPERM, B_PT_SBOX, B_PT_SMC, B_PT_SFR, B_PT_SWT,
-  B_PT_SQK, B_PT_SSLOT, B_PT_SPAIRS, B_PT_SPSTART, B_PT_TKEY, B_PT_TPERM, B_PT_TBOX, B_PT_TMC,
-  B_PT_TFR, B_PT_TWT, B_PT_TQK, B_PT_TSLOT, B_PT_TPAIRS, B_PT_TPSTART, B_PT_BCNT, B_PT_BCUR,
-  B_PT_BTMP, B_PT_KCNT, B_PT_KCUR, B_PT_PTMP, B_PT_QNEG, B_PT_PART, B_PT_POTSR, B_PT_GRADSR,
+  B_PT_S4, B_PT_S4S, B_PT_SKEY, B_PT_SPERM, B_PT_SBOX, B_PT_SWT,
+  B_PT_SQK, B_PT_SSLOT, B_PT_SPAIRS, B_PT_SPSTART, B_PT_T4S, B_PT_TPERM, B_PT_TBOX,
+  B_PT_TWT, B_PT_TQK, B_PT_TSLOT, B_PT_TPAIRS, B_PT_TPSTART, B_PT_BCNT,
+  B_PT_BTMP, B_PT_KCNT, B_PT_PARR, B_PT_PTMP, B_PT_QNEG, B_PT_PART, B_PT_POTSR, B_PT_GRADSR,
   B_PT_GRAD, B_PT_POTOUT,
   // segmented batches: cell table and launch prefixes
   B_BT_CELLS, B_BT_PREFIX,
@@ -473,14 +473,10 @@ int evaluate(ewg_context* c, int n, const double* pos, long sa, long sd, const d
   double4* s4s = dbuf<double4>(c, B_S4S, n, &rc);
   float4* x32s = dbuf<float4>(c, B_X32S, n, &rc);
   int* boxkey = dbuf<int>(c, B_BOXKEY, n, &rc);
-  int4* mcv = dbuf<int4>(c, B_MC, n, &rc);
-  double4* fr = dbuf<double4>(c, B_FR, n, &rc);
   int* counts = dbuf<int>(c, B_COUNTS, ntiles, &rc);
-  int* cursor = dbuf<int>(c, B_CURSOR, ntiles, &rc);
   int* boxstart = dbuf<int>(c, B_BOXSTART, nboxes + 1, &rc);
   int* permbox = dbuf<int>(c, B_PERMBOX, n, &rc);
   int* bcounts = dbuf<int>(c, B_BCOUNTS, nboxes, &rc);
-  int* bcursor = dbuf<int>(c, B_BCURSOR, nboxes, &rc);
   int* btmp = dbuf<int>(c, B_BTMP, n, &rc);
   double* pot_sr = dbuf<double>(c, B_POT_SR, n, &rc);
   double* f_sr = dbuf<double>(c, B_F_SR, 3 * static_cast<size_t>(n), &rc);
@@ -495,7 +491,8 @@ int evaluate(ewg_context* c, int n, const double* pos, long sa, long sd, const d
   int4* slot = dbuf<int4>(c, B_SLOT, n, &rc);
   double* part = dbuf<double>(c, B_PART, ms.part / 8, &rc);
   const int npairs_max = n * mp.sd.S[0] * mp.sd.S[1] * mp.sd.S[2];
-  int4* pairtmp = dbuf<int4>(c, B_PAIRTMP, npairs_max, &rc);
+  int* arrival = dbuf<int>(c, B_ARRIVAL, npairs_max, &rc);
+  int2* unordered = dbuf<int2>(c, B_PAIRTMP, npairs_max, &rc);
   int2* pairs = dbuf<int2>(c, B_PAIRS, npairs_max, &rc);
   int* pairstart = dbuf<int>(c, B_PAIRSTART, ntiles + 1, &rc);
   int* err = err_flag ? err_flag : dbuf<int>(c, B_ERR, 1, &rc);
@@ -534,30 +531,21 @@ int evaluate(ewg_context* c, int n, const double* pos, long sa, long sd, const d
     if (!err_flag) cudaMemsetAsync(err, 0, sizeof(int), st);
     if (stress12) cudaMemsetAsync(zpart, 0, sizeof(double) * nz, st);  // z-pass partials
     prof_mark(mp.prof, st, ST_PREP);
-    if (!reuse) {
-      launch_atom_prep(pos, sa, sd, q, n, cell, rg.nb, mp.g.n, s4, boxkey, mcv, fr, st);
-      launch_bucket_sort(boxkey, n, nboxes, bcounts, bcursor, boxstart, btmp, permbox, st);
-      if (concurrent) {
-        cudaEventRecord(c->fork, st);
-        cudaStreamWaitEvent(rs, c->fork, 0);
-      }
-      launch_permute_box(s4, permbox, n, cell.lat, s4s, x32s, rs);
-      prof_mark(mp.prof, st, ST_WEIGHTS);
-      launch_weights(mp, mcv, fr, permbox, n, wtab, qk, slot, st);
-      launch_pair_bins(mp, slot, n, counts, cursor, pairstart, pairtmp, pairs, npairs_max, st);
-    } else {
-      // Geometry unchanged: refresh only the charges in the sorted layouts; the
-      // window weights, slots and pair lists stay.
-      launch_atom_prep(pos, sa, sd, q, n, cell, nullptr, nullptr, s4, nullptr, nullptr, nullptr,
-                       st);
-      if (concurrent) {
-        cudaEventRecord(c->fork, st);
-        cudaStreamWaitEvent(rs, c->fork, 0);
-      }
-      launch_permute_box(s4, permbox, n, cell.lat, s4s, x32s, rs);
-      prof_mark(mp.prof, st, ST_WEIGHTS);
-      launch_sorted_charges(mp, q, permbox, n, qk, st);
+    const PairBins bins{counts, arrival, pairstart, unordered, pairs};
+    // Geometry unchanged (reuse): only the charges in the sorted layouts are
+    // refreshed; the window weights, slots and pair lists stay.
+    if (!reuse)
+      launch_atom_sort(pos, sa, sd, q, n, cell, rg.nb,
+                       SortBufs{s4, boxkey, bcounts, btmp, boxstart, permbox, s4s, x32s}, counts,
+                       ntiles, st);
+    else
+      launch_refresh_charges(q, permbox, n, s4s, x32s, qk, mixed, st);
+    if (concurrent) {
+      cudaEventRecord(c->fork, st);
+      cudaStreamWaitEvent(rs, c->fork, 0);
     }
+    prof_mark(mp.prof, st, ST_WEIGHTS);
+    if (!reuse) launch_weights_bins(mp, s4s, n, wtab, qk, slot, bins, st);
     prof_mark(mp.prof, st, ST_REAL);
     launch_real_space(s4s, x32s, permbox, boxstart, n, rg, p.alpha, p.r_cut, mixed, pot_sr, f_sr,
                       err, rs);
@@ -565,12 +553,12 @@ int evaluate(ewg_context* c, int n, const double* pos, long sa, long sd, const d
       launch_real_stress(s4s, x32s, boxstart, n, rg, p.alpha, p.r_cut, p6, stress12, err, rs);
     if (concurrent) cudaEventRecord(c->join, rs);
     prof_mark(mp.prof, st, ST_SPREAD);
-    launch_spread(mp, pairstart, pairs, wtab, qk, grid, st);
+    launch_spread(mp, bins, slot, n, reuse, wtab, qk, grid, st);
     launch_forward_and_weight(mp, grid, A1, A2, B2, nc, st, zpart);
     if (stress12) launch_sum_partials(zpart, mp.g.K1 * mp.g.K2, 6, stress12 + 6, st);
     launch_inverse(mp, B2, B1, outg, nc, st);
     prof_mark(mp.prof, st, ST_GATHER);
-    launch_gather(mp, pairstart, pairs, wtab, outg, nc, part, st);
+    launch_gather(mp, pairstart, unordered, wtab, outg, nc, part, st);
     if (concurrent) cudaStreamWaitEvent(st, c->join, 0);  // pot_sr, f_sr, err ready
     // Both force schemes deliver the fractional derivatives D_d = dphi/ds_d.
     launch_gather_final(mp, slot, permbox, part, nparts, n, q, self_coef, pot_shift, pot_sr, f_sr,
@@ -763,7 +751,6 @@ int seg_plan(ewg_context* c, int n_cells, const int* offsets, const std::vector<
       if (!grouped(bc.g, d)) nmax[d] = std::max(nmax[d], bc.g.n[d]);
     }
     stencil_dims(bc.g, ad, bc.sd);
-    (bc.g.kb ? sp.b.any_kb : sp.b.any_gauss) = 1;
     sp.wstride = std::max<size_t>(sp.wstride, bc.sd.wstride);
     sp.pstride = std::max(sp.pstride, bc.sd.pstride);
     if (bc.sd.pstride > 32) lpa = 32;
@@ -873,6 +860,7 @@ int seg_plan(ewg_context* c, int n_cells, const int* offsets, const std::vector<
       b.groups.push_back(gr);
     }
   b.wstride = static_cast<int>(sp.wstride);
+  b.pstride = sp.pstride;
   for (int d = 0; d < 3; ++d) b.smem[d] = mesh_pass_smem(nmax[d], L, mixed, 0);
   b.smem_z = smz;
   b.n_atoms = pre(SP_ATOMS)[n_cells];
@@ -892,12 +880,9 @@ int seg_plan(ewg_context* c, int n_cells, const int* offsets, const std::vector<
 
 // Device buffers of a segmented batch.
 struct SegBufs {
-  double4 *s4, *s4s, *fr;
-  float4* x32;
-  int *boxkey, *perm, *boxstart, *bcounts, *bcursor, *btmp;
-  int4 *mc, *slot, *pairtmp;
-  int *tcounts, *tcursor, *pairstart;
-  int2* pairs;
+  SortBufs sort;
+  PairBins bins;
+  int4* slot;
   void *wtab, *qk;
   double *part, *pot_sr, *f_sr;
 };
@@ -909,23 +894,21 @@ int seg_prepare(ewg_context* c, SegPlan& sp, SegBufs& sb) {
   const BatchLaunch& b = sp.b;
   const size_t rs = b.mixed ? 4 : 8;
   const size_t na = std::max(b.n_atoms, 1);
-  sb.s4 = dbuf<double4>(c, B_S4, na, &rc);
-  sb.s4s = dbuf<double4>(c, B_S4S, na, &rc);
-  sb.x32 = dbuf<float4>(c, B_X32S, na, &rc);
-  sb.boxkey = dbuf<int>(c, B_BOXKEY, na, &rc);
-  sb.perm = dbuf<int>(c, B_PERMBOX, na, &rc);
-  sb.mc = dbuf<int4>(c, B_MC, na, &rc);
-  sb.fr = dbuf<double4>(c, B_FR, na, &rc);
+  const size_t np = std::max<size_t>(sp.pairs_max, 1);
+  sb.sort.s4 = dbuf<double4>(c, B_S4, na, &rc);
+  sb.sort.s4s = dbuf<double4>(c, B_S4S, na, &rc);
+  sb.sort.x32 = dbuf<float4>(c, B_X32S, na, &rc);
+  sb.sort.key = dbuf<int>(c, B_BOXKEY, na, &rc);
+  sb.sort.perm = dbuf<int>(c, B_PERMBOX, na, &rc);
+  sb.sort.tmp = dbuf<int>(c, B_BTMP, na, &rc);
+  sb.sort.starts = dbuf<int>(c, B_BOXSTART, b.n_boxes + 1, &rc);
+  sb.sort.counts = dbuf<int>(c, B_BCOUNTS, std::max(b.n_boxes, 1), &rc);
   sb.slot = dbuf<int4>(c, B_SLOT, na, &rc);
-  sb.btmp = dbuf<int>(c, B_BTMP, na, &rc);
-  sb.boxstart = dbuf<int>(c, B_BOXSTART, b.n_boxes + 1, &rc);
-  sb.bcounts = dbuf<int>(c, B_BCOUNTS, std::max(b.n_boxes, 1), &rc);
-  sb.bcursor = dbuf<int>(c, B_BCURSOR, std::max(b.n_boxes, 1), &rc);
-  sb.tcounts = dbuf<int>(c, B_COUNTS, std::max(b.n_tiles, 1), &rc);
-  sb.tcursor = dbuf<int>(c, B_CURSOR, std::max(b.n_tiles, 1), &rc);
-  sb.pairstart = dbuf<int>(c, B_PAIRSTART, b.n_tiles + 1, &rc);
-  sb.pairtmp = dbuf<int4>(c, B_PAIRTMP, std::max<size_t>(sp.pairs_max, 1), &rc);
-  sb.pairs = dbuf<int2>(c, B_PAIRS, std::max<size_t>(sp.pairs_max, 1), &rc);
+  sb.bins.counts = dbuf<int>(c, B_COUNTS, std::max(b.n_tiles, 1), &rc);
+  sb.bins.arrival = dbuf<int>(c, B_ARRIVAL, np, &rc);
+  sb.bins.starts = dbuf<int>(c, B_PAIRSTART, b.n_tiles + 1, &rc);
+  sb.bins.unordered = dbuf<int2>(c, B_PAIRTMP, np, &rc);
+  sb.bins.pairs = dbuf<int2>(c, B_PAIRS, np, &rc);
   sb.wtab = dbuf<char>(c, B_WTAB, na * sp.wstride * rs, &rc);
   sb.qk = dbuf<char>(c, B_QK, na * rs, &rc);
   sb.part = dbuf<double>(c, B_PART, na * sp.pstride * b.nparts, &rc);
@@ -974,40 +957,32 @@ int seg_prepare(ewg_context* c, SegPlan& sp, SegBufs& sb) {
 }
 
 // The stage sequence of a segmented batch (no host synchronisation, no
-// allocation): the real-space branch on the side stream beside the mesh chain.
+// allocation), all on the context's stream: every stage fills the GPU by itself, and
+// the real-space sum beside the mesh stages only kept their blocks waiting for its
+// own (128 cells 3437 us beside, 3271 us in line; mixed form, 96 cells, 3094 and
+// 2960 us).
 void seg_kernels(ewg_context* c, const SegPlan& sp, const SegBufs& sb, const double* coords,
                  const double* q, double* pot, double* force, int* cellerr) {
   const BatchLaunch& b = sp.b;
-  // With stage timing on, everything runs in line on the context's stream.
   Profiler* prof = &c->prof;
-  const bool concurrent = !prof->on;
-  cudaStream_t st = c->stream, rs = concurrent ? c->side : c->stream;
+  cudaStream_t st = c->stream;
   cudaMemsetAsync(cellerr, 0, sizeof(int) * std::max(b.ncells, 1), st);
   prof_mark(prof, st, ST_PREP);
-  launch_atom_prep_seg(b, coords, q, sb.s4, sb.boxkey, sb.mc, sb.fr, st);
-  launch_bucket_sort(sb.boxkey, b.n_atoms, b.n_boxes, sb.bcounts, sb.bcursor, sb.boxstart, sb.btmp,
-                     sb.perm, st);
-  if (concurrent) {
-    cudaEventRecord(c->fork, st);
-    cudaStreamWaitEvent(rs, c->fork, 0);
-  }
-  launch_permute_box_seg(b, sb.s4, sb.perm, sb.s4s, sb.x32, rs);
+  launch_atom_sort_seg(b, coords, q, sb.sort, sb.bins.counts, b.n_tiles, st);
   prof_mark(prof, st, ST_REAL);
-  launch_real_space_seg(b, sb.s4s, sb.x32, sb.perm, sb.boxstart, sb.pot_sr, sb.f_sr, cellerr, rs);
-  if (concurrent) cudaEventRecord(c->join, rs);
+  launch_real_space_seg(b, sb.sort.s4s, sb.sort.x32, sb.sort.perm, sb.sort.starts, sb.pot_sr,
+                        sb.f_sr, cellerr, st);
   prof_mark(prof, st, ST_WEIGHTS);
-  launch_weights_seg(b, sb.mc, sb.fr, sb.perm, sb.wtab, sb.qk, sb.slot, st);
-  launch_pair_bins_seg(b, sb.slot, sb.tcounts, sb.tcursor, sb.pairstart, sb.pairtmp, sb.pairs, st);
+  launch_weights_bins_seg(b, sb.sort.s4s, sb.wtab, sb.qk, sb.slot, sb.bins, st);
   prof_mark(prof, st, ST_SPREAD);
-  launch_spread_seg(b, sb.pairstart, sb.pairs, sb.wtab, sb.qk, st);
+  launch_spread_seg(b, sb.bins, sb.slot, sb.wtab, sb.qk, st);
   prof_mark(prof, st, ST_FFT_X_R2C);  // the three forward passes together
   launch_forward_and_weight_seg(b, st);
   prof_mark(prof, st, ST_FFT_Y_INV);  // both inverse passes together
   launch_inverse_seg(b, st);
   prof_mark(prof, st, ST_GATHER);
-  launch_gather_seg(b, sb.pairstart, sb.pairs, sb.wtab, sb.part, st);
-  if (concurrent) cudaStreamWaitEvent(st, c->join, 0);
-  launch_gather_final_seg(b, sb.slot, sb.perm, sb.part, q, sb.pot_sr, sb.f_sr, pot, force, st);
+  launch_gather_seg(b, sb.bins.starts, sb.bins.unordered, sb.wtab, sb.part, st);
+  launch_gather_final_seg(b, sb.slot, sb.sort.perm, sb.part, q, sb.pot_sr, sb.f_sr, pot, force, st);
   prof_mark(prof, st, -1);
 }
 
@@ -1833,7 +1808,6 @@ int ewg_direct_potential_force(ewg_context* c, int n, const double* positions,
   float4* x32s = dbuf<float4>(c, B_X32S, n, &rc);
   int* boxkey = dbuf<int>(c, B_BOXKEY, n, &rc);
   int* counts = dbuf<int>(c, B_COUNTS, nboxes, &rc);
-  int* cursor = dbuf<int>(c, B_CURSOR, nboxes, &rc);
   int* boxstart = dbuf<int>(c, B_BOXSTART, nboxes + 1, &rc);
   int* tmp = dbuf<int>(c, B_TMP, n, &rc);
   int* permbox = dbuf<int>(c, B_PERMBOX, n, &rc);
@@ -1853,9 +1827,8 @@ int ewg_direct_potential_force(ewg_context* c, int n, const double* positions,
     cudaMemcpyAsync(dwk, wk.data(), sizeof(double) * nk, cudaMemcpyHostToDevice, st);
   }
   cudaMemsetAsync(err, 0, sizeof(int), st);
-  launch_atom_prep(dcoords, 3, 1, dq, n, cell, rg.nb, nullptr, s4, boxkey, nullptr, nullptr, st);
-  launch_bucket_sort(boxkey, n, nboxes, counts, cursor, boxstart, tmp, permbox, st);
-  launch_permute_box(s4, permbox, n, cell.lat, s4s, x32s, st);
+  launch_atom_sort(dcoords, 3, 1, dq, n, cell, rg.nb,
+                   SortBufs{s4, boxkey, counts, tmp, boxstart, permbox, s4s, x32s}, nullptr, 0, st);
   launch_real_space(s4s, x32s, permbox, boxstart, n, rg, alpha, r_cut, 0, dpot, dforce, err, st);
   launch_structure_factors(dcoords, dq, n, dk, nk, dsk, st);
   launch_direct_kspace(dcoords, dq, n, dk, dwk, dsk, nk, dpot, dforce, st);
@@ -2204,35 +2177,29 @@ int points_mesh(ewg_context* c, const Cell& cell, double tol, int nt, const doub
   const MeshSizes mt = mesh_sizes(tgt.g, tgt.sd, 0, 1, nt, want_grad ? 4 : 1);
   const int spairs = ns * src.sd.S[0] * src.sd.S[1] * src.sd.S[2];
   const int tpairs = nt * tgt.sd.S[0] * tgt.sd.S[1] * tgt.sd.S[2];
-  double4* s4 = dbuf<double4>(c, B_PT_S4, ns, &rc);
+  double4* s4 = dbuf<double4>(c, B_PT_S4, nmax, &rc);
   double4* s4s = dbuf<double4>(c, B_PT_S4S, ns, &rc);
-  float4* x32 = dbuf<float4>(c, B_PT_X32, ns, &rc);
-  int* skey = dbuf<int>(c, B_PT_SKEY, ns, &rc);
+  double4* t4s = dbuf<double4>(c, B_PT_T4S, nt, &rc);
+  int* skey = dbuf<int>(c, B_PT_SKEY, nmax, &rc);
   int* sperm = dbuf<int>(c, B_PT_SPERM, ns, &rc);
   int* sbox = dbuf<int>(c, B_PT_SBOX, nboxes + 1, &rc);
-  int4* smc = dbuf<int4>(c, B_PT_SMC, ns, &rc);
-  double4* sfr = dbuf<double4>(c, B_PT_SFR, ns, &rc);
   void* swt = dbuf<char>(c, B_PT_SWT, ms.wtab, &rc);
   void* sqk = dbuf<char>(c, B_PT_SQK, ms.qk, &rc);
   int4* sslot = dbuf<int4>(c, B_PT_SSLOT, ns, &rc);
   int2* spairs_d = dbuf<int2>(c, B_PT_SPAIRS, spairs, &rc);
   int* spstart = dbuf<int>(c, B_PT_SPSTART, ntiles + 1, &rc);
-  int* tkey = dbuf<int>(c, B_PT_TKEY, nt, &rc);
   int* tperm = dbuf<int>(c, B_PT_TPERM, nt, &rc);
   int* tbox = dbuf<int>(c, B_PT_TBOX, nboxes + 1, &rc);
-  int4* tmc = dbuf<int4>(c, B_PT_TMC, nt, &rc);
-  double4* tfr = dbuf<double4>(c, B_PT_TFR, nt, &rc);
   void* twt = dbuf<char>(c, B_PT_TWT, mt.wtab, &rc);
   void* tqk = dbuf<char>(c, B_PT_TQK, mt.qk, &rc);
   int4* tslot = dbuf<int4>(c, B_PT_TSLOT, nt, &rc);
   int2* tpairs_d = dbuf<int2>(c, B_PT_TPAIRS, tpairs, &rc);
   int* tpstart = dbuf<int>(c, B_PT_TPSTART, ntiles + 1, &rc);
   int* bcnt = dbuf<int>(c, B_PT_BCNT, nboxes, &rc);
-  int* bcur = dbuf<int>(c, B_PT_BCUR, nboxes, &rc);
   int* btmp = dbuf<int>(c, B_PT_BTMP, nmax, &rc);
   int* kcnt = dbuf<int>(c, B_PT_KCNT, ntiles, &rc);
-  int* kcur = dbuf<int>(c, B_PT_KCUR, ntiles, &rc);
-  int4* ptmp = dbuf<int4>(c, B_PT_PTMP, std::max(spairs, tpairs), &rc);
+  int* parr = dbuf<int>(c, B_PT_PARR, std::max(spairs, tpairs), &rc);
+  int2* ptmp = dbuf<int2>(c, B_PT_PTMP, spairs, &rc);
   double* qneg = dbuf<double>(c, B_PT_QNEG, nt, &rc);
   double* part = dbuf<double>(c, B_PT_PART, mt.part / 8, &rc);
   double* potsr = dbuf<double>(c, B_PT_POTSR, nt, &rc);
@@ -2251,20 +2218,20 @@ int points_mesh(ewg_context* c, const Cell& cell, double tol, int nt, const doub
   // pot = real + mesh + shift and grad = real + sum_d D_d b_d.
   launch_fill(qneg, nt, -1.0, st);
   // Sources: box order for the real-space cell list and the mesh tables.
-  launch_atom_prep(ds, 3, 1, dq, ns, cell, rg.nb, src.g.n, s4, skey, smc, sfr, st);
-  launch_bucket_sort(skey, ns, nboxes, bcnt, bcur, sbox, btmp, sperm, st);
-  launch_permute_box(s4, sperm, ns, cell.lat, s4s, x32, st);
-  // Targets: the same box order, for locality in the gather.
-  launch_atom_prep(dt, 3, 1, qneg, nt, cell, rg.nb, tgt.g.n, nullptr, tkey, tmc, tfr, st);
-  launch_bucket_sort(tkey, nt, nboxes, bcnt, bcur, tbox, btmp, tperm, st);
+  const PairBins sbins{kcnt, parr, spstart, ptmp, spairs_d};
+  launch_atom_sort(ds, 3, 1, dq, ns, cell, rg.nb,
+                   SortBufs{s4, skey, bcnt, btmp, sbox, sperm, s4s, nullptr}, kcnt, ntiles, st);
   // Fourier sum: spread the sources, transform, weight, invert, gather.
-  launch_weights(src, smc, sfr, sperm, ns, swt, sqk, sslot, st);
-  launch_pair_bins(src, sslot, ns, kcnt, kcur, spstart, ptmp, spairs_d, spairs, st);
-  launch_spread(src, spstart, spairs_d, swt, sqk, grid, st);
+  launch_weights_bins(src, s4s, ns, swt, sqk, sslot, sbins, st);
+  launch_spread(src, sbins, sslot, ns, false, swt, sqk, grid, st);
   launch_forward_and_weight(src, grid, A1, A2, B2, 1, st, nullptr);
   launch_inverse(src, B2, B1, outg, 1, st);
-  launch_weights(tgt, tmc, tfr, tperm, nt, twt, tqk, tslot, st);
-  launch_pair_bins(tgt, tslot, nt, kcnt, kcur, tpstart, ptmp, tpairs_d, tpairs, st);
+  // Targets: the same box order, for locality in the gather, which takes the pairs
+  // in any order.
+  launch_atom_sort(dt, 3, 1, qneg, nt, cell, rg.nb,
+                   SortBufs{s4, skey, bcnt, btmp, tbox, tperm, t4s, nullptr}, kcnt, ntiles, st);
+  launch_weights_bins(tgt, t4s, nt, twt, tqk, tslot, PairBins{kcnt, parr, tpstart, tpairs_d, nullptr},
+                      st);
   launch_gather(tgt, tpstart, tpairs_d, twt, outg, 1, part, st);
   // Real-space sum over the source cell list.
   PointsReal pr;
@@ -2504,7 +2471,6 @@ int ewg_stress(ewg_context* c, double tol_ewald, double alpha, double* sigma) {
   float4* x32s = dbuf<float4>(c, B_X32S, n, &rc);
   int* boxkey = dbuf<int>(c, B_BOXKEY, n, &rc);
   int* counts = dbuf<int>(c, B_COUNTS, nboxes, &rc);
-  int* cursor = dbuf<int>(c, B_CURSOR, nboxes, &rc);
   int* boxstart = dbuf<int>(c, B_BOXSTART, nboxes + 1, &rc);
   int* tmp = dbuf<int>(c, B_TMP, n, &rc);
   int* permbox = dbuf<int>(c, B_PERMBOX, n, &rc);
@@ -2522,9 +2488,8 @@ int ewg_stress(ewg_context* c, double tol_ewald, double alpha, double* sigma) {
   if (ng) cudaMemcpyAsync(dk, ss.g.data(), sizeof(double) * ss.g.size(), cudaMemcpyHostToDevice, st);
   cudaMemsetAsync(err, 0, sizeof(int), st);
   c->resident.coords_version = -1;  // the sorted layout below is for max_r
-  launch_atom_prep(dcoords, 3, 1, dq, n, cell, rg.nb, nullptr, s4, boxkey, nullptr, nullptr, st);
-  launch_bucket_sort(boxkey, n, nboxes, counts, cursor, boxstart, tmp, permbox, st);
-  launch_permute_box(s4, permbox, n, cell.lat, s4s, x32s, st);
+  launch_atom_sort(dcoords, 3, 1, dq, n, cell, rg.nb,
+                   SortBufs{s4, boxkey, counts, tmp, boxstart, permbox, s4s, x32s}, nullptr, 0, st);
   launch_real_stress(s4s, x32s, boxstart, n, rg, ss.alpha, ss.max_r, p6, o6, err, st);
   launch_structure_factors(dcoords, dq, n, dk, ng, dsk, st);
   launch_recip_stress(dk, dsk, ng, ss.alpha, p6, o6 + 6, st);

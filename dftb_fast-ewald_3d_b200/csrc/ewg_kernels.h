@@ -65,28 +65,28 @@ void prof_collect(Profiler* p);
 
 // ---- atoms: fractional coordinates, keys, sorting (ewg_real.cu) ----------
 
-// Per atom: wrapped fractional coordinates s and charge (double4), real-space
-// box key, mesh lowest point and fraction (nfft/nfft.f90:122-159).  Null
-// outputs (and null nb / ngrid) are skipped.
-// positions: element (i, d) at pos[i * sa + d * sd].
-void launch_atom_prep(const double* pos, long sa, long sd, const double* q, int n, const Cell& cell,
-                      const int nb[3], const int ngrid[3], double4* s4, int* box_key, int4* mesh_c,
-                      double4* mesh_fr, cudaStream_t st);
-
-// Stable counting sort by key: perm[k] = atom with the k-th key in (key, index)
-// order; starts[nkeys + 1] are bucket offsets.  Scratch: counts/cursor (nkeys),
-// tmp (n).
-void launch_bucket_sort(const int* key, int n, int nkeys, int* counts, int* cursor, int* starts,
-                        int* tmp, int* perm, cudaStream_t st);
+// Buffers of the box sort.  Scratch: counts and key (not used by small cells),
+// s4 (unsorted atoms, likewise), tmp.  Results: starts[nboxes + 1], perm (sorted
+// atom k is atom perm[k]; (box, index) order), s4s (wrapped fractional coordinates
+// and charge), x32 (Cartesian position s . lat and charge in FP32; may be null).
+struct SortBufs {
+  double4* s4;
+  int *key, *counts, *tmp;
+  int *starts, *perm;
+  double4* s4s;
+  float4* x32;
+};
+// Atom preparation and deterministic box sort; positions: element (i, d) at
+// pos[i * sa + d * sd].  zero[0..nzero) is cleared on the way.
+void launch_atom_sort(const double* pos, long sa, long sd, const double* q, int n, const Cell& cell,
+                      const int nb[3], const SortBufs& b, int* zero, int nzero, cudaStream_t st);
+// New charges on an unchanged geometry: the charges in s4s, x32 and qk.
+void launch_refresh_charges(const double* q, const int* perm, int n, double4* s4s, float4* x32,
+                            void* qk, int mixed, cudaStream_t st);
 
 // Exclusive scan of counts[0..nkeys) into starts[0..nkeys] (one CTA), chained
 // to the stream's previous kernel when after_kernel.
 void launch_scan(const int* counts, int nkeys, int* starts, bool after_kernel, cudaStream_t st);
-
-// Box-sorted atoms: out[k] = in[perm[k]] (fractional s, q) and x32[k] the
-// Cartesian position s . lat with q, in FP32, for the real-space distance test.
-void launch_permute_box(const double4* in, const int* perm, int n, const double (*lat)[3],
-                        double4* out, float4* x32, cudaStream_t st);
 
 // Charge sums for the parameter chain on device-resident charges:
 // out[0] = sum q, out[1] = sum |q|, out[2] = sum q^2 (fixed-order reduction).
@@ -162,6 +162,14 @@ struct MeshPlan {
                                   // cores on FP32 data, 2 FP32 CUDA cores
   Profiler* prof = nullptr;
   const double* corr2[3] = {nullptr, nullptr, nullptr};  // squared deconvolution factors, index k + H
+};
+
+// (atom, tile) pairs: entry (atom, packed slot) of tile t in [starts[t],
+// starts[t+1]).  counts (one per tile) and arrival (one per atom and slot) are
+// scratch; pairs is the ordered copy that long lists and the FP32 spread use.
+struct PairBins {
+  int *counts, *arrival, *starts;
+  int2 *unordered, *pairs;
 };
 
 // ---- segmented launches of the batched form --------------------------------
@@ -246,8 +254,7 @@ struct BatchLaunch {
   const BatchCell* cells = nullptr;
   int ncells = 0;
   int mixed = 0, nc = 1, nparts = 1, ad = 0;
-  int any_kb = 0, any_gauss = 0;  // windows that occur among the cells
-  int wstride = 0;                // weight values per atom, common to the cells
+  int wstride = 0, pstride = 0;   // weight values and partial slots per atom, common to the cells
   int L = 1;           // FFT lines per CTA, one value for every cell
   int uniform[3] = {0, 0, 0};  // every cell has the same length along this axis
   FftPlan plan[3];             // that length's plan (when uniform)
@@ -271,19 +278,14 @@ struct BatchLaunch {
 };
 
 // Segmented counterparts of the single-cell launchers (same work per cell).
-void launch_atom_prep_seg(const BatchLaunch& b, const double* coords3n, const double* q,
-                          double4* s4, int* box_key, int4* mesh_c, double4* mesh_fr,
-                          cudaStream_t st);
-void launch_permute_box_seg(const BatchLaunch& b, const double4* in, const int* perm,
-                            double4* out, float4* x32, cudaStream_t st);
+void launch_atom_sort_seg(const BatchLaunch& bl, const double* coords3n, const double* q,
+                          const SortBufs& b, int* zero, int nzero, cudaStream_t st);
 void launch_real_space_seg(const BatchLaunch& b, const double4* s4s, const float4* x32,
                            const int* perm, const int* box_start, double* pot, double* force,
                            int* cell_err, cudaStream_t st);
-void launch_weights_seg(const BatchLaunch& b, const int4* mesh_c, const double4* mesh_fr,
-                        const int* perm, void* wtab, void* qk, int4* slot, cudaStream_t st);
-void launch_pair_bins_seg(const BatchLaunch& b, const int4* slot, int* counts, int* cursor,
-                          int* tile_start, int4* tmp, int2* pairs, cudaStream_t st);
-void launch_spread_seg(const BatchLaunch& b, const int* tile_start, const int2* pairs,
+void launch_weights_bins_seg(const BatchLaunch& b, const double4* s4s, void* wtab, void* qk,
+                             int4* slot, const PairBins& pb, cudaStream_t st);
+void launch_spread_seg(const BatchLaunch& b, const PairBins& pb, const int4* slot,
                        const void* wtab, const void* qk, cudaStream_t st);
 void launch_forward_and_weight_seg(const BatchLaunch& b, cudaStream_t st);
 void launch_inverse_seg(const BatchLaunch& b, cudaStream_t st);
@@ -303,28 +305,19 @@ void mesh_pass_blocks(const MeshGeom& g, int L, int nc, int out[5]);
 size_t mesh_pass_smem(int n, int L, bool mixed, int extra);
 
 // Tiled window weights per sorted atom (wtab: wstride values per atom), slot
-// origin and count per axis (slot: first | count << 16 in x, y, z), and the
-// charges in sorted order (qk).  mesh_c / mesh_fr are in atom order and are
-// read through the permutation (sorted atom k is atom perm[k]; the cell-list
-// box order, which keeps neighbouring atoms close in the tables).
-void launch_weights(const MeshPlan& mp, const int4* mesh_c, const double4* mesh_fr,
-                    const int* perm, int n, void* wtab, void* qk, int4* slot, cudaStream_t st);
-
-// Only the charges in sorted order, qk[k] = q[perm[k]] (FP32 in the mixed form):
-// the resident path's refresh when the geometry and so the weights and the
-// pair lists are unchanged.
-void launch_sorted_charges(const MeshPlan& mp, const double* q, const int* perm, int n, void* qk,
-                           cudaStream_t st);
-
-// Bins every (atom, tile) pair by tile, buckets ordered by atom index:
-// pairs[tile_start[t] .. tile_start[t+1]) = (atom, packed slot).  Scratch:
-// counts/cursor (ntiles), tmp (npairs_max); npairs_max = n * S_x * S_y * S_z.
-void launch_pair_bins(const MeshPlan& mp, const int4* slot, int n, int* counts, int* cursor,
-                      int* tile_start, int4* tmp, int2* pairs, int npairs_max, cudaStream_t st);
+// origin and count per axis (slot: first | count << 16 in x, y, z), the charges in
+// sorted order (qk), and the (atom, tile) pairs binned by tile in no fixed order
+// (b.counts zero on entry).  s4s: the sorted atoms (the cell-list box order keeps
+// neighbouring atoms close in the tables).  The stream's previous operation must be
+// a kernel.
+void launch_weights_bins(const MeshPlan& mp, const double4* s4s, int n, void* wtab, void* qk,
+                         int4* slot, const PairBins& b, cudaStream_t st);
 
 // Tile-owned deterministic spread (adjoint_nfft_3d step 1, nfft/nfft.f90:253-278).
-void launch_spread(const MeshPlan& mp, const int* tile_start, const int2* pairs, const void* wtab,
-                   const void* qk, void* grid, cudaStream_t st);
+// It takes each tile's list in order of the atoms; ordered: an earlier call with the
+// same bins has put the lists that need it into b.pairs.
+void launch_spread(const MeshPlan& mp, const PairBins& b, const int4* slot, int n, bool ordered,
+                   const void* wtab, const void* qk, void* grid, cudaStream_t st);
 
 // Pruned forward transform of the real grid to the compact spectrum, fused with
 // the influence weights and the first inverse pass: grid -> A1 -> A2 -> B2.

@@ -267,7 +267,7 @@ extern "C" int ewg_direct_potential_force_static(int n, const double* coords_dev
   float4* x32s = cv.take<float4>(n);
   int* boxkey = cv.take<int>(n);
   int* counts = cv.take<int>(nboxes);
-  int* cursor = cv.take<int>(nboxes);
+  cv.take<int>(nboxes);  // part of the documented limit
   int* starts = cv.take<int>(nboxes + 1);
   int* tmp = cv.take<int>(n);
   int* perm = cv.take<int>(n);
@@ -276,10 +276,8 @@ extern "C" int ewg_direct_potential_force_static(int n, const double* coords_dev
   if (!cv.fits()) return EWG_ERR_SCRATCH_LIMIT;
 
   cudaMemsetAsync(err, 0, sizeof(int), st);
-  launch_atom_prep(coords_device, 3, 1, charges_device, n, cell, rg.nb, nullptr, s4, boxkey,
-                   nullptr, nullptr, st);
-  launch_bucket_sort(boxkey, n, nboxes, counts, cursor, starts, tmp, perm, st);
-  launch_permute_box(s4, perm, n, cell.lat, s4s, x32s, st);
+  launch_atom_sort(coords_device, 3, 1, charges_device, n, cell, rg.nb,
+                   SortBufs{s4, boxkey, counts, tmp, starts, perm, s4s, x32s}, nullptr, 0, st);
   launch_real_space(s4s, x32s, perm, starts, n, rg, alpha, r_cut, 0, pot_device, fbuf, err, st);
   k_modes_box<<<static_cast<unsigned>(nmodes), 256, 0, st>>>(coords_device, charges_device, n, mb,
                                                              modes);

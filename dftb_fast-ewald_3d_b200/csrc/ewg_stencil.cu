@@ -70,46 +70,56 @@ __device__ __forceinline__ void store_row(double* out, const double (&v)[8]) {
 __device__ __forceinline__ int slot_first(int packed) { return packed & 0xffff; }
 __device__ __forceinline__ int slot_count(int packed) { return packed >> 16; }
 
+// Mesh stencil origin of a wrapped fractional coordinate: lowest grid point
+// floor(s n) (mod n) and the fraction s n - lowest (nfft/nfft.f90:148-152).
+__device__ __forceinline__ int lowest_point(double s, int n, double* frac) {
+  const double scaled = s * n;
+  const int lowest = static_cast<int>(floor(scaled));
+  *frac = scaled - static_cast<double>(lowest);
+  return lowest >= n ? lowest - n : lowest;
+}
+
+// Tiles the stencil [c + lo, c + lo + W - 1] (mod n) runs through, starting at
+// `first`; a stencil that comes back into its first tile, or covers the whole
+// axis, touches every tile once (repeated points are folded into the weights).
+__device__ __forceinline__ void stencil_tiles(int c, const StencilDims& sd, int d, int* first,
+                                              int* count) {
+  const int nd = sd.n[d], nt = sd.ntiles[d];
+  if (sd.W >= nd) {
+    *first = 0;
+    *count = nt;
+    return;
+  }
+  const int p0 = pmod(c + sd.lo, nd);
+  int t = p0 / kTileX;
+  *first = t;
+  int covered = min((t + 1) * kTileX, nd) - p0, m = 1;
+  while (covered < sd.W) {
+    t = t + 1 == nt ? 0 : t + 1;
+    ++m;
+    covered += min((t + 1) * kTileX, nd) - t * kTileX;
+  }
+  *count = min(m, nt);
+}
+
 // ---------------------------------------------------------------------------
-// Tiled window weights, one thread per (atom, axis, tile slot): eight points
-// each, so an atom's S_x + S_y + S_z rows are computed in parallel.
+// Tiled window weights of wide windows (rows beyond kAxisRow values per atom),
+// one thread per (atom, axis, tile slot), eight points each.
 // ---------------------------------------------------------------------------
 // Row r (axis and slot) of sorted atom k.
 template <typename R>
-__device__ __forceinline__ void weights_row(const int4* __restrict__ mc,
-                                            const double4* __restrict__ fr,
-                                            const int* __restrict__ perm, int k, int r,
+__device__ __forceinline__ void weights_row(const double4* __restrict__ s4s, int k, int r,
                                             const StencilDims& sd, R* __restrict__ wtab,
                                             R* __restrict__ qk, int4* __restrict__ slot) {
   const int d = r < sd.S[0] ? 0 : (r < sd.S[0] + sd.S[1] ? 1 : 2);
   const int s = r - (d == 0 ? 0 : (d == 1 ? sd.S[0] : sd.S[0] + sd.S[1]));
-  const int i = perm[k];
-  const int4 c4 = mc[i];
-  const double4 f4 = fr[i];
-  const int c = d == 0 ? c4.x : (d == 1 ? c4.y : c4.z);
-  const double frac = d == 0 ? f4.x : (d == 1 ? f4.y : f4.z);
+  const double4 s4 = s4s[k];
   const int nd = sd.n[d], T = sd.T[d], nt = sd.ntiles[d];
+  double frac;
+  const int c = lowest_point(d == 0 ? s4.x : (d == 1 ? s4.y : s4.z), nd, &frac);
   const int lo = sd.lo, hi = sd.lo + sd.W - 1, W = sd.W;
-  // Tiles the stencil [c + lo, c + hi] (mod n) runs through, starting at `first`;
-  // a stencil that comes back into its first tile, or covers the whole axis,
-  // touches every tile once (repeated points are folded into the weights).
   int first, count;
-  if (W >= nd) {
-    first = 0;
-    count = nt;
-  } else {
-    const int p0 = pmod(c + lo, nd);
-    int t = p0 / T;
-    first = t;
-    int covered = min((t + 1) * T, nd) - p0;
-    count = 1;
-    while (covered < W) {
-      t = t + 1 == nt ? 0 : t + 1;
-      ++count;
-      covered += min((t + 1) * T, nd) - t * T;
-    }
-    count = min(count, nt);
-  }
+  stencil_tiles(c, sd, d, &first, &count);
   R* out = wtab + static_cast<size_t>(k) * sd.wstride + sd.woff[d] + s * T;
   // Window derivative with respect to the atom's fractional coordinate s_d:
   // the point sits at u = o - frac grid units from the atom, and
@@ -161,13 +171,12 @@ __device__ __forceinline__ void weights_row(const int4* __restrict__ mc,
   sp[d] = first | (count << 16);
   if (d == 0) {
     sp[3] = 0;
-    qk[k] = static_cast<R>(f4.w);
+    qk[k] = static_cast<R>(s4.w);
   }
 }
 
 template <typename R>
-__global__ void k_weights_tiled(const int4* __restrict__ mc, const double4* __restrict__ fr,
-                                const int* __restrict__ perm, int n, StencilDims sd,
+__global__ void k_weights_tiled(const double4* __restrict__ s4s, int n, StencilDims sd,
                                 R* __restrict__ wtab, R* __restrict__ qk,
                                 int4* __restrict__ slot) {
   chain_enter();
@@ -175,8 +184,7 @@ __global__ void k_weights_tiled(const int4* __restrict__ mc, const double4* __re
   const long idx = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= static_cast<long>(SS) * n) return;
   const int k = static_cast<int>(idx / SS);
-  weights_row<R>(mc, fr, perm, k, static_cast<int>(idx - static_cast<long>(k) * SS), sd, wtab, qk,
-                 slot);
+  weights_row<R>(s4s, k, static_cast<int>(idx - static_cast<long>(k) * SS), sd, wtab, qk, slot);
 }
 
 // Every cell of a batch: item idx is (atom, row) of its cell (prefix over the
@@ -184,8 +192,7 @@ __global__ void k_weights_tiled(const int4* __restrict__ mc, const double4* __re
 // per-atom stride.
 template <typename R>
 __global__ void k_weights_seg(const BatchCell* __restrict__ cells, const int* __restrict__ prefix,
-                              int ncells, long nitems, const int4* __restrict__ mc,
-                              const double4* __restrict__ fr, const int* __restrict__ perm,
+                              int ncells, long nitems, const double4* __restrict__ s4s,
                               R* __restrict__ wtab, R* __restrict__ qk, int4* __restrict__ slot) {
   chain_enter();
   const long idx = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -193,165 +200,18 @@ __global__ void k_weights_seg(const BatchCell* __restrict__ cells, const int* __
   const int c = seg_cell(prefix, ncells, idx);
   const BatchCell& bc = cells[c];
   const StencilDims sd = bc.sd;
-  if (sd.kb) return;  // k_weights_kb_seg
   const int SS = sd.S[0] + sd.S[1] + sd.S[2];
   const int local = static_cast<int>(idx - prefix[c]);
   const int kl = local / SS;
-  weights_row<R>(mc, fr, perm, bc.atom0 + kl, local - kl * SS, sd, wtab, qk, slot);
+  weights_row<R>(s4s, bc.atom0 + kl, local - kl * SS, sd, wtab, qk, slot);
 }
 
-// ---------------------------------------------------------------------------
-// Kaiser-Bessel weights (plain form).  A warp takes one axis of 32 atoms, a lane
-// one atom: the W = 14 weights are polynomials in the atom's fraction with the
-// same coefficients for every lane, read as constant operands, so the 14 x 15
-// multiply-adds of a lane need no memory access.  (Evaluated row by row in the
-// layout above, neighbouring lanes would need different polynomials and so
-// gather their coefficients.)  The values go to the tiled rows through shared
-// memory, from where the CTA writes the rows of its 32 atoms, a contiguous piece
-// of the table, with full 16-byte stores.  Bounded by those stores (576 B per
-// atom): at 32,769 atoms 18.9 MB.
-// ---------------------------------------------------------------------------
-constexpr int kKbCoefs = kKbDegree + 1;
-constexpr int kKbAtoms = 32;              // atoms per CTA, one warp per axis
-constexpr int kKbRow = 3 * 3 * kTileX;    // most values of an atom's three axes
-__constant__ double c_kb[kKbWidth * kKbCoefs];
-
-// Shared values per atom: the rows (and, for ad, derivative rows) plus padding
-// that spreads the lanes over the banks and keeps rows 16-byte aligned.
-__host__ __device__ constexpr int kb_pitch(int ad) { return (ad ? 2 : 1) * kKbRow + 2; }
-
-// The weights of sorted atom k along axis d into its shared row w (derivative
-// rows dw, null without them), and its slot record.
-__device__ __forceinline__ void kb_axis(const int4* __restrict__ mc,
-                                        const double4* __restrict__ fr,
-                                        const int* __restrict__ perm, int k, int d,
-                                        const StencilDims& sd, double* __restrict__ w,
-                                        double* __restrict__ dw, double* __restrict__ qk,
-                                        int4* __restrict__ slot) {
-  const int i = perm[k];
-  const int4 c4 = mc[i];
-  const double4 f4 = fr[i];
-  const int c = d == 0 ? c4.x : (d == 1 ? c4.y : c4.z);
-  const double frac = d == 0 ? f4.x : (d == 1 ? f4.y : f4.z);
-  const int nd = sd.n[d], nt = sd.ntiles[d];
-  int p0 = c + kKbLow;
-  if (p0 < 0) p0 += nd;
-  const int first = p0 / kTileX;
-  // Whole tiles of 8 points: the stencil covers (p0 mod 8) + 14 row points.
-  const int row0 = p0 - first * kTileX;
-  const int count = min((row0 + kKbWidth + kTileX - 1) / kTileX, nt);
-  const double t = 2.0 * frac - 1.0;
-  const double dscale = 2.0 * static_cast<double>(nd);  // dt/ds_d
-  const int span = nt * kTileX;
-  double* out = w + sd.woff[d];
-#pragma unroll
-  for (int j = 0; j < kKbWidth; ++j) {
-    const double* cf = c_kb + j * kKbCoefs;
-    double v = cf[kKbDegree], dv = 0.0;
-#pragma unroll
-    for (int e = kKbDegree - 1; e >= 0; --e) {
-      if (dw) dv = fma(dv, t, v);
-      v = fma(v, t, cf[e]);
-    }
-    int r = row0 + j;
-    if (r >= span) r -= span;  // back in the first tile (nt = 2)
-    out[r] = v;
-    if (dw) dw[sd.woff[d] + r] = dscale * dv;
-  }
-  int* sp = reinterpret_cast<int*>(&slot[k]);
-  sp[d] = first | (count << 16);
-  if (d == 0) {
-    sp[3] = 0;
-    qk[k] = f4.w;
-  }
-}
-
-// Zeroes the CTA's shared rows, fills them and writes each row's first
-// rowlen(k) values (0: not a row of this window) to the table.
-template <class Fill, class RowLen>
-__device__ __forceinline__ void kb_rows(double* sm, int pitch, int k0, int n, int wstride,
-                                        double* __restrict__ wtab, Fill fill, RowLen rowlen) {
-  __shared__ int len[kKbAtoms];
-  const int lane = threadIdx.x & 31, d = threadIdx.x >> 5;
-  for (int e = threadIdx.x; e < kKbAtoms * pitch; e += 3 * 32) sm[e] = 0.0;
-  if (threadIdx.x < kKbAtoms) len[threadIdx.x] = k0 + lane < n ? rowlen(k0 + lane) : 0;
-  __syncthreads();
-  if (len[lane]) fill(k0 + lane, d, sm + lane * pitch);
-  __syncthreads();
-  const int half = pitch / 2;
-  for (int e = threadIdx.x; e < kKbAtoms * half; e += 3 * 32) {
-    const int a = e / half, v = 2 * (e - a * half);
-    if (v < len[a])
-      *reinterpret_cast<double2*>(wtab + static_cast<size_t>(k0 + a) * wstride + v) =
-          *reinterpret_cast<const double2*>(sm + a * pitch + v);
-  }
-}
-
-template <bool AD>
-__global__ void __launch_bounds__(96) k_weights_kb(const int4* __restrict__ mc,
-                                                   const double4* __restrict__ fr,
-                                                   const int* __restrict__ perm, int n,
-                                                   StencilDims sd, double* __restrict__ wtab,
-                                                   double* __restrict__ qk,
-                                                   int4* __restrict__ slot) {
-  chain_enter();
-  __shared__ __align__(16) double sm[kKbAtoms * kb_pitch(AD)];
-  kb_rows(
-      sm, kb_pitch(AD), blockIdx.x * kKbAtoms, n, sd.wstride, wtab,
-      [&](int k, int d, double* row) {
-        kb_axis(mc, fr, perm, k, d, sd, row, AD ? row + sd.dwoff : nullptr, qk, slot);
-      },
-      [&](int) { return sd.wstride; });
-}
-
-// Every cell of a batch; rows of cells with a Gaussian window are k_weights_seg's.
-template <bool AD>
-__global__ void __launch_bounds__(96) k_weights_kb_seg(
-    const BatchCell* __restrict__ cells, const int* __restrict__ atom_prefix, int ncells, int n,
-    int wstride, const int4* __restrict__ mc, const double4* __restrict__ fr,
-    const int* __restrict__ perm, double* __restrict__ wtab, double* __restrict__ qk,
-    int4* __restrict__ slot) {
-  chain_enter();
-  __shared__ __align__(16) double sm[kKbAtoms * kb_pitch(AD)];
-  kb_rows(
-      sm, kb_pitch(AD), blockIdx.x * kKbAtoms, n, wstride, wtab,
-      [&](int k, int d, double* row) {
-        const StencilDims sd = cells[seg_cell(atom_prefix, ncells, k)].sd;
-        kb_axis(mc, fr, perm, k, d, sd, row, AD ? row + sd.dwoff : nullptr, qk, slot);
-      },
-      [&](int k) {
-        const StencilDims& sd = cells[seg_cell(atom_prefix, ncells, k)].sd;
-        return sd.kb ? (AD ? 2 : 1) * sd.dwoff : 0;
-      });
-}
-
-// ---------------------------------------------------------------------------
-// (atom, tile) pair binning.
-// ---------------------------------------------------------------------------
-template <class F>
-__device__ __forceinline__ void for_each_tile(const int4& si, const StencilDims& sd, F f) {
-  const int cx = slot_count(si.x), cy = slot_count(si.y), cz = slot_count(si.z);
-  const int fx = slot_first(si.x), fy = slot_first(si.y), fz = slot_first(si.z);
-  for (int sz = 0; sz < cz; ++sz) {
-    const int tz = (fz + sz) % sd.ntiles[2];
-    for (int sy = 0; sy < cy; ++sy) {
-      const int ty = (fy + sy) % sd.ntiles[1];
-      for (int sx = 0; sx < cx; ++sx) {
-        const int tx = (fx + sx) % sd.ntiles[0];
-        f((tz * sd.ntiles[1] + ty) * sd.ntiles[0] + tx, sx | (sy << 8) | (sz << 16));
-      }
-    }
-  }
-}
-
-// One thread per (atom, slot of the S_x x S_y x S_z block); slots past the
-// atom's own tile counts are skipped.
-// Slot s of sorted atom k: its tile (the cell's own numbering) and packed
-// slot, false for slots past the atom's tile counts.
-__device__ __forceinline__ bool pair_of(const int4* __restrict__ slot, int k, int s,
-                                        const StencilDims& sd, int* tile, int* packed) {
+// Slot s of the S_x x S_y x S_z block of an atom with slot record si: its tile
+// (the cell's own numbering) and packed slot; false for slots past the atom's own
+// tile counts.
+__device__ __forceinline__ bool pair_of(const int4& si, int s, const StencilDims& sd, int* tile,
+                                        int* packed) {
   const int sx = s % sd.S[0], sy = (s / sd.S[0]) % sd.S[1], sz = s / (sd.S[0] * sd.S[1]);
-  const int4 si = slot[k];
   if (sx >= slot_count(si.x) || sy >= slot_count(si.y) || sz >= slot_count(si.z)) return false;
   const int tx = (slot_first(si.x) + sx) % sd.ntiles[0];
   const int ty = (slot_first(si.y) + sy) % sd.ntiles[1];
@@ -361,6 +221,181 @@ __device__ __forceinline__ bool pair_of(const int4* __restrict__ slot, int k, in
   return true;
 }
 
+// ---------------------------------------------------------------------------
+// Tiled window weights, a warp per axis of 32 atoms, a lane per atom, and the
+// counts of the (atom, tile) pairs.
+//
+// A lane evaluates exactly the W points of its stencil: the Kaiser-Bessel
+// weights as polynomials in the atom's fraction with the same coefficients for
+// every lane, constant operands without a memory access; the Gaussian by its
+// exponential.  (One thread per row of 8 points evaluated 24 or 32 points for 13 to
+// 25, and neighbouring lanes would gather different polynomials.)  The values go
+// to the tiled rows through shared memory, from where the CTA writes the rows of
+// its atoms, a contiguous piece of the table, with 16-byte stores; those bound it
+// (576 B per atom and 14 points in FP64).  Then the CTA counts its atoms' tiles
+// and keeps each pair's arrival number in its tile, which saves a launch and the
+// scatter its own round of atomics.
+// ---------------------------------------------------------------------------
+constexpr int kKbCoefs = kKbDegree + 1;
+constexpr int kAxisAtoms = 32;    // atoms per CTA
+constexpr int kAxisRow = 200;     // most values per atom (windows up to m = 12, ad): 52 KB of rows
+__constant__ double c_kb[kKbWidth * kKbCoefs];
+
+// Shared values per atom: the rows (and, for ad, derivative rows) plus padding
+// that spreads the lanes over the banks and keeps rows 16-byte aligned.
+__host__ __device__ constexpr int axis_pitch(int row) { return row + 2; }
+
+// The weights of an atom with fractional coordinate s along axis d into its shared
+// row w, zeroed before (with sd.ad the derivatives dwoff further on); returns the
+// slot record.
+__device__ __forceinline__ int axis_weights(double s, int d, const StencilDims& sd,
+                                            double* __restrict__ w) {
+  const int nd = sd.n[d], nt = sd.ntiles[d];
+  double frac;
+  const int c = lowest_point(s, nd, &frac);
+  int first, count;
+  stencil_tiles(c, sd, d, &first, &count);
+  double* out = w + sd.woff[d];
+  if (sd.kb) {  // more points than the window is wide, in whole tiles
+    int p0 = c + kKbLow;
+    if (p0 < 0) p0 += nd;
+    const int row0 = p0 - first * kTileX;
+    const double t = 2.0 * frac - 1.0;
+    const double dscale = 2.0 * static_cast<double>(nd);  // dt/ds_d
+#pragma unroll
+    for (int j = 0; j < kKbWidth; ++j) {
+      const double* cf = c_kb + j * kKbCoefs;
+      double v = cf[kKbDegree], dv = 0.0;
+#pragma unroll
+      for (int e = kKbDegree - 1; e >= 0; --e) {
+        if (sd.ad) dv = fma(dv, t, v);
+        v = fma(v, t, cf[e]);
+      }
+      int r = row0 + j;
+      if (r >= nd) r -= nd;  // back in the first tile (nt = 2)
+      out[r] = v;
+      if (sd.ad) out[sd.dwoff + r] = dscale * dv;
+    }
+  } else {
+    // d/ds_d [pref exp(-u^2 / b)] = n_d (2 u / b) pref exp(-u^2 / b) at u = o - frac.
+    const double dscale = -2.0 * static_cast<double>(nd) / sd.b;
+    int o = sd.lo + sd.W - 1;
+    int p = pmod(c + o, nd);
+    for (; o >= sd.lo; --o) {
+      const double dd = frac - static_cast<double>(o);
+      const double e = sd.pref * exp(-(dd * dd) / sd.b);
+      const int t = p / kTileX;
+      int sl = t - first;
+      if (sl < 0) sl += nt;
+      const int r = sl * kTileX + (p - t * kTileX);
+      out[r] += e;  // a point that the stencil reaches again carries the sum
+      if (sd.ad) out[sd.dwoff + r] += dscale * dd * e;
+      p = p == 0 ? nd - 1 : p - 1;
+    }
+  }
+  return first | (count << 16);
+}
+
+// Row values as the table's type, 16 bytes at a time (rows are multiples of 8 values).
+__device__ __forceinline__ void copy_row(double* __restrict__ dst, const double* __restrict__ src,
+                                         int v) {
+  *reinterpret_cast<double2*>(dst + v) = *reinterpret_cast<const double2*>(src + v);
+}
+__device__ __forceinline__ void copy_row(float* __restrict__ dst, const double* __restrict__ src,
+                                         int v) {
+  *reinterpret_cast<float4*>(dst + v) =
+      make_float4(static_cast<float>(src[v]), static_cast<float>(src[v + 1]),
+                  static_cast<float>(src[v + 2]), static_cast<float>(src[v + 3]));
+}
+
+// dims(k): the stencil geometry of atom k; pairs0(k): the atom's first place in
+// arrival; tile0(k): its cell's first tile.
+template <typename R, class Dims, class Pairs0, class Tile0>
+__device__ __forceinline__ void weights_axis_body(double* __restrict__ sm, int row, int wstride,
+                                                  int pstride, const double4* __restrict__ s4s,
+                                                  int n, R* __restrict__ wtab,
+                                                  R* __restrict__ qk, int4* __restrict__ slot,
+                                                  int* __restrict__ tile_counts,
+                                                  int* __restrict__ arrival, Dims dims,
+                                                  Pairs0 pairs0, Tile0 tile0) {
+  __shared__ int sslot[3][kAxisAtoms];
+  const int lane = threadIdx.x & 31, d = threadIdx.x >> 5;
+  const int k0 = blockIdx.x * kAxisAtoms, na = min(kAxisAtoms, n - k0);
+  const int pitch = axis_pitch(row);
+  for (int e = threadIdx.x; e < kAxisAtoms * pitch; e += 96) sm[e] = 0.0;
+  __syncthreads();
+  if (lane < na) {
+    const double4 s4 = s4s[k0 + lane];
+    sslot[d][lane] = axis_weights(d == 0 ? s4.x : (d == 1 ? s4.y : s4.z), d, dims(k0 + lane),
+                                  sm + lane * pitch);
+    if (d == 0) qk[k0 + lane] = static_cast<R>(s4.w);
+  }
+  __syncthreads();
+  constexpr int kVec = 16 / sizeof(R);
+  const int chunks = row / kVec;
+  for (int e = threadIdx.x; e < na * chunks; e += 96) {
+    const int a = e / chunks, v = kVec * (e - a * chunks);
+    copy_row(wtab + static_cast<size_t>(k0 + a) * wstride, sm + a * pitch, v);
+  }
+  if (threadIdx.x < na)
+    slot[k0 + threadIdx.x] =
+        make_int4(sslot[0][threadIdx.x], sslot[1][threadIdx.x], sslot[2][threadIdx.x], 0);
+  for (int e = threadIdx.x; e < na * pstride; e += 96) {
+    const int a = e / pstride, k = k0 + a, s = e - a * pstride;
+    const StencilDims& sd = dims(k);
+    if (s >= sd.S[0] * sd.S[1] * sd.S[2]) continue;
+    int tile, packed;
+    if (pair_of(make_int4(sslot[0][a], sslot[1][a], sslot[2][a], 0), s, sd, &tile, &packed))
+      arrival[pairs0(k) + s] = atomicAdd(&tile_counts[tile0(k) + tile], 1);
+  }
+}
+
+template <typename R>
+__global__ void __launch_bounds__(96) k_weights_axis(const double4* __restrict__ s4s, int n,
+                                                     StencilDims sd, R* __restrict__ wtab,
+                                                     R* __restrict__ qk, int4* __restrict__ slot,
+                                                     int* __restrict__ tile_counts,
+                                                     int* __restrict__ arrival) {
+  chain_enter();
+  extern __shared__ __align__(16) double sm_rows[];
+  const int S = sd.S[0] * sd.S[1] * sd.S[2];
+  weights_axis_body(
+      sm_rows, sd.wstride, sd.wstride, S, s4s, n, wtab, qk, slot, tile_counts, arrival,
+      [&](int) -> const StencilDims& { return sd; }, [&](int k) { return static_cast<size_t>(k) * S; },
+      [](int) { return 0; });
+}
+
+// Every cell of a batch (atom_prefix: first atom of each cell, slot_prefix: first
+// (atom, slot) item).
+template <typename R>
+__global__ void __launch_bounds__(96) k_weights_axis_seg(
+    const BatchCell* __restrict__ cells, const int* __restrict__ atom_prefix,
+    const int* __restrict__ slot_prefix, int ncells, int n, int wstride, int pstride,
+    const double4* __restrict__ s4s, R* __restrict__ wtab, R* __restrict__ qk,
+    int4* __restrict__ slot, int* __restrict__ tile_counts, int* __restrict__ arrival) {
+  chain_enter();
+  extern __shared__ __align__(16) double sm_rows[];
+  __shared__ int cid[kAxisAtoms];
+  const int k0 = blockIdx.x * kAxisAtoms;
+  if (threadIdx.x < kAxisAtoms)
+    cid[threadIdx.x] = seg_cell(atom_prefix, ncells, min(k0 + static_cast<int>(threadIdx.x), n - 1));
+  __syncthreads();
+  weights_axis_body(
+      sm_rows, wstride, wstride, pstride, s4s, n, wtab, qk, slot, tile_counts, arrival,
+      [&](int k) -> const StencilDims& { return cells[cid[k - k0]].sd; },
+      [&](int k) {
+        const int c = cid[k - k0];
+        const StencilDims& sd = cells[c].sd;
+        return slot_prefix[c] + static_cast<size_t>(k - cells[c].atom0) * sd.S[0] * sd.S[1] * sd.S[2];
+      },
+      [&](int k) { return cells[cid[k - k0]].tile0; });
+}
+
+// ---------------------------------------------------------------------------
+// (atom, tile) pair binning: counts (with arrival numbers), scan, scatter, and the
+// order of each tile's list by atom, which the tensor-core spread makes itself (the
+// gathers do not depend on it).
+// ---------------------------------------------------------------------------
 // Item idx of a batch's (atom, slot) launch: its cell, sorted atom, tile
 // (global numbering: the cell's tile0 added) and packed slot.
 __device__ __forceinline__ bool pair_of_seg(const BatchCell* __restrict__ cells,
@@ -374,29 +409,30 @@ __device__ __forceinline__ bool pair_of_seg(const BatchCell* __restrict__ cells,
   const int kl = local / S;
   *k = bc.atom0 + kl;
   const StencilDims sd = bc.sd;
-  if (!pair_of(slot, *k, local - kl * S, sd, tile, packed)) return false;
+  if (!pair_of(slot[*k], local - kl * S, sd, tile, packed)) return false;
   *tile += bc.tile0;
   return true;
 }
 
 __global__ void k_pair_count_seg(const BatchCell* __restrict__ cells,
                                  const int* __restrict__ prefix, int ncells, long nitems,
-                                 const int4* __restrict__ slot, int* __restrict__ counts) {
+                                 const int4* __restrict__ slot, int* __restrict__ counts,
+                                 int* __restrict__ arrival) {
   const long idx = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
   int tile, k, packed;
   if (idx < nitems && pair_of_seg(cells, prefix, ncells, idx, slot, &tile, &k, &packed))
-    atomicAdd(&counts[tile], 1);
+    arrival[idx] = atomicAdd(&counts[tile], 1);
 }
 
 __global__ void k_pair_scatter_seg(const BatchCell* __restrict__ cells,
                                    const int* __restrict__ prefix, int ncells, long nitems,
                                    const int4* __restrict__ slot, const int* __restrict__ starts,
-                                   int* __restrict__ cursor, int2* __restrict__ tmp) {
+                                   const int* __restrict__ arrival, int2* __restrict__ tmp) {
   chain_enter();
   const long idx = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
   int tile, k, packed;
   if (idx < nitems && pair_of_seg(cells, prefix, ncells, idx, slot, &tile, &k, &packed))
-    tmp[starts[tile] + atomicAdd(&cursor[tile], 1)] = make_int2(k, packed);
+    tmp[starts[tile] + arrival[idx]] = make_int2(k, packed);
 }
 
 // As k_pair_rank, the entry's cell found from its atom (sorted ranges follow
@@ -430,22 +466,24 @@ __device__ __forceinline__ bool pair_of_thread(const int4* __restrict__ slot, in
   if (t >= static_cast<long>(n) * S) return false;
   *k = static_cast<int>(t / S);
   const int s = static_cast<int>(t - static_cast<long>(*k) * S);
-  return pair_of(slot, *k, s, sd, tile, packed);
+  return pair_of(slot[*k], s, sd, tile, packed);
 }
 
 __global__ void k_pair_count(const int4* __restrict__ slot, int n, StencilDims sd,
-                             int* __restrict__ counts) {
+                             int* __restrict__ counts, int* __restrict__ arrival) {
   int tile, k, packed;
-  if (pair_of_thread(slot, n, sd, &tile, &k, &packed)) atomicAdd(&counts[tile], 1);
+  if (pair_of_thread(slot, n, sd, &tile, &k, &packed))
+    arrival[static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x] = atomicAdd(&counts[tile], 1);
 }
 
 __global__ void k_pair_scatter(const int4* __restrict__ slot, int n, StencilDims sd,
-                               const int* __restrict__ starts, int* __restrict__ cursor,
+                               const int* __restrict__ starts, const int* __restrict__ arrival,
                                int2* __restrict__ tmp) {
   chain_enter();
   int tile, k, packed;
   if (pair_of_thread(slot, n, sd, &tile, &k, &packed))
-    tmp[starts[tile] + atomicAdd(&cursor[tile], 1)] = make_int2(k, packed);
+    tmp[starts[tile] + arrival[static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x]] =
+        make_int2(k, packed);
 }
 
 // One thread per entry: orders each tile's bucket by atom index (atoms are
@@ -589,6 +627,7 @@ constexpr int kGatherAdWarps = 2;  // tensor-core gather with window derivatives
 // about 13 CTAs per SM) and two warps per tile.
 constexpr int kGatherAdF32Atoms = 1, kGatherAdF32Warps = 2;
 constexpr int kSpreadAtoms = 32;  // tensor-core spread: atoms staged per round, one per lane
+constexpr int kSpreadList = 128;  // longest tile list that the spread orders in shared memory
 constexpr int kWRow = 12;         // doubles per staged weight row: 8 used; the
                                   // padding makes the fragment reads conflict-free
 
@@ -616,9 +655,10 @@ __device__ __forceinline__ void stage2(double* dst, const float* src) {
 template <typename R>
 __device__ __forceinline__ void spread_tiles_dmma_body(int tx, int ty, int tz,
                                                        const int* __restrict__ tile_start,
-                                                       const int2* __restrict__ pairs,
-                                                       const R* __restrict__ wtab,
-                                                       const R* __restrict__ qk, StencilDims sd,
+                                                       const int2* __restrict__ unordered,
+                                                       int2* pairs, const R* __restrict__ wtab,
+                                                       const R* __restrict__ qk,
+                                                       const StencilDims& sd,
                                                        R* __restrict__ grid) {
   chain_enter();
   __shared__ __align__(16) double sW[3][kSpreadAtoms][kWRow];
@@ -631,12 +671,50 @@ __device__ __forceinline__ void spread_tiles_dmma_body(int tx, int ty, int tz,
 #pragma unroll
   for (int z = 0; z < TZ; ++z) acc[z][0] = acc[z][1] = 0.0;
   const int p0 = tile_start[tile], p1 = tile_start[tile + 1];
+  // The list in order of its atoms (unique within a tile): an entry's place is the
+  // number of entries with a smaller atom.  The lists hold some 40 entries, counted
+  // by a lane each in shared memory, four atoms to a load: less work than a launch
+  // of its own and than the list's way through global memory.
+  __shared__ int2 sList[kSpreadList];
+  const bool in_shared = unordered && p1 - p0 <= kSpreadList;
+  if (in_shared) {
+    const int m = p1 - p0;
+    int* ids = reinterpret_cast<int*>(&sW[0][0][0]);
+    int2 v[kSpreadList / 32];
+#pragma unroll
+    for (int h = 0; h < kSpreadList / 32; ++h) {
+      const int e = h * 32 + lane;
+      v[h] = e < m ? unordered[p0 + e] : make_int2(INT_MAX, 0);
+      ids[e] = v[h].x;
+    }
+    __syncwarp();
+    int place[kSpreadList / 32] = {0};
+    for (int j = 0; j < m; j += 4) {
+      const int4 x = *reinterpret_cast<const int4*>(ids + j);
+#pragma unroll
+      for (int h = 0; h < kSpreadList / 32; ++h)
+        place[h] += (x.x < v[h].x) + (x.y < v[h].x) + (x.z < v[h].x) + (x.w < v[h].x);
+    }
+#pragma unroll
+    for (int h = 0; h < kSpreadList / 32; ++h)
+      if (h * 32 + lane < m) sList[place[h]] = v[h];
+    __syncwarp();
+  } else if (unordered) {  // a long list goes through its ordered copy
+    for (int e = p0 + lane; e < p1; e += 32) {
+      const int2 v = unordered[e];
+      int place = p0;
+#pragma unroll 8
+      for (int j = p0; j < p1; ++j) place += unordered[j].x < v.x;
+      pairs[place] = v;
+    }
+    __syncwarp();
+  }
   for (int b0 = p0; b0 < p1; b0 += kSpreadAtoms) {
     const int nb = min(kSpreadAtoms, p1 - b0);
     __syncwarp();  // the previous round's weights are no longer read
     const int a = lane;
     if (a < nb) {
-      const int2 pr = pairs[b0 + a];
+      const int2 pr = in_shared ? sList[b0 - p0 + a] : pairs[b0 + a];
       const R* wk = wtab + static_cast<size_t>(pr.x) * sd.wstride;
       const R* src[3] = {wk + sd.woff[0] + (pr.y & 0xff) * TX,
                          wk + sd.woff[1] + ((pr.y >> 8) & 0xff) * TY,
@@ -1380,21 +1458,21 @@ __global__ void __launch_bounds__(kSpreadLanes) k_spread_tiles(const int* __rest
 }
 template <typename R>
 __global__ void __launch_bounds__(32) k_spread_tiles_dmma(const int* __restrict__ tile_start,
-                                                          const int2* __restrict__ pairs,
-                                                          const R* __restrict__ wtab,
+                                                          const int2* __restrict__ unordered,
+                                                          int2* pairs, const R* __restrict__ wtab,
                                                           const R* __restrict__ qk,
                                                           StencilDims sd, R* __restrict__ grid) {
-  spread_tiles_dmma_body<R>(blockIdx.x, blockIdx.y, blockIdx.z, tile_start, pairs, wtab, qk, sd,
-                            grid);
+  spread_tiles_dmma_body<R>(blockIdx.x, blockIdx.y, blockIdx.z, tile_start, unordered, pairs, wtab,
+                            qk, sd, grid);
 }
 template <typename R>
 __global__ void __launch_bounds__(32) k_spread_tiles_dmma_seg(
     const BatchCell* __restrict__ cells, const int* __restrict__ prefix, int ncells,
-    const int* __restrict__ tile_start, const int2* __restrict__ pairs,
+    const int* __restrict__ tile_start, const int2* __restrict__ unordered, int2* pairs,
     const R* __restrict__ wtab, const R* __restrict__ qk) {
   int tx, ty, tz;
   const BatchCell& bc = tile_of_block(cells, prefix, ncells, &tx, &ty, &tz);
-  spread_tiles_dmma_body<R>(tx, ty, tz, tile_start + bc.tile0, pairs, wtab, qk, bc.sd,
+  spread_tiles_dmma_body<R>(tx, ty, tz, tile_start + bc.tile0, unordered, pairs, wtab, qk, bc.sd,
                             static_cast<R*>(bc.grid));
 }
 
@@ -1458,78 +1536,83 @@ __global__ void __launch_bounds__(32 * WARPS) k_gather_tiles_dmma_ad_seg(
                                       static_cast<const R*>(bc.out), part);
 }
 
-template <typename R>
-__global__ void k_sorted_charges(const double* __restrict__ q, const int* __restrict__ perm, int n,
-                                 R* __restrict__ qk) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) qk[k] = static_cast<R>(q[perm[k]]);
-}
-
 inline int blocks_for(long n, int threads) { return static_cast<int>((n + threads - 1) / threads); }
 
 }  // namespace
 
-void launch_weights(const MeshPlan& mp, const int4* mc, const double4* fr, const int* perm, int n,
-                    void* wtab, void* qk, int4* slot, cudaStream_t st) {
-  if (n == 0) return;
-  const long threads = static_cast<long>(mp.sd.S[0] + mp.sd.S[1] + mp.sd.S[2]) * n;
-  if (mp.sd.kb)
-    launch_chained(mp.sd.ad ? k_weights_kb<true> : k_weights_kb<false>, blocks_for(n, kKbAtoms),
-                   96, 0, st, mc, fr, perm, n, mp.sd, static_cast<double*>(wtab),
-                   static_cast<double*>(qk), slot);
-  else if (mp.mixed)
-    launch_chained(k_weights_tiled<float>, blocks_for(threads, 128), 128, 0, st,
-        mc, fr, perm, n, mp.sd, static_cast<float*>(wtab), static_cast<float*>(qk), slot);
-  else
-    launch_chained(k_weights_tiled<double>, blocks_for(threads, 128), 128, 0, st,
-        mc, fr, perm, n, mp.sd, static_cast<double*>(wtab), static_cast<double*>(qk), slot);
-  ++g_launches;
-}
+namespace {
+size_t axis_smem(int row) { return sizeof(double) * kAxisAtoms * axis_pitch(row); }
 
-void launch_sorted_charges(const MeshPlan& mp, const double* q, const int* perm, int n, void* qk,
-                           cudaStream_t st) {
-  if (n == 0) return;
-  if (mp.mixed)
-    k_sorted_charges<float><<<blocks_for(n, 256), 256, 0, st>>>(q, perm, n, static_cast<float*>(qk));
-  else
-    k_sorted_charges<double><<<blocks_for(n, 256), 256, 0, st>>>(q, perm, n, static_cast<double*>(qk));
-  ++g_launches;
-}
+// Lists this long on average are ordered by a launch of their own, one thread per
+// entry, instead of by the spread's one warp per tile (both grow with the square
+// of the length; the tolerances in use give lists of 30 to 70).
+constexpr int kOwnRank = 256;
+bool own_rank(size_t npairs, size_t ntiles) { return npairs > kOwnRank * ntiles; }
 
-void launch_pair_bins(const MeshPlan& mp, const int4* slot, int n, int* counts, int* cursor,
-                      int* tile_start, int4* tmp, int2* pairs, int npairs_max, cudaStream_t st) {
-  const int ntiles = mp.sd.ntiles[0] * mp.sd.ntiles[1] * mp.sd.ntiles[2];
-  const long nthreads = static_cast<long>(n) * mp.sd.S[0] * mp.sd.S[1] * mp.sd.S[2];
-  int2* t2 = reinterpret_cast<int2*>(tmp);
-  cudaMemsetAsync(counts, 0, sizeof(int) * ntiles, st);
-  cudaMemsetAsync(cursor, 0, sizeof(int) * ntiles, st);
-  if (n > 0) {
-    k_pair_count<<<blocks_for(nthreads, 256), 256, 0, st>>>(slot, n, mp.sd, counts);
+template <typename R>
+void weights_bins(const MeshPlan& mp, const double4* s4s, int n, R* wtab, R* qk, int4* slot,
+                  const PairBins& b, cudaStream_t st) {
+  const StencilDims& sd = mp.sd;
+  const int ntiles = sd.ntiles[0] * sd.ntiles[1] * sd.ntiles[2];
+  const long items = static_cast<long>(n) * sd.S[0] * sd.S[1] * sd.S[2];
+  if (sd.wstride <= kAxisRow) {
+    launch_chained(k_weights_axis<R>, blocks_for(n, kAxisAtoms), 96, axis_smem(sd.wstride), st, s4s,
+                   n, sd, wtab, qk, slot, b.counts, b.arrival);
     ++g_launches;
-  }
-  launch_scan(counts, ntiles, tile_start, n > 0, st);
-  if (n > 0) {
-    launch_chained(k_pair_scatter, blocks_for(nthreads, 256), 256, 0, st, slot, n, mp.sd, tile_start, cursor,
-                                                               t2);
-    launch_chained(k_pair_rank, blocks_for(npairs_max, 256), 256, 0, st, t2, tile_start, ntiles, slot, mp.sd,
-                                                              pairs);
+  } else {
+    const long threads = static_cast<long>(sd.S[0] + sd.S[1] + sd.S[2]) * n;
+    launch_chained(k_weights_tiled<R>, blocks_for(threads, 128), 128, 0, st, s4s, n, sd, wtab, qk,
+                   slot);
+    k_pair_count<<<blocks_for(items, 256), 256, 0, st>>>(slot, n, sd, b.counts, b.arrival);
     g_launches += 2;
   }
+  launch_scan(b.counts, ntiles, b.starts, true, st);
+  launch_chained(k_pair_scatter, blocks_for(items, 256), 256, 0, st, slot, n, sd, b.starts,
+                 b.arrival, b.unordered);
+  ++g_launches;
+}
+}  // namespace
+
+void launch_weights_bins(const MeshPlan& mp, const double4* s4s, int n, void* wtab, void* qk,
+                         int4* slot, const PairBins& b, cudaStream_t st) {
+  if (n == 0) {
+    const int ntiles = mp.sd.ntiles[0] * mp.sd.ntiles[1] * mp.sd.ntiles[2];
+    cudaMemsetAsync(b.starts, 0, sizeof(int) * (ntiles + 1), st);
+    return;
+  }
+  if (mp.mixed)
+    weights_bins(mp, s4s, n, static_cast<float*>(wtab), static_cast<float*>(qk), slot, b, st);
+  else
+    weights_bins(mp, s4s, n, static_cast<double*>(wtab), static_cast<double*>(qk), slot, b, st);
 }
 
-void launch_spread(const MeshPlan& mp, const int* tile_start, const int2* pairs, const void* wtab,
-                   const void* qk, void* grid, cudaStream_t st) {
+void launch_spread(const MeshPlan& mp, const PairBins& b, const int4* slot, int n, bool ordered,
+                   const void* wtab, const void* qk, void* grid, cudaStream_t st) {
+  const int ntiles = mp.sd.ntiles[0] * mp.sd.ntiles[1] * mp.sd.ntiles[2];
+  const size_t items = static_cast<size_t>(n) * mp.sd.S[0] * mp.sd.S[1] * mp.sd.S[2];
+  const bool cores = mp.mixed && mp.stencil == 2;
+  const int* tile_start = b.starts;
+  int2* pairs = b.pairs;
+  const int2* unordered = b.unordered;
+  if (n > 0 && (cores || own_rank(items, ntiles))) {
+    if (!ordered) {
+      launch_chained(k_pair_rank, blocks_for(items, 256), 256, 0, st, unordered, tile_start, ntiles,
+                     slot, mp.sd, pairs);
+      ++g_launches;
+    }
+    unordered = nullptr;
+  }
   dim3 grd(mp.sd.ntiles[0], mp.sd.ntiles[1], mp.sd.ntiles[2]);
-  if (mp.mixed && mp.stencil == 2)  // FP32 CUDA-core spread
+  if (cores)  // FP32 CUDA-core spread
     launch_chained(k_spread_tiles<float>, grd, kSpreadLanes, 0, st, tile_start, pairs,
                    static_cast<const float*>(wtab), static_cast<const float*>(qk), mp.sd,
                    static_cast<float*>(grid));
   else if (mp.mixed)  // FP32 weights and grid, FP64 products on the tensor cores
-    launch_chained(k_spread_tiles_dmma<float>, grd, 32, 0, st, tile_start, pairs,
+    launch_chained(k_spread_tiles_dmma<float>, grd, 32, 0, st, tile_start, unordered, pairs,
                    static_cast<const float*>(wtab), static_cast<const float*>(qk), mp.sd,
                    static_cast<float*>(grid));
   else
-    launch_chained(k_spread_tiles_dmma<double>, grd, 32, 0, st, tile_start, pairs,
+    launch_chained(k_spread_tiles_dmma<double>, grd, 32, 0, st, tile_start, unordered, pairs,
                    static_cast<const double*>(wtab), static_cast<const double*>(qk), mp.sd,
                    static_cast<double*>(grid));
   ++g_launches;
@@ -1625,58 +1708,60 @@ void launch_gather_final(const MeshPlan& mp, const int4* slot, const int* perm, 
   ++g_launches;
 }
 
-void launch_weights_seg(const BatchLaunch& b, const int4* mc, const double4* fr, const int* perm,
-                        void* wtab, void* qk, int4* slot, cudaStream_t st) {
-  if (b.n_weights == 0) return;
-  if (b.any_kb) {
-    launch_chained(b.ad ? k_weights_kb_seg<true> : k_weights_kb_seg<false>,
-                   blocks_for(b.n_atoms, kKbAtoms), 96, 0, st, b.cells, b.p_atoms, b.ncells,
-                   b.n_atoms, b.wstride, mc, fr, perm, static_cast<double*>(wtab),
-                   static_cast<double*>(qk), slot);
+namespace {
+template <typename R>
+void weights_bins_seg(const BatchLaunch& b, const double4* s4s, R* wtab, R* qk, int4* slot,
+                      const PairBins& pb, cudaStream_t st) {
+  if (b.wstride <= kAxisRow) {
+    launch_chained(k_weights_axis_seg<R>, blocks_for(b.n_atoms, kAxisAtoms), 96,
+                   axis_smem(b.wstride), st, b.cells, b.p_atoms, b.p_slots, b.ncells, b.n_atoms,
+                   b.wstride, b.pstride, s4s, wtab, qk, slot, pb.counts, pb.arrival);
     ++g_launches;
-    if (!b.any_gauss) return;
-  }
-  if (b.mixed)
-    launch_chained(k_weights_seg<float>, blocks_for(b.n_weights, 128), 128, 0, st, b.cells,
-                   b.p_weights, b.ncells, b.n_weights, mc, fr, perm, static_cast<float*>(wtab),
-                   static_cast<float*>(qk), slot);
-  else
-    launch_chained(k_weights_seg<double>, blocks_for(b.n_weights, 128), 128, 0, st, b.cells,
-                   b.p_weights, b.ncells, b.n_weights, mc, fr, perm, static_cast<double*>(wtab),
-                   static_cast<double*>(qk), slot);
-  ++g_launches;
-}
-
-void launch_pair_bins_seg(const BatchLaunch& b, const int4* slot, int* counts, int* cursor,
-                          int* tile_start, int4* tmp, int2* pairs, cudaStream_t st) {
-  int2* t2 = reinterpret_cast<int2*>(tmp);
-  cudaMemsetAsync(counts, 0, sizeof(int) * b.n_tiles, st);
-  cudaMemsetAsync(cursor, 0, sizeof(int) * b.n_tiles, st);
-  if (b.n_slots > 0) {
-    k_pair_count_seg<<<blocks_for(b.n_slots, 256), 256, 0, st>>>(b.cells, b.p_slots, b.ncells,
-                                                                 b.n_slots, slot, counts);
-    ++g_launches;
-  }
-  launch_scan(counts, b.n_tiles, tile_start, b.n_slots > 0, st);
-  if (b.n_slots > 0) {
-    launch_chained(k_pair_scatter_seg, blocks_for(b.n_slots, 256), 256, 0, st, b.cells, b.p_slots,
-                   b.ncells, b.n_slots, slot, tile_start, cursor, t2);
-    launch_chained(k_pair_rank_seg, blocks_for(b.n_slots, 256), 256, 0, st, b.cells, b.p_atoms,
-                   b.ncells, t2, tile_start, b.n_tiles, slot, pairs);
+  } else {
+    launch_chained(k_weights_seg<R>, blocks_for(b.n_weights, 128), 128, 0, st, b.cells,
+                   b.p_weights, b.ncells, b.n_weights, s4s, wtab, qk, slot);
+    k_pair_count_seg<<<blocks_for(b.n_slots, 256), 256, 0, st>>>(
+        b.cells, b.p_slots, b.ncells, b.n_slots, slot, pb.counts, pb.arrival);
     g_launches += 2;
   }
+  launch_scan(pb.counts, b.n_tiles, pb.starts, true, st);
+  launch_chained(k_pair_scatter_seg, blocks_for(b.n_slots, 256), 256, 0, st, b.cells, b.p_slots,
+                 b.ncells, b.n_slots, slot, pb.starts, pb.arrival, pb.unordered);
+  ++g_launches;
+}
+}  // namespace
+
+void launch_weights_bins_seg(const BatchLaunch& b, const double4* s4s, void* wtab, void* qk,
+                             int4* slot, const PairBins& pb, cudaStream_t st) {
+  if (b.n_slots == 0) {
+    cudaMemsetAsync(pb.starts, 0, sizeof(int) * (b.n_tiles + 1), st);
+    return;
+  }
+  if (b.mixed)
+    weights_bins_seg(b, s4s, static_cast<float*>(wtab), static_cast<float*>(qk), slot, pb, st);
+  else
+    weights_bins_seg(b, s4s, static_cast<double*>(wtab), static_cast<double*>(qk), slot, pb, st);
 }
 
-void launch_spread_seg(const BatchLaunch& b, const int* tile_start, const int2* pairs,
+void launch_spread_seg(const BatchLaunch& b, const PairBins& pb, const int4* slot,
                        const void* wtab, const void* qk, cudaStream_t st) {
   if (b.n_tiles == 0) return;
+  const int* tile_start = pb.starts;
+  int2* pairs = pb.pairs;
+  const int2* unordered = pb.unordered;
+  if (b.n_slots > 0 && own_rank(b.n_slots, b.n_tiles)) {
+    launch_chained(k_pair_rank_seg, blocks_for(b.n_slots, 256), 256, 0, st, b.cells, b.p_atoms,
+                   b.ncells, unordered, tile_start, b.n_tiles, slot, pairs);
+    ++g_launches;
+    unordered = nullptr;
+  }
   if (b.mixed)
     launch_chained(k_spread_tiles_dmma_seg<float>, b.n_tiles, 32, 0, st, b.cells, b.p_tiles,
-                   b.ncells, tile_start, pairs, static_cast<const float*>(wtab),
+                   b.ncells, tile_start, unordered, pairs, static_cast<const float*>(wtab),
                    static_cast<const float*>(qk));
   else
     launch_chained(k_spread_tiles_dmma_seg<double>, b.n_tiles, 32, 0, st, b.cells, b.p_tiles,
-                   b.ncells, tile_start, pairs, static_cast<const double*>(wtab),
+                   b.ncells, tile_start, unordered, pairs, static_cast<const double*>(wtab),
                    static_cast<const double*>(qk));
   ++g_launches;
 }
@@ -1750,6 +1835,12 @@ int stencil_configure_kernels() {
     Table() { kb_polynomials(coef); }
   };
   static const Table t;
+  const int rows = static_cast<int>(axis_smem(kAxisRow));
+  for (const void* k : {reinterpret_cast<const void*>(k_weights_axis<double>),
+                        reinterpret_cast<const void*>(k_weights_axis<float>),
+                        reinterpret_cast<const void*>(k_weights_axis_seg<double>),
+                        reinterpret_cast<const void*>(k_weights_axis_seg<float>)})
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, rows);
   return cudaMemcpyToSymbol(c_kb, t.coef, sizeof(t.coef)) == cudaSuccess ? EWG_OK : EWG_ERR_CUDA;
 }
 
