@@ -5,7 +5,9 @@
 // that, how many loads an SM has in flight: with three radices of at most 8 a
 // line went three times through registers and twice through shared memory, each
 // thread with 5 to 8 loads outstanding between barriers.  Here a line goes
-// through registers twice: a thread loads R0 elements of its line at once, does
+// through registers twice (32,769 atoms, 192 points per axis, in us: x R2C 23, y
+// forward 16, z 43, y inverse 41, x C2R 82; 216,000 sites, 336 points: 146, 88, 425,
+// 262, 561, the last two at 4.0 and 3.4 TB/s): a thread loads R0 elements of its line at once, does
 // an R0-point transform in registers, leaves them in one shared buffer, and after
 // one barrier takes R1 of them through the second transform and out.  A CTA
 // holds 8 lines (128-byte rows: global and shared accesses are coalesced and
@@ -25,97 +27,135 @@
 
 namespace ewg {
 
+// LF: lines that are neighbours in the thread index (and in shared memory), 8 for
+// the strided axes, whose memory holds neighbouring lines side by side, 4 or 1 for
+// the x axis, whose memory holds a line's elements side by side.  The CTA's 8 / LF
+// groups of lines follow one another.
 template <int N, int R0, int R1>
 struct TwoPass {
   static_assert(R0 * R1 == N, "radices");
   static constexpr int L = 8;
   static constexpr int length = N;
-  static constexpr int radix0 = R0;
-  static constexpr int threads = L * (R0 > R1 ? R0 : R1);
+  static constexpr int radix0 = R0, radix1 = R1;
+  static constexpr int per_line = R0 > R1 ? R0 : R1;  // threads per line
+  static constexpr int threads = L * per_line;
+  // Element e of a line between the radices sits at (e + e / R0) LF (+ the line): the
+  // padding keeps the strided writes of the first radix free of bank conflicts
+  // when fewer than 8 lines lie side by side.
+  static constexpr int padded(int lf) { return lf < 8 ? N + R1 : N; }
   // Shared elements of one transform.
-  static constexpr int elems = N * L;
+  static constexpr int elems(int lf) { return padded(lf) * L; }
 
-  // ld(e) gives element e of this thread's line, st(e, v) takes element e of the
-  // result.  OWN: st writes to `a`, so every thread has read its elements first.
-  template <int SIGN, bool OWN, class Ld, class St>
-  __device__ __forceinline__ static void run(cx<double>* __restrict__ a,
-                                             const cx<double>* __restrict__ tw, Ld ld, St st) {
-    const int line = threadIdx.x & (L - 1), i = threadIdx.x / L;
-    if (i < R1) {
-      cx<double> u[R0];
+  // This thread's place: line within its group, butterfly, group.
+  template <int LF>
+  struct At {
+    int line, i, group;
+    // A batch's CTA can have more threads than this length uses: they get an i or a
+    // group past the last.
+    __device__ __forceinline__ At()
+        : line(threadIdx.x % LF),
+          i(LF == 8 ? threadIdx.x / 8 : threadIdx.x / LF % per_line),
+          group(LF == 8 ? 0 : threadIdx.x / (LF * per_line)) {}
+  };
+
+  // First radix: u holds elements i + j R1 of the thread's line.
+  template <int SIGN, int LF>
+  __device__ __forceinline__ static void first(const At<LF>& t, cx<double> (&u)[R0],
+                                               cx<double>* __restrict__ a) {
+    constexpr int kStep = LF < 8 ? R0 + 1 : R0;
+    dft_reg<double, SIGN, R0>(u);
+    cx<double>* dst = a + (t.group * padded(LF) + t.i * kStep) * LF + t.line;
 #pragma unroll
-      for (int j = 0; j < R0; ++j) u[j] = ld(i + j * R1);
-      dft_reg<double, SIGN, R0>(u);
-      cx<double>* dst = a + i * R0 * L + line;
+    for (int j = 0; j < R0; ++j) dst[j * LF] = u[j];
+  }
+  // Second radix: v becomes elements i + j R0 of the result.
+  template <int SIGN, int LF>
+  __device__ __forceinline__ static void second(const At<LF>& t, const cx<double>* __restrict__ a,
+                                                const cx<double>* __restrict__ tw,
+                                                cx<double> (&v)[R1]) {
+    constexpr int kStep = LF < 8 ? R0 + 1 : R0;
+    const cx<double>* src = a + (t.group * padded(LF) + t.i) * LF + t.line;
 #pragma unroll
-      for (int j = 0; j < R0; ++j) dst[j * L] = u[j];
+    for (int j = 0; j < R1; ++j) v[j] = src[j * kStep * LF];
+    // Twiddles w^(i j), w = exp(SIGN 2 pi i / N): every fourth power from the table,
+    // the others one or two products away (a few ulp).
+    cx<double> w1 = twiddle(tw, t.i, SIGN), w2, w3;
+    if (R1 > 2) w2 = mul(w1, w1);
+    if (R1 > 3) w3 = mul(w2, w1);
+    cx<double> base = w1;
+#pragma unroll
+    for (int j = 1; j < R1; ++j) {
+      if (j % 4 == 0) base = twiddle(tw, t.i * j, SIGN);
+      cx<double> w;
+      if (j < 4)
+        w = j == 1 ? w1 : (j == 2 ? w2 : w3);
+      else
+        w = j % 4 == 0 ? base : mul(base, j % 4 == 1 ? w1 : (j % 4 == 2 ? w2 : w3));
+      v[j] = mul(v[j], w);
     }
-    __syncthreads();
-    cx<double> v[R1];
-    if (i < R0) {
-      const cx<double>* src = a + i * L + line;
-#pragma unroll
-      for (int j = 0; j < R1; ++j) v[j] = src[j * R0 * L];
-      // Twiddles w^(i j), w = exp(SIGN 2 pi i / N): every fourth power from the
-      // table, the others one or two products away (a few ulp).
-      cx<double> w1 = twiddle(tw, i, SIGN), w2, w3;
-      if (R1 > 2) w2 = mul(w1, w1);
-      if (R1 > 3) w3 = mul(w2, w1);
-      cx<double> base = w1;
-#pragma unroll
-      for (int j = 1; j < R1; ++j) {
-        if (j % 4 == 0) base = twiddle(tw, i * j, SIGN);
-        cx<double> w;
-        if (j < 4)
-          w = j == 1 ? w1 : (j == 2 ? w2 : w3);
-        else
-          w = j % 4 == 0 ? base : mul(base, j % 4 == 1 ? w1 : (j % 4 == 2 ? w2 : w3));
-        v[j] = mul(v[j], w);
-      }
-      dft_reg<double, SIGN, R1>(v);
-    }
-    if (OWN) __syncthreads();
-    if (i < R0) {
-#pragma unroll
-      for (int j = 0; j < R1; ++j) st(i + j * R0, v[j]);
-    }
+    dft_reg<double, SIGN, R1>(v);
   }
 };
 
+// An element of global memory, or zero: a predicated load.  (As a branch around the
+// load, the compiler waited for a part of a thread's loads before it issued the
+// next.)
+__device__ __forceinline__ cx<double> load_if(const cx<double>* p, bool take) {
+  cx<double> v;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
+      "mov.f64 %1, 0d0000000000000000;\n\t@q ld.global.v2.f64 {%0, %1}, [%2];\n\t}"
+      : "=&d"(v.x), "=&d"(v.y)
+      : "l"(p), "r"(static_cast<int>(take)));
+  return v;
+}
+__device__ __forceinline__ cx<double> times_i(cx<double> v, double f) { return mk(-f * v.y, f * v.x); }
+
 // x, real to complex: row pairs (2p, 2p+1) form one complex line; k1 = 0..K1-1
-// of each row is kept.
+// of each row is kept.  Neighbouring threads take neighbouring x of one line.
 template <class SH>
 __device__ __forceinline__ void x_r2c_body(const PassCell& pc, int bx) {
-  constexpr int L = SH::L, n1 = SH::length;
+  constexpr int L = SH::L, n1 = SH::length, R0 = SH::radix0, R1 = SH::radix1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cx<double>* a = reinterpret_cast<cx<double>*>(smem_raw);
   const cx<double>* tw = plan_twiddles<double>(pc.fft[0]);
   const int K1 = pc.g.K1, npairs = pc.g.n[1] * pc.g.n[2] / 2;
-  const int pair0 = bx * L, mine = pair0 + (threadIdx.x & (L - 1));
-  const bool valid = mine < npairs;
-  const double* ra = static_cast<const double*>(pc.grid) + static_cast<size_t>(2 * (valid ? mine : 0)) * n1;
-  auto load = [&](int x) { return mk(ra[x], ra[n1 + x]); };
-  auto store = [&](int k, cx<double> v) { a[k * L + (threadIdx.x & (L - 1))] = v; };
-  SH::template run<-1, true>(a, tw, load, store);
+  const typename SH::template At<1> t;
+  const int pair0 = bx * L, mine = min(pair0 + t.group, npairs - 1);
+  if (t.i < R1 && t.group < L) {
+    const double* ra = static_cast<const double*>(pc.grid) + static_cast<size_t>(2 * mine) * n1 + t.i;
+    cx<double> u[R0];
+#pragma unroll
+    for (int j = 0; j < R0; ++j) u[j] = mk(ra[j * R1], ra[n1 + j * R1]);
+    SH::template first<-1, 1>(t, u, a);
+  }
   __syncthreads();
-  // Output k1 fastest: consecutive threads write consecutive k1 of one row pair.
+  cx<double> v[R1];
+  const bool on = t.i < R0 && t.group < L;
+  if (on) SH::template second<-1, 1>(t, a, tw, v);
+  __syncthreads();
+  if (on) {
+#pragma unroll
+    for (int j = 0; j < R1; ++j) a[t.group * n1 + t.i + j * R0] = v[j];
+  }
+  __syncthreads();
+  // The two rows' spectra from the line's, k1 fastest: whole rows of output.
   cx<double>* A1 = static_cast<cx<double>*>(pc.A1);
-  for (int t = threadIdx.x; t < L * K1; t += blockDim.x) {
-    const int l = t & (L - 1), k = t / L;
-    if (pair0 + l >= npairs) continue;
-    const cx<double> z = a[k * L + l];
-    cx<double> zc = a[(k == 0 ? 0 : n1 - k) * L + l];
-    zc.y = -zc.y;
-    cx<double>* o = A1 + static_cast<size_t>(2 * (pair0 + l)) * K1 + k;
-    o[0] = mk(0.5 * (z.x + zc.x), 0.5 * (z.y + zc.y));
-    o[K1] = mk(0.5 * (z.y - zc.y), -0.5 * (z.x - zc.x));
+  for (int l = threadIdx.x / 32; l < L && pair0 + l < npairs; l += (blockDim.x + 31) / 32) {
+    const cx<double>* z0 = a + l * n1;
+    cx<double>* o = A1 + static_cast<size_t>(2 * (pair0 + l)) * K1;
+    for (int k = threadIdx.x & 31; k < K1; k += min(32, blockDim.x - (threadIdx.x & ~31))) {
+      const cx<double> z = z0[k], zc = z0[k == 0 ? 0 : n1 - k];
+      o[k] = mk(0.5 * (z.x + zc.x), 0.5 * (z.y - zc.y));
+      o[K1 + k] = mk(0.5 * (z.y + zc.y), -0.5 * (z.x - zc.x));
+    }
   }
 }
 
 // y forward: lines over i2 for (i3, 8 values of k1); keeps k2 in [-H2, H2].
 template <class SH>
 __device__ __forceinline__ void y_fwd_body(const PassCell& pc, int local) {
-  constexpr int L = SH::L, n2 = SH::length;
+  constexpr int L = SH::L, n2 = SH::length, R0 = SH::radix0, R1 = SH::radix1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cx<double>* a = reinterpret_cast<cx<double>*>(smem_raw);
   const cx<double>* tw = plan_twiddles<double>(pc.fft[1]);
@@ -125,12 +165,22 @@ __device__ __forceinline__ void y_fwd_body(const PassCell& pc, int local) {
   const cx<double>* src =
       static_cast<const cx<double>*>(pc.A1) + static_cast<size_t>(i3) * n2 * K1 + (kin ? kl : 0);
   cx<double>* dst = static_cast<cx<double>*>(pc.A2) + static_cast<size_t>(i3) * K2 * K1 + kl;
-  auto load = [&](int i2) { return src[i2 * K1]; };
-  auto store = [&](int e, cx<double> v) {
-    const int k2i = e <= H2 ? e + H2 : e - n2 + H2;
-    if (kin && (e <= H2 || e >= n2 - H2)) dst[k2i * K1] = v;
-  };
-  SH::template run<-1, false>(a, tw, load, store);
+  const typename SH::template At<8> t;
+  if (t.i < R1) {
+    cx<double> u[R0];
+#pragma unroll
+    for (int j = 0; j < R0; ++j) u[j] = src[(t.i + j * R1) * K1];
+    SH::template first<-1, 8>(t, u, a);
+  }
+  __syncthreads();
+  if (t.i >= R0) return;
+  cx<double> v[R1];
+  SH::template second<-1, 8>(t, a, tw, v);
+#pragma unroll
+  for (int j = 0; j < R1; ++j) {
+    const int e = t.i + j * R0, k2i = e <= H2 ? e + H2 : e - n2 + H2;
+    if (kin && (e <= H2 || e >= n2 - H2)) dst[k2i * K1] = v[j];
+  }
 }
 
 // z forward, influence weights, z inverse of P and (forces) T3 = 2 pi i k3 P, for
@@ -138,10 +188,10 @@ __device__ __forceinline__ void y_fwd_body(const PassCell& pc, int local) {
 template <class SH, bool STRESS>
 __device__ __forceinline__ void z_body(const PassCell& pc, int local, int nz,
                                        double* __restrict__ stress) {
-  constexpr int L = SH::L, n3 = SH::length;
+  constexpr int L = SH::L, n3 = SH::length, R0 = SH::radix0, R1 = SH::radix1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cx<double>* a = reinterpret_cast<cx<double>*>(smem_raw);
-  cx<double>* q = a + SH::elems;  // K3 weighted modes per line
+  cx<double>* q = a + SH::elems(8);  // K3 weighted modes per line
   const cx<double>* tw = plan_twiddles<double>(pc.fft[2]);
   const int K1 = pc.g.K1, K2 = pc.g.K2, K3 = pc.g.K3, kb = (K1 + L - 1) / L;
   const int h1 = K1 - 1, h2 = (K2 - 1) / 2, h3 = (K3 - 1) / 2;
@@ -151,7 +201,13 @@ __device__ __forceinline__ void z_body(const PassCell& pc, int local, int nz,
   const size_t zstride = static_cast<size_t>(K2) * K1;
   const size_t at = static_cast<size_t>(k2i) * K1 + (kin ? k1 : 0);
   const cx<double>* src = static_cast<const cx<double>*>(pc.A2) + at;
-  auto load_fwd = [&](int i3) { return src[i3 * zstride]; };
+  const typename SH::template At<8> t;
+  if (t.i < R1) {
+    cx<double> u[R0];
+#pragma unroll
+    for (int j = 0; j < R0; ++j) u[j] = src[(t.i + j * R1) * zstride];
+    SH::template first<-1, 8>(t, u, a);
+  }
   // The mode's share of the weight that does not depend on k3.
   constexpr double twoPi = 2.0 * 3.14159265358979323846;
   const double inv4a2 = 1.0 / (4.0 * (pc.g.alpha * pc.g.alpha));
@@ -173,19 +229,24 @@ __device__ __forceinline__ void z_body(const PassCell& pc, int local, int nz,
   }
   const double* corr3 = pc.corr2[2];
   double sv[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  auto keep = [&](int e, cx<double> v) {
-    if (e <= h3)
-      q[(e + h3) * L + line] = v;
-    else if (e >= n3 - h3)
-      q[(e - n3 + h3) * L + line] = v;
-  };
-  SH::template run<-1, false>(a, tw, load_fwd, keep);
+  __syncthreads();
+  if (t.i < R0) {
+    cx<double> v[R1];
+    SH::template second<-1, 8>(t, a, tw, v);
+#pragma unroll
+    for (int j = 0; j < R1; ++j) {
+      const int e = t.i + j * R0;
+      if (e <= h3)
+        q[(e + h3) * L + line] = v[j];
+      else if (e >= n3 - h3)
+        q[(e - n3 + h3) * L + line] = v[j];
+    }
+  }
   // Each thread weights the modes that it has put into q itself (no barrier), in
   // a loop that is not unrolled: inlined into the transform, one exponential and
   // one division per output cost it 100 registers.
-  const int i = threadIdx.x / L;
 #pragma unroll 1
-  for (int e = i; i < SH::radix0 && e < n3; e += SH::radix0) {
+  for (int e = t.i; t.i < R0 && e < n3; e += R0) {
     if (e > h3 && e < n3 - h3) continue;
     const int k3 = e <= h3 ? e : e - n3;
     const double kx = fma(static_cast<double>(k3), b3[0], b12[0]);
@@ -235,18 +296,28 @@ __device__ __forceinline__ void z_body(const PassCell& pc, int local, int nz,
   }
   cx<double>* dst = static_cast<cx<double>*>(pc.B2) + at;
   for (int c = 0; c < nz; ++c) {
-    auto load_inv = [&](int e) {
-      if (e > h3 && e < n3 - h3) return mk(0.0, 0.0);
-      const int k3 = e <= h3 ? e : e - n3;
-      const cx<double> v = q[(k3 + h3) * L + line];
-      if (c == 0) return v;
-      const double t = twoPi * k3;
-      return mk(-t * v.y, t * v.x);  // 2 pi i k3 v
-    };
-    auto store = [&](int i3, cx<double> v) {
-      if (kin) dst[i3 * zstride] = v;
-    };
-    SH::template run<1, false>(a, tw, load_inv, store);
+    if (t.i < R1) {
+      cx<double> u[R0];
+#pragma unroll
+      for (int j = 0; j < R0; ++j) {
+        const int e = t.i + j * R1, k3 = e <= h3 ? e : e - n3;
+        u[j] = mk(0.0, 0.0);
+        if (e <= h3 || e >= n3 - h3) {
+          u[j] = q[(k3 + h3) * L + line];
+          if (c > 0) u[j] = times_i(u[j], twoPi * k3);  // 2 pi i k3 v
+        }
+      }
+      SH::template first<1, 8>(t, u, a);
+    }
+    __syncthreads();
+    if (t.i < R0) {
+      cx<double> v[R1];
+      SH::template second<1, 8>(t, a, tw, v);
+      if (kin) {
+#pragma unroll
+        for (int j = 0; j < R1; ++j) dst[(t.i + j * R0) * zstride] = v[j];
+      }
+    }
     dst += n3 * zstride;
     __syncthreads();
   }
@@ -256,70 +327,100 @@ __device__ __forceinline__ void z_body(const PassCell& pc, int local, int nz,
 // components IFFT_y(P) and, for forces, IFFT_y(2 pi i k2 P), IFFT_y(T3).
 template <class SH>
 __device__ __forceinline__ void y_inv_body(const PassCell& pc, int local) {
-  constexpr int L = SH::L, n2 = SH::length;
+  constexpr int L = SH::L, n2 = SH::length, R0 = SH::radix0, R1 = SH::radix1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cx<double>* a = reinterpret_cast<cx<double>*>(smem_raw);
   const cx<double>* tw = plan_twiddles<double>(pc.fft[1]);
   const int K1 = pc.g.K1, K2 = pc.g.K2, H2 = (K2 - 1) / 2, n3 = pc.g.n[2], kb = (K1 + L - 1) / L;
-  const int t = local / kb, kl = (local - t * kb) * L + (threadIdx.x & (L - 1));
-  const int c = t / n3, i3 = t - c * n3;
+  const int ci = local / kb, kl = (local - ci * kb) * L + (threadIdx.x & (L - 1));
+  const int c = ci / n3, i3 = ci - c * n3;
   const int cs = c == 2 ? 1 : 0;
   const bool dk2 = c == 1, kin = kl < K1;
   const cx<double>* src = static_cast<const cx<double>*>(pc.B2) +
                           ((static_cast<size_t>(cs) * n3 + i3) * K2 + H2) * K1 + (kin ? kl : 0);
   cx<double>* dst =
       static_cast<cx<double>*>(pc.B1) + (static_cast<size_t>(c) * n3 + i3) * n2 * K1 + kl;
-  auto load = [&](int i2) {
-    if (i2 > H2 && i2 < n2 - H2) return mk(0.0, 0.0);
-    const int k2 = i2 <= H2 ? i2 : i2 - n2;
-    const cx<double> v = src[k2 * K1];
-    if (!dk2) return v;
-    const double f = 2.0 * 3.14159265358979323846 * k2;
-    return mk(-f * v.y, f * v.x);
-  };
-  auto store = [&](int i2, cx<double> v) {
-    if (kin) dst[i2 * K1] = v;
-  };
-  SH::template run<1, false>(a, tw, load, store);
+  const typename SH::template At<8> t;
+  if (t.i < R1) {
+    cx<double> u[R0];
+#pragma unroll
+    for (int j = 0; j < R0; ++j) {
+      const int i2 = t.i + j * R1, k2 = i2 <= H2 ? i2 : i2 - n2;
+      u[j] = load_if(src + k2 * K1, i2 <= H2 || i2 >= n2 - H2);
+    }
+    if (dk2) {
+#pragma unroll
+      for (int j = 0; j < R0; ++j) {
+        const int i2 = t.i + j * R1;
+        u[j] = times_i(u[j], 2.0 * 3.14159265358979323846 * (i2 <= H2 ? i2 : i2 - n2));
+      }
+    }
+    SH::template first<1, 8>(t, u, a);
+  }
+  __syncthreads();
+  if (t.i >= R0 || !kin) return;
+  cx<double> v[R1];
+  SH::template second<1, 8>(t, a, tw, v);
+#pragma unroll
+  for (int j = 0; j < R1; ++j) dst[(t.i + j * R0) * K1] = v[j];
 }
 
-// x, complex to real: the lines of a CTA are (row pair, component), the component
-// fastest, so neighbouring threads write one point's components; outputs phi =
-// C2R(Y0) and, with NC = 4, D1 = C2R(2 pi i k1 Y0), C2R(Y2), C2R(Y3), interleaved.
+// x, complex to real: a line is a row pair's component, the NC components of one
+// pair neighbours, so that neighbouring threads write one point's components and
+// neighbouring points; outputs phi = C2R(Y0) and, with NC = 4, D1 = C2R(2 pi i k1 Y0),
+// C2R(Y2), C2R(Y3), interleaved.
 template <class SH, int NC>
 __device__ __forceinline__ void x_c2r_body(const PassCell& pc, int bx) {
-  constexpr int L = SH::L, n1 = SH::length, NP = L / NC;
+  constexpr int L = SH::L, n1 = SH::length, NP = L / NC, R0 = SH::radix0, R1 = SH::radix1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cx<double>* a = reinterpret_cast<cx<double>*>(smem_raw);
   const cx<double>* tw = plan_twiddles<double>(pc.fft[0]);
   const int K1 = pc.g.K1, nrows = pc.g.n[1] * pc.g.n[2];
-  const int line = threadIdx.x & (L - 1), cc = line % NC, pr = bx * NP + line / NC;
-  const bool valid = 2 * pr < nrows;
-  const int cs = cc <= 1 ? 0 : cc - 1;
-  const bool dk1 = cc == 1;
-  const cx<double>* sa = static_cast<const cx<double>*>(pc.B1) +
-                         (static_cast<size_t>(cs) * nrows + (valid ? 2 * pr : 0)) * K1;
-  double* oa = static_cast<double*>(pc.out) + 2 * static_cast<size_t>(pr) * n1 * NC + cc;
-  auto load = [&](int x) {
-    if (x >= K1 && x <= n1 - K1) return mk(0.0, 0.0);
-    const bool lo = x < K1;
-    const int kx = lo ? x : n1 - x;
-    cx<double> fa = sa[kx], fb = sa[K1 + kx];
-    if (dk1) {
-      const double t = 2.0 * 3.14159265358979323846 * kx;
-      fa = mk(-t * fa.y, t * fa.x);
-      fb = mk(-t * fb.y, t * fb.x);
+  const typename SH::template At<NC> t;
+  const int pr = bx * NP + t.group;
+  const bool valid = 2 * pr < nrows && t.group < NP;
+  if (t.i < R1 && t.group < NP) {
+    const int cs = t.line <= 1 ? 0 : t.line - 1;
+    const cx<double>* sa = static_cast<const cx<double>*>(pc.B1) +
+                           (static_cast<size_t>(cs) * nrows + (valid ? 2 * pr : 0)) * K1;
+    cx<double> u[R0];
+    // The rows' two halves of the loads in turn: R0 of them in flight at a time.
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      cx<double> fa[(R0 + 1) / 2], fb[(R0 + 1) / 2];
+#pragma unroll
+      for (int j = h; j < R0; j += 2) {
+        const int x = t.i + j * R1, kx = x < K1 ? x : n1 - x;
+        const bool in = x < K1 || x > n1 - K1;
+        fa[j / 2] = load_if(sa + kx, in);
+        fb[j / 2] = load_if(sa + K1 + kx, in);
+      }
+#pragma unroll
+      for (int j = h; j < R0; j += 2) {
+        const int x = t.i + j * R1;
+        cx<double> p = fa[j / 2], q = fb[j / 2];
+        if (t.line == 1) {
+          const double f = 2.0 * 3.14159265358979323846 * (x < K1 ? x : n1 - x);
+          p = times_i(p, f);
+          q = times_i(q, f);
+        }
+        // Hermitian continuation; the k1 = 0 modes' imaginary parts drop out.
+        const double s = x == 0 ? 0.0 : (x < K1 ? 1.0 : -1.0);
+        u[j] = mk(p.x - s * q.y, s * p.y + q.x);
+      }
     }
-    // Hermitian continuation; the k1 = 0 modes' imaginary parts drop out.
-    const double s = x == 0 ? 0.0 : (lo ? 1.0 : -1.0);
-    return mk(fa.x - s * fb.y, s * fa.y + fb.x);
-  };
-  auto store = [&](int x, cx<double> v) {
-    if (!valid) return;
-    oa[x * NC] = v.x;
-    oa[(n1 + x) * NC] = v.y;
-  };
-  SH::template run<1, false>(a, tw, load, store);
+    SH::template first<1, NC>(t, u, a);
+  }
+  __syncthreads();
+  if (t.i >= R0 || !valid) return;
+  cx<double> v[R1];
+  SH::template second<1, NC>(t, a, tw, v);
+  double* oa = static_cast<double*>(pc.out) + (2 * static_cast<size_t>(pr) * n1 + t.i) * NC + t.line;
+#pragma unroll
+  for (int j = 0; j < R1; ++j) {
+    oa[j * R0 * NC] = v[j].x;
+    oa[(n1 + j * R0) * NC] = v[j].y;
+  }
 }
 
 // ---- kernels ----------------------------------------------------------------
@@ -356,7 +457,7 @@ void go64(K kernel, const Launch64& l, size_t sm, A... args) {
 // A single cell's pass at the length of SH.
 template <class SH>
 void launch64(const Launch64& l) {
-  const size_t sm = sizeof(cx<double>) * SH::elems;
+  const size_t sm = sizeof(cx<double>) * SH::elems(l.pass == P64_R2C || l.pass == P64_C2R ? 1 : 8);
   const size_t smz = sm + sizeof(cx<double>) * SH::L * static_cast<size_t>(l.K3);
   switch (l.pass) {
     case P64_R2C: go64<SH>(k64_pass<SH, P64_R2C, 0>, l, sm, *l.one, 1, l.stress); break;
@@ -398,7 +499,8 @@ struct Seg64 {
   static constexpr int threads = most({SHS::threads...});
   template <int PASS, int VAR>
   static void go(const Launch64& l) {
-    size_t sm = sizeof(cx<double>) * 8 * static_cast<size_t>(l.nmax);
+    const int x = PASS == P64_R2C || PASS == P64_C2R ? 1 : 8;
+    size_t sm = sizeof(cx<double>) * most({(SHS::length <= l.nmax ? SHS::elems(x) : 0)...});
     if (PASS == P64_Z) sm += sizeof(cx<double>) * 8 * static_cast<size_t>(l.K3);
     go64<Seg64>(k64_pass_seg<threads, PASS, VAR, SHS...>, l, sm, l.cells, l.group, l.nz);
   }
