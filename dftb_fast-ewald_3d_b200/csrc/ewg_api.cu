@@ -547,8 +547,8 @@ int evaluate(ewg_context* c, int n, const double* pos, long sa, long sd, const d
     prof_mark(mp.prof, st, ST_WEIGHTS);
     if (!reuse) launch_weights_bins(mp, s4s, n, wtab, qk, slot, bins, st);
     prof_mark(mp.prof, st, ST_REAL);
-    launch_real_space(s4s, x32s, permbox, boxstart, n, rg, p.alpha, p.r_cut, mixed, pot_sr, f_sr,
-                      err, rs);
+    launch_real_space(s4s, x32s, permbox, boxstart, n, rg, p.alpha, p.r_cut, mixed, pot_sr,
+                      want_force ? f_sr : nullptr, err, rs);
     if (stress12)  // real-space virial over the same pairs
       launch_real_stress(s4s, x32s, boxstart, n, rg, p.alpha, p.r_cut, p6, stress12, err, rs);
     if (concurrent) cudaEventRecord(c->join, rs);
@@ -971,7 +971,7 @@ void seg_kernels(ewg_context* c, const SegPlan& sp, const SegBufs& sb, const dou
   launch_atom_sort_seg(b, coords, q, sb.sort, sb.bins.counts, b.n_tiles, st);
   prof_mark(prof, st, ST_REAL);
   launch_real_space_seg(b, sb.sort.s4s, sb.sort.x32, sb.sort.perm, sb.sort.starts, sb.pot_sr,
-                        sb.f_sr, cellerr, st);
+                        force ? sb.f_sr : nullptr, cellerr, st);
   prof_mark(prof, st, ST_WEIGHTS);
   launch_weights_bins_seg(b, sb.sort.s4s, sb.wtab, sb.qk, sb.slot, sb.bins, st);
   prof_mark(prof, st, ST_SPREAD);

@@ -92,7 +92,7 @@ void launch_scan(const int* counts, int nkeys, int* starts, bool after_kernel, c
 // out[0] = sum q, out[1] = sum |q|, out[2] = sum q^2 (fixed-order reduction).
 void launch_charge_sums(const double* q, int n, double* partial, double* out, cudaStream_t st);
 
-// Real-space erfc pair sum (fft/ewald_fft_3d_real.f90:81-187 and
+// Real-space erfc pair sum (force null: the potential alone; fft/ewald_fft_3d_real.f90:81-187 and
 // direct/ewald_direct_3d.f90:192-309) over box-sorted atoms.  Writes pot and
 // force (3,N) by original atom index.  mixed != 0 evaluates the pair terms in
 // FP32 and accumulates in FP64.

@@ -458,6 +458,13 @@ struct QueueBase {
   }
 };
 
+// An int as a double through its bits (2^52 + 2^31 + n, less the offset): one FP64
+// addition instead of a conversion at a quarter of its rate.
+__device__ __forceinline__ double small_double(int n) {
+  return __hiloint2double(0x43300000, static_cast<int>(static_cast<unsigned>(n) ^ 0x80000000u)) -
+         4503601774854144.0;
+}
+
 // Entries (j, S); at evaluation the separation, the exact cutoff test and the
 // coincidence test are done in FP64.  F32TERM: the pair term then runs in FP32
 // on the FP64 separation rounded once (the mixed form); otherwise in FP64.
@@ -473,7 +480,8 @@ struct PairQueue : QueueBase<Pair, int4> {
       : QueueBase<Pair, int4>(qbuf, p), srt(s), ai(a), g(&geo), cut2(c2), pre2(p2) {}
   __device__ __forceinline__ void eval_entry(const int4& e) {
     const double4 aj = srt[e.x];
-    const double d1 = (ai.x - aj.x) - e.y, d2 = (ai.y - aj.y) - e.z, d3 = (ai.z - aj.z) - e.w;
+    const double d1 = (ai.x - aj.x) - small_double(e.y), d2 = (ai.y - aj.y) - small_double(e.z),
+                 d3 = (ai.z - aj.z) - small_double(e.w);
     double sep[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) sep[c] = d1 * g->lat[0][c] + d2 * g->lat[1][c] + d3 * g->lat[2][c];
@@ -484,7 +492,7 @@ struct PairQueue : QueueBase<Pair, int4> {
         this->pair.eval32(make_float4(static_cast<float>(sep[0]), static_cast<float>(sep[1]),
                                       static_cast<float>(sep[2]), static_cast<float>(aj.w)));
       else
-        this->pair.eval(make_double4(sep[0], sep[1], sep[2], aj.w));
+        this->pair.eval(make_double4(sep[0], sep[1], sep[2], aj.w), r2);
     }
   }
   __device__ __forceinline__ void operator()(const Candidate& c) {
@@ -726,24 +734,51 @@ inline float prefilter_bound(const RealGeom& g, double r_cut) {
   return static_cast<float>(r * r);
 }
 
+// exp(x^2) erfc(x) = s P(s), s = 1 / (1 + 0.3 x): P is smooth on the half line, and a
+// polynomial of degree 17 in t (s mapped from [1/3.1, 1], x <= 7, to [-1, 1]) gives
+// it to a few units of 1e-16; beyond x = 7 the exponential that multiplies it is
+// below 1e-21.  The coefficients of t^k are those of the Chebyshev interpolant at 18
+// nodes, with erfcx from the power series of erf (x < 0.8) and its continued
+// fraction in 64-bit-mantissa arithmetic; the same for every lane, they are constant
+// operands.
+constexpr int kErfcDegree = 17;
+constexpr double kErfcP = 0.3, kErfcLow = 1.0 / (1.0 + kErfcP * 7.0);
+__constant__ double c_erfc[kErfcDegree + 1] = {
+    0.4395437674721796, 0.30529357714526528, 0.16371613627256329,
+    0.067209167578163864, 0.020227023028525769, 0.0039119665897932396,
+    0.00022645085997755068, -0.00010700946583254409, -2.4566325660992749e-05,
+    2.2716990739404845e-06, 1.3416217162359745e-06, -6.160564444921783e-08,
+    -7.2547061079187976e-08, 4.2702688499460546e-09, 4.0071758010561274e-09,
+    -4.5555884373469113e-10, -1.7922918704726953e-10, 3.4283662328802062e-11};
+
 // Pair term of fft/ewald_fft_3d_real.f90:153-172: FP64 (eval, FP64 separation),
-// or its FP32 form (eval32, FP32 separation), accumulated in FP64.
+// or its FP32 form (eval32, FP32 separation), accumulated in FP64; FORCE: with the
+// force.  The FP64 term takes one reciprocal square root, one exponential for both
+// of its terms, a reciprocal and the polynomial above, about 100 FP64 operations where
+// the square root, two divisions, erfc and exp took 170; it is what bounds the FP64
+// kernel.
+template <bool FORCE>
 struct EwaldPair {
   double alpha, qi;
   double pot = 0.0, f[3] = {0.0, 0.0, 0.0};
   int bad = 0;
-  __device__ __forceinline__ void eval(const double4& e) {
-    const double r2 = e.x * e.x + e.y * e.y + e.z * e.z;
-    const double qj = e.w;
-    const double r = sqrt(r2);
-    const double rinv = 1.0 / r;
-    const double ecr = erfc(alpha * r) * rinv;  // erfc(alpha r) / r
-    pot += qj * ecr;
-    const double ff =
-        qi * qj * (2.0 * alpha / kSqrtPi * exp(-alpha * alpha * r2) + ecr) * (rinv * rinv);
-    f[0] += ff * e.x;
-    f[1] += ff * e.y;
-    f[2] += ff * e.z;
+  __device__ __forceinline__ void eval(const double4& e, double r2) {
+    const double y = rsqrt(r2);
+    const double x = alpha * (r2 * y);
+    const double g = exp(-(x * x));
+    const double s = __drcp_rn(fma(kErfcP, x, 1.0));
+    const double t = fma(s, 2.0 / (1.0 - kErfcLow), -(1.0 + kErfcLow) / (1.0 - kErfcLow));
+    double p = c_erfc[kErfcDegree];
+#pragma unroll
+    for (int k = kErfcDegree - 1; k >= 0; --k) p = fma(p, t, c_erfc[k]);
+    const double ecr = g * (s * p) * y;  // erfc(alpha r) / r
+    pot = fma(e.w, ecr, pot);
+    if (FORCE) {
+      const double ff = qi * e.w * fma(2.0 * alpha / kSqrtPi, g, ecr) * (y * y);
+      f[0] = fma(ff, e.x, f[0]);
+      f[1] = fma(ff, e.y, f[1]);
+      f[2] = fma(ff, e.z, f[2]);
+    }
   }
   __device__ __forceinline__ void eval32(const float4& e) {
     const float r2f = fmaf(e.x, e.x, fmaf(e.y, e.y, e.z * e.z));
@@ -753,12 +788,14 @@ struct EwaldPair {
     const float ec = erfcf(af * r);
     const float pe = e.w * ec * rinv;
     pot += static_cast<double>(pe);
-    const float ff = static_cast<float>(qi) * e.w *
-                     (2.0f * af * 0.56418958354775628695f * expf(-af * af * r2f) + ec * rinv) *
-                     (rinv * rinv);
-    f[0] += static_cast<double>(ff * e.x);
-    f[1] += static_cast<double>(ff * e.y);
-    f[2] += static_cast<double>(ff * e.z);
+    if (FORCE) {
+      const float ff = static_cast<float>(qi) * e.w *
+                       (2.0f * af * 0.56418958354775628695f * expf(-af * af * r2f) + ec * rinv) *
+                       (rinv * rinv);
+      f[0] += static_cast<double>(ff * e.x);
+      f[1] += static_cast<double>(ff * e.y);
+      f[2] += static_cast<double>(ff * e.z);
+    }
   }
 };
 
@@ -768,7 +805,7 @@ struct EwaldPair {
 // to the mesh kernels beside it: 32,769 atoms 674 -> 662 us per evaluation against
 // CTAs of 256 threads, mixed form 364 -> 359.
 // The warp of sorted atom k (box_start: the cell's own box numbering).
-template <bool MIXED>
+template <bool MIXED, bool FORCE>
 __device__ __forceinline__ void real_space_body(const double4* __restrict__ srt,
                                                 const float4* __restrict__ x32,
                                                 const int* __restrict__ perm,
@@ -781,16 +818,27 @@ __device__ __forceinline__ void real_space_body(const double4* __restrict__ srt,
   __shared__ RunTable runs[kRealThreads / 32];
   const int lane = threadIdx.x & 31;
   const double4 ai = srt[k];
-  EwaldPair pair;
+  EwaldPair<FORCE> pair;
   pair.alpha = alpha;
   pair.qi = ai.w;
-  PairQueue<EwaldPair, MIXED> pq(queue[threadIdx.x >> 5], pair, srt, ai, g, cut2, pre2);
+  PairQueue<EwaldPair<FORCE>, MIXED> pq(queue[threadIdx.x >> 5], pair, srt, ai, g, cut2, pre2);
   if (g.flat)
     for_each_candidate_flat(x32, box_start, k, ai, g, cut2 * (1.0 + 1e-9), runs[threadIdx.x >> 5],
                               pq);
   else
     for_each_candidate(x32, box_start, k, ai, g, pq);
   pq.flush();
+  const int bad = __any_sync(0xffffffffu, pair.bad);
+  if constexpr (!FORCE) {  // the same tree as below
+    double t = pair.pot;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+    if (lane == 0) {
+      pot[perm[k]] = t;
+      if (bad) atomicOr(err, 1);
+    }
+    return;
+  }
   // Transposed reduction of (pot, f_x, f_y, f_z): halves and quarters of the
   // warp each keep some of the four sums and pass the others on (6 shuffles of
   // doubles instead of 20); lanes 0, 8, 16, 24 end with the four totals.
@@ -803,7 +851,6 @@ __device__ __forceinline__ void real_space_body(const double4* __restrict__ srt,
   t += __shfl_xor_sync(0xffffffffu, t, 4);
   t += __shfl_xor_sync(0xffffffffu, t, 2);
   t += __shfl_xor_sync(0xffffffffu, t, 1);
-  const int bad = __any_sync(0xffffffffu, pair.bad);
   if ((lane & 7) == 0) {
     const int i = perm[k];
     const int c = lane >> 3;  // 0: pot, 1..3: force component c - 1
@@ -815,7 +862,7 @@ __device__ __forceinline__ void real_space_body(const double4* __restrict__ srt,
   }
 }
 
-template <bool MIXED>
+template <bool MIXED, bool FORCE>
 __global__ void __launch_bounds__(kRealThreads, 16) k_real_space(const double4* __restrict__ srt,
                                                              const float4* __restrict__ x32,
                                                              const int* __restrict__ perm,
@@ -827,12 +874,12 @@ __global__ void __launch_bounds__(kRealThreads, 16) k_real_space(const double4* 
                                                              int* __restrict__ err) {
   const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (k >= n) return;
-  real_space_body<MIXED>(srt, x32, perm, box_start, k, g, alpha, cut2, pre2, pot, force, err);
+  real_space_body<MIXED, FORCE>(srt, x32, perm, box_start, k, g, alpha, cut2, pre2, pot, force, err);
 }
 
 // Every cell of a batch: the warp's atom k picks its cell's cell-list geometry,
 // splitting and cutoff; a coincident pair flags the cell (err[cell]).
-template <bool MIXED>
+template <bool MIXED, bool FORCE>
 __global__ void __launch_bounds__(kRealThreads, 16) k_real_space_seg(
     const BatchCell* __restrict__ cells, const int* __restrict__ prefix, int ncells,
     const double4* __restrict__ srt, const float4* __restrict__ x32, const int* __restrict__ perm,
@@ -843,7 +890,7 @@ __global__ void __launch_bounds__(kRealThreads, 16) k_real_space_seg(
   const int c = seg_cell(prefix, ncells, k);
   const BatchCell& bc = cells[c];
   const RealGeom g = bc.rg;
-  real_space_body<MIXED>(srt, x32, perm, box_start + bc.box0, k, g, bc.alpha, bc.cut2, bc.pre2,
+  real_space_body<MIXED, FORCE>(srt, x32, perm, box_start + bc.box0, k, g, bc.alpha, bc.cut2, bc.pre2,
                          pot, force, err + c);
 }
 
@@ -855,9 +902,8 @@ struct StressPair {
   double alpha, qi;
   double s[6] = {0, 0, 0, 0, 0, 0};  // xx, yy, zz, xy, xz, yz
   int bad = 0;
-  __device__ __forceinline__ void eval(const double4& e) {
-    const double d2 = e.x * e.x + e.y * e.y + e.z * e.z;
-    const double rr = sqrt(d2);
+  __device__ __forceinline__ void eval(const double4& e, double r2) {
+    const double rr = sqrt(r2);
     const double fac = alpha * rr;
     const double dr = (-2.0 / kSqrtPi * exp(-fac * fac) * fac - erfc(fac)) / (rr * rr * rr);
     const double w = dr * qi * e.w;
@@ -1081,12 +1127,10 @@ void launch_real_space(const double4* srt, const float4* x32, const int* perm,
   if (n == 0) return;
   const int blocks = blocks_for(static_cast<long>(n) * 32, kRealThreads);
   const float pre2 = prefilter_bound(g, r_cut);
-  if (mixed)
-    k_real_space<true><<<blocks, kRealThreads, 0, st>>>(srt, x32, perm, box_start, n, g, alpha,
-                                                        r_cut * r_cut, pre2, pot, force, err);
-  else
-    k_real_space<false><<<blocks, kRealThreads, 0, st>>>(srt, x32, perm, box_start, n, g, alpha,
-                                                         r_cut * r_cut, pre2, pot, force, err);
+  auto kernel = mixed ? (force ? k_real_space<true, true> : k_real_space<true, false>)
+                      : (force ? k_real_space<false, true> : k_real_space<false, false>);
+  kernel<<<blocks, kRealThreads, 0, st>>>(srt, x32, perm, box_start, n, g, alpha, r_cut * r_cut,
+                                          pre2, pot, force, err);
   ++g_launches;
 }
 
@@ -1095,14 +1139,10 @@ void launch_real_space_seg(const BatchLaunch& b, const double4* s4s, const float
                            int* cell_err, cudaStream_t st) {
   if (b.n_atoms == 0) return;
   const int blocks = blocks_for(static_cast<long>(b.n_atoms) * 32, kRealThreads);
-  if (b.mixed)
-    k_real_space_seg<true><<<blocks, kRealThreads, 0, st>>>(b.cells, b.p_atoms, b.ncells, s4s, x32,
-                                                            perm, box_start, b.n_atoms, pot,
-                                                            force, cell_err);
-  else
-    k_real_space_seg<false><<<blocks, kRealThreads, 0, st>>>(b.cells, b.p_atoms, b.ncells, s4s,
-                                                             x32, perm, box_start, b.n_atoms, pot,
-                                                             force, cell_err);
+  auto kernel = b.mixed ? (force ? k_real_space_seg<true, true> : k_real_space_seg<true, false>)
+                        : (force ? k_real_space_seg<false, true> : k_real_space_seg<false, false>);
+  kernel<<<blocks, kRealThreads, 0, st>>>(b.cells, b.p_atoms, b.ncells, s4s, x32, perm, box_start,
+                                          b.n_atoms, pot, force, cell_err);
   ++g_launches;
 }
 
