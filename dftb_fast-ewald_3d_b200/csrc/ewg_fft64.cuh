@@ -200,35 +200,17 @@ __device__ __forceinline__ void z_body(const PassCell& pc, int local, int nz,
   const bool kin = k1 < K1;
   const size_t zstride = static_cast<size_t>(K2) * K1;
   const size_t at = static_cast<size_t>(k2i) * K1 + (kin ? k1 : 0);
-  const cx<double>* src = static_cast<const cx<double>*>(pc.A2) + at;
   const typename SH::template At<8> t;
   if (t.i < R1) {
+    // Addresses one from the other: as offsets of one pointer they would hold two
+    // registers each.
+    const cx<double>* src = static_cast<const cx<double>*>(pc.A2) + at + t.i * zstride;
+    const size_t step = R1 * zstride;
     cx<double> u[R0];
 #pragma unroll
-    for (int j = 0; j < R0; ++j) u[j] = src[(t.i + j * R1) * zstride];
+    for (int j = 0; j < R0; ++j, src += step) u[j] = *src;
     SH::template first<-1, 8>(t, u, a);
   }
-  // The mode's share of the weight that does not depend on k3.
-  constexpr double twoPi = 2.0 * 3.14159265358979323846;
-  const double inv4a2 = 1.0 / (4.0 * (pc.g.alpha * pc.g.alpha));
-  // c(k) = ([k in S] + [-k in S]) / 2, S_d = [M/2 - M, M/2 - 1]: per axis the
-  // flags of k_d and -k_d (k_d = -M/2 of an even M lies in S, +M/2 does not).
-  const int lo1 = pc.g.M[0] / 2 - pc.g.M[0], hi1 = pc.g.M[0] / 2 - 1;
-  const int lo2 = pc.g.M[1] / 2 - pc.g.M[1], hi2 = pc.g.M[1] / 2 - 1;
-  const int lo3 = pc.g.M[2] / 2 - pc.g.M[2], hi3 = pc.g.M[2] / 2 - 1;
-  const int in12 = (k1 >= lo1 && k1 <= hi1 && k2 >= lo2 && k2 <= hi2) ? 1 : 0;
-  const int im12 = (-k1 >= lo1 && -k1 <= hi1 && -k2 >= lo2 && -k2 <= hi2) ? 1 : 0;
-  const double w12 = kin ? 4.0 * 3.14159265358979323846 / pc.g.volume * pc.corr2[0][k1 + h1] *
-                               pc.corr2[1][k2i]
-                         : 0.0;
-  double b12[3], b3[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    b12[c] = twoPi * (k1 * pc.g.rec[0][c] + k2 * pc.g.rec[1][c]);
-    b3[c] = twoPi * pc.g.rec[2][c];
-  }
-  const double* corr3 = pc.corr2[2];
-  double sv[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   __syncthreads();
   if (t.i < R0) {
     cx<double> v[R1];
@@ -242,35 +224,60 @@ __device__ __forceinline__ void z_body(const PassCell& pc, int local, int nz,
         q[(e - n3 + h3) * L + line] = v[j];
     }
   }
-  // Each thread weights the modes that it has put into q itself (no barrier), in
-  // a loop that is not unrolled: inlined into the transform, one exponential and
-  // one division per output cost it 100 registers.
-#pragma unroll 1
-  for (int e = t.i; t.i < R0 && e < n3; e += R0) {
-    if (e > h3 && e < n3 - h3) continue;
-    const int k3 = e <= h3 ? e : e - n3;
-    const double kx = fma(static_cast<double>(k3), b3[0], b12[0]);
-    const double ky = fma(static_cast<double>(k3), b3[1], b12[1]);
-    const double kz = fma(static_cast<double>(k3), b3[2], b12[2]);
-    const double kk2 = kx * kx + ky * ky + kz * kz;
-    const int in3 = (k3 >= lo3 && k3 <= hi3) ? in12 : 0, im3 = (-k3 >= lo3 && -k3 <= hi3) ? im12 : 0;
-    const cx<double> v = q[(k3 + h3) * L + line];
-    double wt = 0.0;
-    if (kk2 >= 1.0e-24 && in3 + im3 > 0 && !(k1 == 0 && k2 == 0 && k3 == 0)) {
-      const double ik2 = 1.0 / kk2;
-      wt = 0.5 * (in3 + im3) * w12 * exp(-kk2 * inv4a2) * ik2 * corr3[k3 + h3];
-      if constexpr (STRESS) {
-        const double en = (k1 > 0 ? 1.0 : 0.5) * wt * (v.x * v.x + v.y * v.y);
-        const double f = 2.0 * (inv4a2 + ik2);
-        sv[0] += en * (f * kx * kx - 1.0);
-        sv[1] += en * (f * ky * ky - 1.0);
-        sv[2] += en * (f * kz * kz - 1.0);
-        sv[3] += en * f * kx * ky;
-        sv[4] += en * f * kx * kz;
-        sv[5] += en * f * ky * kz;
-      }
+  // Influence weights.  Each thread weights the modes that it has put into q itself
+  // (no barrier), two at a time: inlined into the transform, one exponential and one
+  // division per output cost it 100 registers, and one at a time they are a chain
+  // of latencies.
+  constexpr double twoPi = 2.0 * 3.14159265358979323846;
+  double sv[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  if (t.i < R0) {
+    // The mode's share of the weight that does not depend on k3.
+    const double inv4a2 = 1.0 / (4.0 * (pc.g.alpha * pc.g.alpha));
+    // c(k) = ([k in S] + [-k in S]) / 2, S_d = [M/2 - M, M/2 - 1]: per axis the
+    // flags of k_d and -k_d (k_d = -M/2 of an even M lies in S, +M/2 does not).
+    const int lo1 = pc.g.M[0] / 2 - pc.g.M[0], hi1 = pc.g.M[0] / 2 - 1;
+    const int lo2 = pc.g.M[1] / 2 - pc.g.M[1], hi2 = pc.g.M[1] / 2 - 1;
+    const int lo3 = pc.g.M[2] / 2 - pc.g.M[2], hi3 = pc.g.M[2] / 2 - 1;
+    const bool in12 = k1 >= lo1 && k1 <= hi1 && k2 >= lo2 && k2 <= hi2;
+    const bool im12 = -k1 >= lo1 && -k1 <= hi1 && -k2 >= lo2 && -k2 <= hi2;
+    const double w12 = kin ? 2.0 * 3.14159265358979323846 / pc.g.volume * pc.corr2[0][k1 + h1] *
+                                 pc.corr2[1][k2i]
+                           : 0.0;
+    const double* corr3 = pc.corr2[2] + h3;
+    double b12[3], b3[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      b12[c] = twoPi * (k1 * pc.g.rec[0][c] + k2 * pc.g.rec[1][c]);
+      b3[c] = twoPi * pc.g.rec[2][c];
     }
-    q[(k3 + h3) * L + line] = mk(wt * v.x, wt * v.y);
+#pragma unroll 2
+    for (int e = t.i; e < n3; e += R0) {
+      if (e > h3 && e < n3 - h3) continue;
+      const int k3 = e <= h3 ? e : e - n3;
+      const double kx = fma(static_cast<double>(k3), b3[0], b12[0]);
+      const double ky = fma(static_cast<double>(k3), b3[1], b12[1]);
+      const double kz = fma(static_cast<double>(k3), b3[2], b12[2]);
+      const double kk2 = kx * kx + ky * ky + kz * kz;
+      const double ik2 = 1.0 / kk2;
+      const int in3 = (in12 && k3 >= lo3 && k3 <= hi3) + (im12 && -k3 >= lo3 && -k3 <= hi3);
+      const bool on = kk2 >= 1.0e-24 && (k1 != 0 || k2 != 0 || k3 != 0) && in3 > 0;
+      const double wt = on ? in3 * w12 * exp(-kk2 * inv4a2) * ik2 * corr3[k3] : 0.0;
+      cx<double>* m = q + (k3 + h3) * L + line;
+      const cx<double> v = *m;
+      if constexpr (STRESS) {
+        if (on) {
+          const double en = (k1 > 0 ? 1.0 : 0.5) * wt * (v.x * v.x + v.y * v.y);
+          const double f = 2.0 * (inv4a2 + ik2);
+          sv[0] += en * (f * kx * kx - 1.0);
+          sv[1] += en * (f * ky * ky - 1.0);
+          sv[2] += en * (f * kz * kz - 1.0);
+          sv[3] += en * f * kx * ky;
+          sv[4] += en * f * kx * kz;
+          sv[5] += en * f * ky * kz;
+        }
+      }
+      *m = mk(wt * v.x, wt * v.y);
+    }
   }
   __syncthreads();
   if constexpr (STRESS) {  // fixed-order CTA sum: shuffle tree per warp, then warps in order
@@ -294,31 +301,36 @@ __device__ __forceinline__ void z_body(const PassCell& pc, int local, int nz,
       stress[static_cast<size_t>(local) * 6 + threadIdx.x] = t;
     }
   }
-  cx<double>* dst = static_cast<cx<double>*>(pc.B2) + at;
+#pragma unroll 1
   for (int c = 0; c < nz; ++c) {
-    if (t.i < R1) {
+    // An index that the compiler takes for a new one in each round: it would keep
+    // the rounds' common factors and twiddles, 50 registers of them, across both.
+    typename SH::template At<8> r = t;
+    asm volatile("" : "+r"(r.i));
+    if (r.i < R1) {
       cx<double> u[R0];
 #pragma unroll
       for (int j = 0; j < R0; ++j) {
-        const int e = t.i + j * R1, k3 = e <= h3 ? e : e - n3;
+        const int e = r.i + j * R1, k3 = e <= h3 ? e : e - n3;
         u[j] = mk(0.0, 0.0);
         if (e <= h3 || e >= n3 - h3) {
           u[j] = q[(k3 + h3) * L + line];
           if (c > 0) u[j] = times_i(u[j], twoPi * k3);  // 2 pi i k3 v
         }
       }
-      SH::template first<1, 8>(t, u, a);
+      SH::template first<1, 8>(r, u, a);
     }
     __syncthreads();
-    if (t.i < R0) {
+    if (r.i < R0) {
       cx<double> v[R1];
-      SH::template second<1, 8>(t, a, tw, v);
-      if (kin) {
+      SH::template second<1, 8>(r, a, tw, v);
+      cx<double>* dst = static_cast<cx<double>*>(pc.B2) + at +
+                        (static_cast<size_t>(c) * n3 + r.i) * zstride;
+      const size_t step = R0 * zstride;
 #pragma unroll
-        for (int j = 0; j < R1; ++j) dst[(t.i + j * R0) * zstride] = v[j];
-      }
+      for (int j = 0; j < R1; ++j, dst += step)
+        if (kin) *dst = v[j];
     }
-    dst += n3 * zstride;
     __syncthreads();
   }
 }
@@ -435,8 +447,14 @@ __device__ __forceinline__ void pass64_body(const PassCell& pc, int local, int n
   if constexpr (PASS == P64_C2R) x_c2r_body<SH, VAR>(pc, local);
 }
 
+// CTAs per SM that the z pass's registers are bounded for (without spills: 92 at radices
+// up to 16, 168 above); unbounded it took 144 and 255, 12 and 6 warps an SM.
+constexpr int min_blocks64(int pass, int threads) {
+  return pass == P64_Z ? (threads <= 128 ? 5 : 2) : 0;
+}
+
 template <class SH, int PASS, int VAR>
-__global__ void __launch_bounds__(SH::threads) k64_pass(const __grid_constant__ PassCell pc, int nz,
+__global__ void __launch_bounds__(SH::threads, min_blocks64(PASS, SH::threads)) k64_pass(const __grid_constant__ PassCell pc, int nz,
                                                         double* __restrict__ stress) {
   chain_enter();
   pass64_body<SH, PASS, VAR>(pc, blockIdx.x, nz, stress);
