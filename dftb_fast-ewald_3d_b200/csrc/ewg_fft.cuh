@@ -52,6 +52,29 @@ __device__ __forceinline__ cx<R> scale(cx<R> a, R s) {
   return mk(a.x * s, a.y * s);
 }
 
+// An element of global memory, or zero: a predicated load.  (As a branch around the
+// load, the compiler waited for a part of a thread's loads before it issued the
+// next: the y inverse and x C2R passes of 216,000 sites took 779 and 1022 us for 262
+// and 561.)
+__device__ __forceinline__ cx<double> load_if(const cx<double>* p, bool take) {
+  cx<double> v;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
+      "mov.f64 %1, 0d0000000000000000;\n\t@q ld.global.v2.f64 {%0, %1}, [%2];\n\t}"
+      : "=&d"(v.x), "=&d"(v.y)
+      : "l"(p), "r"(static_cast<int>(take)));
+  return v;
+}
+__device__ __forceinline__ cx<float> load_if(const cx<float>* p, bool take) {
+  cx<float> v;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+      "mov.f32 %1, 0f00000000;\n\t@q ld.global.v2.f32 {%0, %1}, [%2];\n\t}"
+      : "=&f"(v.x), "=&f"(v.y)
+      : "l"(p), "r"(static_cast<int>(take)));
+  return v;
+}
+
 template <typename R>
 __device__ __forceinline__ cx<R> twiddle(const cx<R>* __restrict__ tw, int e, int sign) {
   cx<R> w = tw[e];

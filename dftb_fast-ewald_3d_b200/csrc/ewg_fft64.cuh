@@ -97,18 +97,6 @@ struct TwoPass {
   }
 };
 
-// An element of global memory, or zero: a predicated load.  (As a branch around the
-// load, the compiler waited for a part of a thread's loads before it issued the
-// next.)
-__device__ __forceinline__ cx<double> load_if(const cx<double>* p, bool take) {
-  cx<double> v;
-  asm volatile(
-      "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
-      "mov.f64 %1, 0d0000000000000000;\n\t@q ld.global.v2.f64 {%0, %1}, [%2];\n\t}"
-      : "=&d"(v.x), "=&d"(v.y)
-      : "l"(p), "r"(static_cast<int>(take)));
-  return v;
-}
 __device__ __forceinline__ cx<double> times_i(cx<double> v, double f) { return mk(-f * v.y, f * v.x); }
 
 // x, real to complex: row pairs (2p, 2p+1) form one complex line; k1 = 0..K1-1

@@ -305,14 +305,8 @@ __device__ __forceinline__ void fft_y_inv_body(int bx, int by, int bz, const cx<
   const cx<R>* src = B2 + ((static_cast<size_t>(cs) * n3 + i3) * K2 + H2) * K1 + kl;
   cx<R>* dst = B1 + (static_cast<size_t>(c) * n3 + i3) * n2 * K1 + kl;
   auto load = [&](int, int i2) {
-    int k2;
-    if (i2 <= H2)
-      k2 = i2;
-    else if (i2 >= n2 - H2)
-      k2 = i2 - n2;
-    else
-      return mk(R(0), R(0));
-    cx<R> v = kin ? src[k2 * K1] : mk(R(0), R(0));
+    const int k2 = i2 <= H2 ? i2 : i2 - n2;
+    cx<R> v = load_if(src + k2 * K1, kin && (i2 <= H2 || i2 >= n2 - H2));
     if (dk2) {
       const R t = static_cast<R>(2.0 * 3.14159265358979323846 * k2);
       v = mk(-t * v.y, t * v.x);
@@ -361,24 +355,17 @@ __device__ __forceinline__ void fft_x_c2r_body(int bx, int by, const cx<R>* __re
   auto load = [&](int, int x) {
     const bool lo = x < K1;
     const bool hi = x > n1 - K1;
-    cx<R> fa = mk(R(0), R(0)), fb = mk(R(0), R(0));
-    if (valid && (lo || hi)) {
-      const int kx = lo ? x : n1 - x;
-      fa = sa[kx];
-      fb = sb[kx];
-      if (dk1) {
-        const R t = static_cast<R>(2.0 * 3.14159265358979323846 * kx);
-        fa = mk(-t * fa.y, t * fa.x);
-        fb = mk(-t * fb.y, t * fb.x);
-      }
-      if (x == 0) {
-        fa.y = R(0);
-        fb.y = R(0);
-      } else if (hi) {
-        fa.y = -fa.y;
-        fb.y = -fb.y;
-      }
+    const int kx = lo ? x : n1 - x;
+    const bool in = valid && (lo || hi);
+    cx<R> fa = load_if(sa + kx, in), fb = load_if(sb + kx, in);
+    if (dk1) {
+      const R t = static_cast<R>(2.0 * 3.14159265358979323846 * kx);
+      fa = mk(-t * fa.y, t * fa.x);
+      fb = mk(-t * fb.y, t * fb.x);
     }
+    const R s = x == 0 ? R(0) : (hi && !lo ? R(-1) : R(1));  // exact factors
+    fa.y = s * fa.y;
+    fb.y = s * fb.y;
     return mk(fa.x - fb.y, fa.y + fb.x);
   };
   auto store = [&](int, int x, cx<R> v, cx<R>*) {
