@@ -388,9 +388,9 @@ int mesh_geometry(const Cell& cell, const ewg_params& p, bool mixed, MeshGeom& g
   return EWG_OK;
 }
 
-// Particle-side tiling: per axis the most tiles one stencil can touch
-// (brute force over start points, so partial last tiles are covered) and the
-// per-atom weight layout.
+// Particle-side tiling: per axis the most tiles one stencil can touch (with a part
+// tile at the end of the axis by brute force over the start points) and the per-atom
+// weight layout.
 void stencil_dims(const MeshGeom& g, bool ad, StencilDims& sd) {
   int off = 0;
   for (int d = 0; d < 3; ++d) {
@@ -399,7 +399,10 @@ void stencil_dims(const MeshGeom& g, bool ad, StencilDims& sd) {
     sd.T[d] = T;
     sd.ntiles[d] = nt;
     int most = nt;
-    if (g.W < n) {
+    if (g.W < n && n % T == 0) {
+      // Whole tiles: the most from a start on the last point of a tile.
+      most = std::min(nt, (g.W + T - 2) / T + 1);
+    } else if (g.W < n) {
       // Walk each start point's stencil through the tiles, as the weights kernel does.
       most = 1;
       for (int c = 0; c < n; ++c) {
@@ -2560,6 +2563,14 @@ int ewg_batch_potential_force_ov(ewg_context* c, int n_cells, const int* offsets
   // evaluations are queued with no host wait.
   int* cellerr = dbuf<int>(c, B_CELLERR, std::max(n_cells, 1), &rc);
   if (rc) return rc;
+  // The uploads go first and run while the host checks and plans the cells; every
+  // return after them waits for them (the caller's arrays must outlive the copies).
+  cudaMemcpyAsync(dcoords, coords, sizeof(double) * 3 * total, cudaMemcpyHostToDevice, c->stream);
+  cudaMemcpyAsync(dq, charges, sizeof(double) * total, cudaMemcpyHostToDevice, c->stream);
+  auto fail = [&](int code) {
+    cudaStreamSynchronize(c->stream);
+    return code;
+  };
   // The lanes: the context itself when one lane is asked for (or profiling is
   // on, which times stages on the context's own stream), else sub-contexts of
   // the same device, form and settings, each with its own buffers and streams.
@@ -2593,8 +2604,8 @@ int ewg_batch_potential_force_ov(ewg_context* c, int n_cells, const int* offsets
   SegPlan sp;
   SegBufs sb{};
   if (segmented) {
-    if ((rc = seg_plan(c, n_cells, offsets, cells, params, force != nullptr, sp))) return rc;
-    if ((rc = seg_prepare(c, sp, sb))) return rc;
+    if ((rc = seg_plan(c, n_cells, offsets, cells, params, force != nullptr, sp))) return fail(rc);
+    if ((rc = seg_prepare(c, sp, sb))) return fail(rc);
   }
   const int nl = segmented ? 1
                  : c->prof.on ? 1
@@ -2602,23 +2613,22 @@ int ewg_batch_potential_force_ov(ewg_context* c, int n_cells, const int* offsets
   if (nl > 1) {
     while (static_cast<int>(c->lanes.size()) < nl) {
       ewg_context* l = nullptr;
-      if ((rc = ewg_create(&l, c->device, c->precision))) return rc;
+      if ((rc = ewg_create(&l, c->device, c->precision))) return fail(rc);
       c->lanes.push_back(l);
       cudaEvent_t e;
-      if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return EWG_ERR_CUDA;
+      if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+        return fail(EWG_ERR_CUDA);
       c->lane_done.push_back(e);
     }
     if (!c->lanes_ready &&
         cudaEventCreateWithFlags(&c->lanes_ready, cudaEventDisableTiming) != cudaSuccess)
-      return EWG_ERR_CUDA;
+      return fail(EWG_ERR_CUDA);
     for (int l = 0; l < nl; ++l) {
       c->lanes[l]->force_scheme = c->force_scheme;
       c->lanes[l]->background = c->background;
       c->lanes[l]->graphs_on = c->graphs_on;
     }
   }
-  cudaMemcpyAsync(dcoords, coords, sizeof(double) * 3 * total, cudaMemcpyHostToDevice, c->stream);
-  cudaMemcpyAsync(dq, charges, sizeof(double) * total, cudaMemcpyHostToDevice, c->stream);
   // The device work of the whole batch: the cells round-robin on the lanes,
   // forked from and joined back to the context's stream.
   auto launch_batch = [&]() -> int {
