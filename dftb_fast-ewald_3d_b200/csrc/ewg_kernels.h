@@ -84,9 +84,9 @@ void launch_atom_sort(const double* pos, long sa, long sd, const double* q, int 
 void launch_refresh_charges(const double* q, const int* perm, int n, double4* s4s, float4* x32,
                             void* qk, int mixed, cudaStream_t st);
 
-// Exclusive scan of counts[0..nkeys) into starts[0..nkeys] (one CTA), chained
-// to the stream's previous kernel when after_kernel.
-void launch_scan(const int* counts, int nkeys, int* starts, bool after_kernel, cudaStream_t st);
+// Exclusive scan of counts[0..nkeys), nkeys > 0, into starts[0..nkeys], chained to the
+// stream's previous kernel.
+void launch_scan(const int* counts, int nkeys, int* starts, cudaStream_t st);
 
 // Charge sums for the parameter chain on device-resident charges:
 // out[0] = sum q, out[1] = sum |q|, out[2] = sum q^2 (fixed-order reduction).

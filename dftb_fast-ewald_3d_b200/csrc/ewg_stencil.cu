@@ -1195,8 +1195,12 @@ __device__ __forceinline__ void gather_tiles_dmma_body(int tx, int ty, int tz,
         const int ps = pr.y;
         const int sidx = ((ps >> 16) * sd.S[1] + ((ps >> 8) & 0xff)) * sd.S[0] + (ps & 0xff);
         double* dst = part + (static_cast<size_t>(pr.x) * nslots + sidx) * NC;
-#pragma unroll
-        for (int c = 0; c < NC; ++c) dst[c] = acc[c];
+        if constexpr (NC == 4) {
+          reinterpret_cast<double2*>(dst)[0] = make_double2(acc[0], acc[1]);
+          reinterpret_cast<double2*>(dst)[1] = make_double2(acc[2], acc[3]);
+        } else {
+          dst[0] = acc[0];
+        }
       }
     }
   }
@@ -1311,8 +1315,8 @@ __device__ __forceinline__ void gather_tiles_dmma_ad_body(
       const int ps = pr.y;
       const int sidx = ((ps >> 16) * sd.S[1] + ((ps >> 8) & 0xff)) * sd.S[0] + (ps & 0xff);
       double* dst = part + (static_cast<size_t>(pr.x) * nslots + sidx) * 4;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) dst[c] = acc[c];
+      reinterpret_cast<double2*>(dst)[0] = make_double2(acc[0], acc[1]);
+      reinterpret_cast<double2*>(dst)[1] = make_double2(acc[2], acc[3]);
     }
   }
 }
@@ -1351,8 +1355,16 @@ __device__ __forceinline__ void gather_final_body(const int4* __restrict__ slot,
   for (int s = lane; s < (live ? nslots : 0); s += LPA) {
     const int sx = s % sd.S[0], sy = (s / sd.S[0]) % sd.S[1], sz = s / (sd.S[0] * sd.S[1]);
     if (sx < cx && sy < cy && sz < cz) {  // slots past the atom's tiles hold no partial
-#pragma unroll
-      for (int c = 0; c < NC; ++c) acc[c] += pk[s * NC + c];
+      if constexpr (NC == 4) {  // a slot's four values, 32 bytes, in two loads
+        const double2 p0 = reinterpret_cast<const double2*>(pk)[2 * s];
+        const double2 p1 = reinterpret_cast<const double2*>(pk)[2 * s + 1];
+        acc[0] += p0.x;
+        acc[1] += p0.y;
+        acc[2] += p1.x;
+        acc[3] += p1.y;
+      } else {
+        acc[0] += pk[s];
+      }
     }
   }
   // A fixed shuffle tree within the atom's LPA lanes.
@@ -1566,7 +1578,7 @@ void weights_bins(const MeshPlan& mp, const double4* s4s, int n, R* wtab, R* qk,
     k_pair_count<<<blocks_for(items, 256), 256, 0, st>>>(slot, n, sd, b.counts, b.arrival);
     g_launches += 2;
   }
-  launch_scan(b.counts, ntiles, b.starts, true, st);
+  launch_scan(b.counts, ntiles, b.starts, st);
   launch_chained(k_pair_scatter, blocks_for(items, 256), 256, 0, st, slot, n, sd, b.starts,
                  b.arrival, b.unordered);
   ++g_launches;
@@ -1724,7 +1736,7 @@ void weights_bins_seg(const BatchLaunch& b, const double4* s4s, R* wtab, R* qk, 
         b.cells, b.p_slots, b.ncells, b.n_slots, slot, pb.counts, pb.arrival);
     g_launches += 2;
   }
-  launch_scan(pb.counts, b.n_tiles, pb.starts, true, st);
+  launch_scan(pb.counts, b.n_tiles, pb.starts, st);
   launch_chained(k_pair_scatter_seg, blocks_for(b.n_slots, 256), 256, 0, st, b.cells, b.p_slots,
                  b.ncells, b.n_slots, slot, pb.starts, pb.arrival, pb.unordered);
   ++g_launches;
