@@ -29,7 +29,7 @@ enum BufId {
   B_BCOUNTS, B_BTMP, B_EXT_T, B_EXT_S, B_EXT_SQ, B_EXT_TQ, B_EXT_BLUR, B_EXT_R,
   B_EXT_G, B_EXT_SF, B_EXT_SF2, B_EXT_OUT, B_EXT_OUT2, B_X32S, B_TUNE_POT, B_TUNE_FORCE,
   // mesh-based point potentials: source (S) and target (T) tables
-  B_PT_S4, B_PT_S4S, B_PT_SKEY, B_PT_SPERM, B_PT_SBOX, B_PT_SWT,
+  B_PT_S4, B_PT_S4S, B_PT_X32, B_PT_SKEY, B_PT_SPERM, B_PT_SBOX, B_PT_SWT,
   B_PT_SQK, B_PT_SSLOT, B_PT_SPAIRS, B_PT_SPSTART, B_PT_T4S, B_PT_TPERM, B_PT_TBOX,
   B_PT_TWT, B_PT_TQK, B_PT_TSLOT, B_PT_TPAIRS, B_PT_TPSTART, B_PT_BCNT,
   B_PT_BTMP, B_PT_KCNT, B_PT_PARR, B_PT_PTMP, B_PT_QNEG, B_PT_PART, B_PT_POTSR, B_PT_GRADSR,
@@ -2182,6 +2182,7 @@ int points_mesh(ewg_context* c, const Cell& cell, double tol, int nt, const doub
   const int tpairs = nt * tgt.sd.S[0] * tgt.sd.S[1] * tgt.sd.S[2];
   double4* s4 = dbuf<double4>(c, B_PT_S4, nmax, &rc);
   double4* s4s = dbuf<double4>(c, B_PT_S4S, ns, &rc);
+  float4* x32 = dbuf<float4>(c, B_PT_X32, ns, &rc);
   double4* t4s = dbuf<double4>(c, B_PT_T4S, nt, &rc);
   int* skey = dbuf<int>(c, B_PT_SKEY, nmax, &rc);
   int* sperm = dbuf<int>(c, B_PT_SPERM, ns, &rc);
@@ -2223,7 +2224,7 @@ int points_mesh(ewg_context* c, const Cell& cell, double tol, int nt, const doub
   // Sources: box order for the real-space cell list and the mesh tables.
   const PairBins sbins{kcnt, parr, spstart, ptmp, spairs_d};
   launch_atom_sort(ds, 3, 1, dq, ns, cell, rg.nb,
-                   SortBufs{s4, skey, bcnt, btmp, sbox, sperm, s4s, nullptr}, kcnt, ntiles, st);
+                   SortBufs{s4, skey, bcnt, btmp, sbox, sperm, s4s, x32}, kcnt, ntiles, st);
   // Fourier sum: spread the sources, transform, weight, invert, gather.
   launch_weights_bins(src, s4s, ns, swt, sqk, sslot, sbins, st);
   launch_spread(src, sbins, sslot, ns, false, swt, sqk, grid, st);
@@ -2237,20 +2238,25 @@ int points_mesh(ewg_context* c, const Cell& cell, double tol, int nt, const doub
                       st);
   launch_gather(tgt, tpstart, tpairs_d, twt, outg, 1, part, st);
   // Real-space sum over the source cell list.
-  PointsReal pr;
-  for (int d = 0; d < 3; ++d) {
-    pr.nb[d] = rg.nb[d];
-    pr.R[d] = rg.R[d];
-    for (int e = 0; e < 3; ++e) {
-      pr.lat[d][e] = cell.lat[d][e];
-      pr.rec[d][e] = cell.rec[d][e];
+  if (!sblur && !tblur) {
+    launch_points_flat(nt, t4s, tperm, dt, s4s, x32, sperm, ds, sbox, rg, p.alpha, r_pair, potsr,
+                       want_grad ? gradsr : nullptr, st);
+  } else {
+    PointsReal pr;
+    for (int d = 0; d < 3; ++d) {
+      pr.nb[d] = rg.nb[d];
+      pr.R[d] = rg.R[d];
+      for (int e = 0; e < 3; ++e) {
+        pr.lat[d][e] = cell.lat[d][e];
+        pr.rec[d][e] = cell.rec[d][e];
+      }
     }
+    pr.r_cut2 = r_pair * r_pair;
+    pr.alpha = p.alpha;
+    pr.want_pot = 1;
+    pr.want_grad = want_grad ? 1 : 0;
+    launch_points_real(nt, dt, tblur, ns, s4s, sperm, ds, sblur, sbox, pr, potsr, gradsr, st);
   }
-  pr.r_cut2 = r_pair * r_pair;
-  pr.alpha = p.alpha;
-  pr.want_pot = 1;
-  pr.want_grad = want_grad ? 1 : 0;
-  launch_points_real(nt, dt, tblur, ns, s4s, sperm, ds, sblur, sbox, pr, potsr, gradsr, st);
   const double shift = -kPi * qsum / (cell.volume * p.alpha * p.alpha);
   launch_gather_final(tgt, tslot, tperm, part, want_grad ? 4 : 1, nt, qneg, 0.0, shift, potsr,
                       gradsr, pot_out, dgrad, want_grad ? cell.rec : nullptr, st);

@@ -883,6 +883,105 @@ __global__ void __launch_bounds__(kRealThreads, 16) k_real_space_seg(
                          pot, force, err + c);
 }
 
+// ---------------------------------------------------------------------------
+// Real-space half of the mesh-based point potentials without blur: per target the
+// pair terms of ewaldReal / derivEwaldReal (dftb/coulomb.F90:2520-2625) over the
+// sources within the cutoff, by the flat candidate scan and queue of the atoms' sum
+// (a lane per box and its sources in turn, with every distance in FP64, took 4 times
+// as long).  The targets go in their own box order, so that neighbouring warps share
+// the sources they read.
+// ---------------------------------------------------------------------------
+constexpr double kTolSameDist2 = 1.0e-5 * 1.0e-5;  // common/accuracy.F90:69, squared
+
+template <bool GRAD>
+struct PointQueue : QueueBase<EwaldPair<GRAD>, int4> {
+  const double4* __restrict__ srt;
+  double4 ai;
+  const RealGeom* g;
+  double cut2;
+  float pre2;
+  const double* x;                    // the target's Cartesian position
+  const double* __restrict__ sc;      // sources' positions and order
+  const int* __restrict__ sperm;
+  __device__ __forceinline__ PointQueue(int4* qbuf, EwaldPair<GRAD>& p, const double4* s,
+                                        const double4& a, const RealGeom& geo, double c2, float p2,
+                                        const double* xt, const double* sources, const int* order)
+      : QueueBase<EwaldPair<GRAD>, int4>(qbuf, p), srt(s), ai(a), g(&geo), cut2(c2), pre2(p2),
+        x(xt), sc(sources), sperm(order) {}
+  __device__ __forceinline__ void eval_entry(const int4& e) {
+    const double4 aj = srt[e.x];
+    const double d1 = (ai.x - aj.x) - small_double(e.y), d2 = (ai.y - aj.y) - small_double(e.z),
+                 d3 = (ai.z - aj.z) - small_double(e.w);
+    double sep[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sep[c] = d1 * g->lat[0][c] + d2 * g->lat[1][c] + d3 * g->lat[2][c];
+    const double r2 = sep[0] * sep[0] + sep[1] * sep[1] + sep[2] * sep[2];
+    if (r2 > cut2) return;
+    if (r2 >= kTolSameDist2) {
+      this->pair.eval(make_double4(sep[0], sep[1], sep[2], aj.w), r2);
+      return;
+    }
+    // ewaldReal skips the coincident image; ewald subtracts the self term when the two
+    // points themselves (not an image) coincide.  derivEwaldReal skips r below the
+    // squared tolerance (a distance against a squared tolerance, as the reference
+    // writes it).
+    const double p = this->pair.pot;
+    if (r2 >= kTolSameDist2 * kTolSameDist2)
+      this->pair.eval(make_double4(sep[0], sep[1], sep[2], aj.w), r2);
+    this->pair.pot = p;
+    const double* y = sc + 3 * static_cast<size_t>(sperm[e.x]);
+    const double c0 = x[0] - y[0], c1 = x[1] - y[1], c2 = x[2] - y[2];
+    if (c0 * c0 + c1 * c1 + c2 * c2 < kTolSameDist2)
+      this->pair.pot -= 2.0 * this->pair.alpha / kSqrtPi * aj.w;
+  }
+  __device__ __forceinline__ void operator()(const Candidate& c) {
+    this->push(c.valid && c.r2 <= pre2, make_int4(c.j, c.sx, c.sy, c.sz),
+               [this](const int4& e) { eval_entry(e); });
+  }
+  __device__ __forceinline__ void flush() {
+    this->drain([this](const int4& e) { eval_entry(e); });
+  }
+};
+
+template <bool GRAD>
+__global__ void __launch_bounds__(kRealThreads, 16) k_points_flat(
+    int nt, const double4* __restrict__ t4s, const int* __restrict__ tperm,
+    const double* __restrict__ tc, const double4* __restrict__ srt,
+    const float4* __restrict__ x32, const int* __restrict__ sperm, const double* __restrict__ sc,
+    const int* __restrict__ box_start, RealGeom g, double alpha, double cut2, float pre2,
+    double* __restrict__ pot, double* __restrict__ grad) {
+  __shared__ __align__(16) int4 queue[kRealThreads / 32][kQueue];
+  __shared__ RunTable runs[kRealThreads / 32];
+  const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (k >= nt) return;
+  const int t = tperm[k];
+  const double4 ai = t4s[k];
+  EwaldPair<GRAD> pair;
+  pair.alpha = alpha;
+  pair.qi = -1.0;  // the force on a charge of -1 is the potential's gradient
+  PointQueue<GRAD> pq(queue[threadIdx.x >> 5], pair, srt, ai, g, cut2, pre2,
+                      tc + 3 * static_cast<size_t>(t), sc, sperm);
+  // No source is the target itself: index -1.
+  if (g.flat)
+    for_each_candidate_flat(x32, box_start, -1, ai, g, cut2 * (1.0 + 1e-9),
+                            runs[threadIdx.x >> 5], pq);
+  else
+    for_each_candidate(x32, box_start, -1, ai, g, pq);
+  pq.flush();
+  double v[4] = {pair.pot, pair.f[0], pair.f[1], pair.f[2]};
+#pragma unroll
+  for (int c = 0; c < (GRAD ? 4 : 1); ++c)
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], off);
+  if ((threadIdx.x & 31) == 0) {
+    pot[t] = v[0];
+    if (GRAD) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) grad[3 * static_cast<size_t>(t) + c] = v[1 + c];
+    }
+  }
+}
+
 // Real-space virial of invRStress with addNeighbourContribsStress
 // (coulomb.F90:2836-2905).  Over the full list with a factor 1/2 (the half
 // list's pairs each appear twice), r (x) f + f (x) r with f = derivRTerm(r) q_i q_j
@@ -1130,6 +1229,19 @@ void launch_real_space_seg(const BatchLaunch& b, const double4* s4s, const float
                         : (force ? k_real_space_seg<false, true> : k_real_space_seg<false, false>);
   kernel<<<blocks, kRealThreads, 0, st>>>(b.cells, b.p_atoms, b.ncells, s4s, x32, perm, box_start,
                                           b.n_atoms, pot, force, cell_err);
+  ++g_launches;
+}
+
+void launch_points_flat(int nt, const double4* t4s, const int* tperm, const double* tc,
+                        const double4* s4s, const float4* x32, const int* sperm, const double* sc,
+                        const int* box_start, const RealGeom& g, double alpha, double r_cut,
+                        double* pot, double* grad, cudaStream_t st) {
+  if (nt == 0) return;
+  const int blocks = blocks_for(static_cast<long>(nt) * 32, kRealThreads);
+  auto kernel = grad ? k_points_flat<true> : k_points_flat<false>;
+  kernel<<<blocks, kRealThreads, 0, st>>>(nt, t4s, tperm, tc, s4s, x32, sperm, sc, box_start, g,
+                                          alpha, r_cut * r_cut, prefilter_bound(g, r_cut), pot,
+                                          grad);
   ++g_launches;
 }
 
