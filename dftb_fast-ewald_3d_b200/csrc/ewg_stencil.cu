@@ -626,7 +626,11 @@ constexpr int kGatherAdWarps = 2;  // tensor-core gather with window derivatives
 // FP32 CUDA-core gather with window derivatives: one atom per lane (74 registers, so
 // about 13 CTAs per SM) and two warps per tile.
 constexpr int kGatherAdF32Atoms = 1, kGatherAdF32Warps = 2;
-constexpr int kSpreadAtoms = 32;  // tensor-core spread: atoms staged per round, one per lane
+// Tensor-core spread: atoms staged per round.  With 16 the rows take half the shared
+// memory and 28 instead of 20 warps fit an SM (216,000 sites 237 -> 217 us, a batch
+// of 128 cells 129 -> 112); where the tiles do not fill the SMs anyway, 32 take fewer
+// rounds (729 tiles 15.1 -> 13.8 us).
+constexpr int kSpreadFew = 16, kSpreadMany = 32, kSpreadFull = 148 * 20;
 constexpr int kSpreadList = 128;  // longest tile list that the spread orders in shared memory
 constexpr int kWRow = 12;         // doubles per staged weight row: 8 used; the
                                   // padding makes the fragment reads conflict-free
@@ -650,9 +654,13 @@ __device__ __forceinline__ void stage2(double* dst, const float* src) {
 }
 
 // One warp per tile owning all eight z-planes, so each step's x and y weights
-// are read from shared memory once for the eight planes; the lanes stage up to
-// 32 atoms' weight rows per round with asynchronous 16-byte copies.
-template <typename R>
+// are read from shared memory once for the eight planes.  Bound by the latency of
+// staging the weight rows, so the warps that fit an SM and the sectors per access
+// count: a row of 64 bytes is copied by four lanes (whole sectors; one lane a row
+// took 55.6 us at 32,769 atoms and 281 at 216,000 sites, this 43.7 and 203), and
+// the entries of a round are read before its first copy, which the compiler moves
+// no load across.
+template <typename R, int ATOMS>
 __device__ __forceinline__ void spread_tiles_dmma_body(int tx, int ty, int tz,
                                                        const int* __restrict__ tile_start,
                                                        const int2* __restrict__ unordered,
@@ -661,8 +669,8 @@ __device__ __forceinline__ void spread_tiles_dmma_body(int tx, int ty, int tz,
                                                        const StencilDims& sd,
                                                        R* __restrict__ grid) {
   chain_enter();
-  __shared__ __align__(16) double sW[3][kSpreadAtoms][kWRow];
-  __shared__ double sQ[kSpreadAtoms];
+  __shared__ __align__(16) double sW[3][ATOMS][kWRow];
+  __shared__ double sQ[ATOMS];
   const int tile = (tz * sd.ntiles[1] + ty) * sd.ntiles[0] + tx;
   const int x0 = tx * TX, y0 = ty * TY, z0 = tz * TZ;
   const int lane = threadIdx.x;
@@ -709,27 +717,33 @@ __device__ __forceinline__ void spread_tiles_dmma_body(int tx, int ty, int tz,
     }
     __syncwarp();
   }
-  for (int b0 = p0; b0 < p1; b0 += kSpreadAtoms) {
-    const int nb = min(kSpreadAtoms, p1 - b0);
+  for (int b0 = p0; b0 < p1; b0 += ATOMS) {
+    const int nb = min(ATOMS, p1 - b0);
     __syncwarp();  // the previous round's weights are no longer read
-    const int a = lane;
-    if (a < nb) {
-      const int2 pr = in_shared ? sList[b0 - p0 + a] : pairs[b0 + a];
-      const R* wk = wtab + static_cast<size_t>(pr.x) * sd.wstride;
-      const R* src[3] = {wk + sd.woff[0] + (pr.y & 0xff) * TX,
-                         wk + sd.woff[1] + ((pr.y >> 8) & 0xff) * TY,
-                         wk + sd.woff[2] + (pr.y >> 16) * TZ};
+    // Four lanes per weight row of 64 bytes, whole sectors to an access; all entries
+    // before the first copy, which the compiler does not move loads across.
+    int2 pr[ATOMS / 8];
+    R q[ATOMS / 8];
 #pragma unroll
-      for (int d = 0; d < 3; ++d)
+    for (int h = 0; h < ATOMS / 8; ++h) {
+      const int a = h * 8 + fr;
+      pr[h] = a >= nb ? make_int2(0, 0) : (in_shared ? sList[b0 - p0 + a] : pairs[b0 + a]);
+    }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) stage2(&sW[d][a][2 * j], src[d] + 2 * j);
-      sQ[a] = qk[pr.x];
-    } else if (a < ((nb + 3) & ~3)) {  // padding atoms of the last group of four
+    for (int h = 0; h < ATOMS / 8; ++h) q[h] = fk == 0 && h * 8 + fr < nb ? qk[pr[h].x] : R(0);
 #pragma unroll
-      for (int d = 0; d < 3; ++d)
+    for (int h = 0; h < ATOMS / 8; ++h) {
+      const int a = h * 8 + fr;
+      if (a < nb) {
+        const R* wk = wtab + static_cast<size_t>(pr[h].x) * sd.wstride + 2 * fk;
+        stage2(&sW[0][a][2 * fk], wk + sd.woff[0] + (pr[h].y & 0xff) * TX);
+        stage2(&sW[1][a][2 * fk], wk + sd.woff[1] + ((pr[h].y >> 8) & 0xff) * TY);
+        stage2(&sW[2][a][2 * fk], wk + sd.woff[2] + (pr[h].y >> 16) * TZ);
+      } else if (a < ((nb + 3) & ~3)) {  // padding atoms of the last group of four
 #pragma unroll
-        for (int j = 0; j < 8; ++j) sW[d][a][j] = 0.0;
-      sQ[a] = 0.0;
+        for (int d = 0; d < 3; ++d) sW[d][a][2 * fk] = sW[d][a][2 * fk + 1] = 0.0;
+      }
+      if (fk == 0) sQ[a] = q[h];
     }
     cp_async_wait_all();
     __syncwarp();
@@ -1065,6 +1079,8 @@ __device__ __forceinline__ void gather_tiles_ad_body(int tx, int ty, int tz,
 // values of one component).  Scaling the A fragment by w3_a(z) lets the DMMA
 // accumulators sum over the planes too.  Each warp takes up to MB M blocks of
 // a round of 8 MB WARPS atoms; per plane and component it issues two DMMAs per M block.
+// The weight rows are staged as in the spread, four threads to a row of 64 bytes (one
+// value, 12,000 sites, 8 calls: 286 -> 238 us; a batch of 128 cells 511 -> 471).
 // At the end the lane holding C for (atom, y pair) folds in w2, and the four
 // lanes of an atom are summed with shuffles in a fixed order.  Partials go to the (atom, slot) array as in the CUDA-core
 // gather; results are deterministic.
@@ -1115,23 +1131,26 @@ __device__ __forceinline__ void gather_tiles_dmma_body(int tx, int ty, int tz,
   for (int b0 = p0; b0 < p1; b0 += kGatherAtoms) {
     const int nb = min(kGatherAtoms, p1 - b0);
     __syncthreads();  // the previous round's weights are no longer read
-    for (int a = threadIdx.x; a < kGatherAtoms; a += blockDim.x) {
+    // Four threads per weight row of 64 bytes, whole sectors to an access; the entries
+    // before the first copy, which the compiler does not move loads across.
+    int2 pr[MB];
+#pragma unroll
+    for (int h = 0; h < MB; ++h) {
+      const int a = h * (8 * WARPS) + (threadIdx.x >> 2);
+      pr[h] = a < nb ? pairs[b0 + a] : make_int2(0, 0);
+    }
+#pragma unroll
+    for (int h = 0; h < MB; ++h) {
+      const int a = h * (8 * WARPS) + (threadIdx.x >> 2), c = 2 * (threadIdx.x & 3);
       if (a < nb) {
-        const int2 pr = pairs[b0 + a];
-        sPair[a] = pr;
-        const R* wk = wtab + static_cast<size_t>(pr.x) * sd.wstride;
-        const R* src[3] = {wk + sd.woff[0] + (pr.y & 0xff) * TX,
-                           wk + sd.woff[1] + ((pr.y >> 8) & 0xff) * TY,
-                           wk + sd.woff[2] + (pr.y >> 16) * TZ};
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) stage2(&sW[d][a][2 * j], src[d] + 2 * j);
+        if (c == 0) sPair[a] = pr[h];
+        const R* wk = wtab + static_cast<size_t>(pr[h].x) * sd.wstride + c;
+        stage2(&sW[0][a][c], wk + sd.woff[0] + (pr[h].y & 0xff) * TX);
+        stage2(&sW[1][a][c], wk + sd.woff[1] + ((pr[h].y >> 8) & 0xff) * TY);
+        stage2(&sW[2][a][c], wk + sd.woff[2] + (pr[h].y >> 16) * TZ);
       } else {  // rows past the list: zero weights, results discarded
 #pragma unroll
-        for (int d = 0; d < 3; ++d)
-#pragma unroll
-          for (int j = 0; j < 8; ++j) sW[d][a][j] = 0.0;
+        for (int d = 0; d < 3; ++d) sW[d][a][c] = sW[d][a][c + 1] = 0.0;
       }
     }
     cp_async_wait_all();  // also completes the tile copies on the first round
@@ -1468,23 +1487,23 @@ __global__ void __launch_bounds__(kSpreadLanes) k_spread_tiles(const int* __rest
                                                                StencilDims sd, R* __restrict__ grid) {
   spread_tiles_body<R>(blockIdx.x, blockIdx.y, blockIdx.z, tile_start, pairs, wtab, qk, sd, grid);
 }
-template <typename R>
+template <typename R, int ATOMS>
 __global__ void __launch_bounds__(32) k_spread_tiles_dmma(const int* __restrict__ tile_start,
                                                           const int2* __restrict__ unordered,
                                                           int2* pairs, const R* __restrict__ wtab,
                                                           const R* __restrict__ qk,
                                                           StencilDims sd, R* __restrict__ grid) {
-  spread_tiles_dmma_body<R>(blockIdx.x, blockIdx.y, blockIdx.z, tile_start, unordered, pairs, wtab,
+  spread_tiles_dmma_body<R, ATOMS>(blockIdx.x, blockIdx.y, blockIdx.z, tile_start, unordered, pairs, wtab,
                             qk, sd, grid);
 }
-template <typename R>
+template <typename R, int ATOMS>
 __global__ void __launch_bounds__(32) k_spread_tiles_dmma_seg(
     const BatchCell* __restrict__ cells, const int* __restrict__ prefix, int ncells,
     const int* __restrict__ tile_start, const int2* __restrict__ unordered, int2* pairs,
     const R* __restrict__ wtab, const R* __restrict__ qk) {
   int tx, ty, tz;
   const BatchCell& bc = tile_of_block(cells, prefix, ncells, &tx, &ty, &tz);
-  spread_tiles_dmma_body<R>(tx, ty, tz, tile_start + bc.tile0, unordered, pairs, wtab, qk, bc.sd,
+  spread_tiles_dmma_body<R, ATOMS>(tx, ty, tz, tile_start + bc.tile0, unordered, pairs, wtab, qk, bc.sd,
                             static_cast<R*>(bc.grid));
 }
 
@@ -1620,11 +1639,13 @@ void launch_spread(const MeshPlan& mp, const PairBins& b, const int4* slot, int 
                    static_cast<const float*>(wtab), static_cast<const float*>(qk), mp.sd,
                    static_cast<float*>(grid));
   else if (mp.mixed)  // FP32 weights and grid, FP64 products on the tensor cores
-    launch_chained(k_spread_tiles_dmma<float>, grd, 32, 0, st, tile_start, unordered, pairs,
+    launch_chained(ntiles > kSpreadFull ? k_spread_tiles_dmma<float, kSpreadFew>
+                                        : k_spread_tiles_dmma<float, kSpreadMany>, grd, 32, 0, st, tile_start, unordered, pairs,
                    static_cast<const float*>(wtab), static_cast<const float*>(qk), mp.sd,
                    static_cast<float*>(grid));
   else
-    launch_chained(k_spread_tiles_dmma<double>, grd, 32, 0, st, tile_start, unordered, pairs,
+    launch_chained(ntiles > kSpreadFull ? k_spread_tiles_dmma<double, kSpreadFew>
+                                        : k_spread_tiles_dmma<double, kSpreadMany>, grd, 32, 0, st, tile_start, unordered, pairs,
                    static_cast<const double*>(wtab), static_cast<const double*>(qk), mp.sd,
                    static_cast<double*>(grid));
   ++g_launches;
@@ -1768,11 +1789,11 @@ void launch_spread_seg(const BatchLaunch& b, const PairBins& pb, const int4* slo
     unordered = nullptr;
   }
   if (b.mixed)
-    launch_chained(k_spread_tiles_dmma_seg<float>, b.n_tiles, 32, 0, st, b.cells, b.p_tiles,
+    launch_chained(k_spread_tiles_dmma_seg<float, kSpreadFew>, b.n_tiles, 32, 0, st, b.cells, b.p_tiles,
                    b.ncells, tile_start, unordered, pairs, static_cast<const float*>(wtab),
                    static_cast<const float*>(qk));
   else
-    launch_chained(k_spread_tiles_dmma_seg<double>, b.n_tiles, 32, 0, st, b.cells, b.p_tiles,
+    launch_chained(k_spread_tiles_dmma_seg<double, kSpreadFew>, b.n_tiles, 32, 0, st, b.cells, b.p_tiles,
                    b.ncells, tile_start, unordered, pairs, static_cast<const double*>(wtab),
                    static_cast<const double*>(qk));
   ++g_launches;
