@@ -484,8 +484,13 @@ void launch64(const Launch64& l) {
 }
 
 // A batch's pass over the cells whose length lies in SHS (all of one class).
+// The same for a batch, whose kernel holds the lengths of a class.
+constexpr int min_blocks_seg(int pass, int threads) {
+  return pass != P64_Z ? 0 : threads <= 64 ? 14 : threads <= 96 ? 8 : threads <= 128 ? 4 : 2;
+}
+
 template <int THREADS, int PASS, int VAR, class... SHS>
-__global__ void __launch_bounds__(THREADS) k64_pass_seg(const BatchCell* __restrict__ cells,
+__global__ void __launch_bounds__(THREADS, min_blocks_seg(PASS, THREADS)) k64_pass_seg(const BatchCell* __restrict__ cells,
                                                         PassGroup g, int nz) {
   chain_enter();
   const int m = seg_cell(g.prefix, g.n, blockIdx.x);

@@ -8,7 +8,9 @@ void launch64_seg0(const Launch64& l) {
         TwoPass<24, 6, 4>,
         TwoPass<32, 8, 4>,
         TwoPass<40, 8, 5>,
-        TwoPass<48, 8, 6>>::launch(l);
+        TwoPass<48, 8, 6>,
+        TwoPass<56, 8, 7>,
+        TwoPass<64, 8, 8>>::launch(l);
 }
 
 }  // namespace ewg

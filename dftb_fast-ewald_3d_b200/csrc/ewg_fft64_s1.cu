@@ -4,9 +4,7 @@
 namespace ewg {
 
 void launch64_seg1(const Launch64& l) {
-  Seg64<TwoPass<56, 8, 7>,
-        TwoPass<64, 8, 8>,
-        TwoPass<72, 9, 8>,
+  Seg64<TwoPass<72, 9, 8>,
         TwoPass<80, 10, 8>,
         TwoPass<96, 12, 8>>::launch(l);
 }

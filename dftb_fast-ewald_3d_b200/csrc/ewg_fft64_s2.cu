@@ -11,8 +11,6 @@ void launch64_seg2(const Launch64& l) {
         TwoPass<160, 16, 10>,
         TwoPass<168, 14, 12>,
         TwoPass<192, 16, 12>,
-        TwoPass<200, 20, 10>,
-        TwoPass<216, 18, 12>,
         TwoPass<224, 16, 14>,
         TwoPass<240, 16, 15>,
         TwoPass<256, 16, 16>>::launch(l);

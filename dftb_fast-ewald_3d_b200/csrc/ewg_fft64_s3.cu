@@ -4,7 +4,9 @@
 namespace ewg {
 
 void launch64_seg3(const Launch64& l) {
-  Seg64<TwoPass<280, 20, 14>,
+  Seg64<TwoPass<200, 20, 10>,
+        TwoPass<216, 18, 12>,
+        TwoPass<280, 20, 14>,
         TwoPass<288, 18, 16>,
         TwoPass<320, 20, 16>,
         TwoPass<336, 21, 16>,
