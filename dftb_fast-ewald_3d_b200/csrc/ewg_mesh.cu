@@ -46,10 +46,27 @@ namespace {
 constexpr size_t kSmemBudget = 200 * 1024;
 
 // Every pass transforms L lines (a power of two, the fastest index) of length n
-// with fft_edges: two buffers of n * L elements in shared memory, blockDim.x =
-// pass_threads(L): 32 threads per line, at least 128 per CTA.  The first and
+// with fft_edges: two buffers of n * L elements in shared memory, at most
+// pass_threads(L) threads: 32 per line, at least 128 per CTA.  The first and
 // last radix passes read and write global memory directly.
 constexpr int pass_threads(int L) { return L >= 4 ? 32 * L : 128; }
+
+// Threads of a CTA of the runtime schedule with sm bytes of shared memory.  A pass
+// of radix r has n / r butterflies per line, 8 at 64 points, so that 32 threads per
+// line leave most of a CTA idle while its registers (64 a thread) keep others out.
+// 8 or 16 per line do the same butterflies with more CTAs to an SM.  They are taken
+// where the shared memory still lets an SM hold `want` threads, and where there are
+// more than four blocks to an SM: fewer are resident at once anyway and end sooner
+// with more threads.  A mixed batch of 96 cells: forward passes 445 -> 276 us, inverse
+// 906 -> 460 (with 1024 wanted throughout 290 and 556).  The z pass, which weights its modes
+// between two transforms, wants 1024: at 224 points it takes 60 us with 768, 47 so.
+int dyn_threads(int L, size_t sm, long blocks, int want) {
+  const int full = pass_threads(L);
+  if (L < 4 || blocks <= 4 * 148) return full;
+  for (int t = 8 * L; t < full; t *= 2)
+    if (t >= 32 && (227 * 1024 / (sm + 1024)) * t >= want) return t;
+  return full;
+}
 
 // The buffer the last pass of `plan` leaves free (its `spare`).
 template <typename R>
@@ -63,6 +80,10 @@ __device__ __forceinline__ cx<R>* spare_buffer(cx<R>* a, cx<R>* b, const FftPlan
 struct DynShape {
   template <int L>
   static constexpr int threads() { return pass_threads(L); }
+  template <int L>
+  static int block(size_t sm, long blocks, int want = 700) {
+    return dyn_threads(L, sm, blocks, want);
+  }
   template <typename R, int SIGN, int L, class Ld, class St>
   __device__ __forceinline__ static void run(cx<R>* a, cx<R>* b, int n, const FftPlan& plan,
                                              const cx<R>* __restrict__ tw, Ld ld, St st) {
@@ -75,6 +96,8 @@ template <int N, int R0, int R1, int R2, int TPL = 32>
 struct StatShape {
   template <int L>
   static constexpr int threads() { return L * TPL; }
+  template <int L>
+  static int block(size_t, long, int = 0) { return threads<L>(); }
   template <typename R, int SIGN, int L, class Ld, class St>
   __device__ __forceinline__ static void run(cx<R>* a, cx<R>* b, int, const FftPlan&,
                                              const cx<R>* __restrict__ tw, Ld ld, St st) {
@@ -592,6 +615,8 @@ bool pass64(const MeshPlan& mp, int pass, int d, const void* grid, const void* A
   return true;
 }
 
+long blocks_of(dim3 g) { return static_cast<long>(g.x) * g.y * g.z; }
+
 template <typename R>
 void forward_impl(const MeshPlan& mp, const void* grid, void* A1v, void* A2v, void* B2v, int nc,
                   double* stress_part, cudaStream_t st) {
@@ -611,7 +636,7 @@ void forward_impl(const MeshPlan& mp, const void* grid, void* A1v, void* A2v, vo
     with_lines(L, [&](auto lc) {
       constexpr int LL = decltype(lc)::value;
       with_shape<R, LL>(mp.fft[0], [&](auto sh) {
-        launch_chained(k_fft_x_r2c<R, LL, decltype(sh)>, blocks, decltype(sh)::template threads<LL>(), sm, st,
+        launch_chained(k_fft_x_r2c<R, LL, decltype(sh)>, blocks, decltype(sh)::template block<LL>(sm, blocks), sm, st,
                        static_cast<const R*>(grid), A1, n1, npairs, g.K1, mp.fft[0]);
       });
     });
@@ -628,7 +653,8 @@ void forward_impl(const MeshPlan& mp, const void* grid, void* A1v, void* A2v, vo
     with_lines(L, [&](auto lc) {
       constexpr int LL = decltype(lc)::value;
       with_shape<R, LL>(mp.fft[1], [&](auto sh) {
-        launch_chained(k_fft_y_fwd<R, LL, decltype(sh)>, grd, decltype(sh)::template threads<LL>(), sm, st, A1, A2, n2,
+        launch_chained(k_fft_y_fwd<R, LL, decltype(sh)>, grd, decltype(sh)::template block<LL>(sm, blocks_of(grd)), sm, st,
+                       A1, A2, n2,
                        g.K1, g.K2, H2, mp.fft[1]);
       });
     });
@@ -659,10 +685,10 @@ void forward_impl(const MeshPlan& mp, const void* grid, void* A1v, void* A2v, vo
       with_shape<R, LL>(mp.fft[2], [&](auto sh) {
         using SH = decltype(sh);
         if (stress_part)
-          launch_chained(k_fft_z_influence<R, LL, true, SH>, grd, SH::template threads<LL>(), sm, st, A2, B2,
+          launch_chained(k_fft_z_influence<R, LL, true, SH>, grd, SH::template block<LL>(sm, blocks_of(grd), 1024), sm, st, A2, B2,
                          n3, g.K1, g.K2, g.K3, nz, ia, mp.fft[2]);
         else
-          launch_chained(k_fft_z_influence<R, LL, false, SH>, grd, SH::template threads<LL>(), sm, st, A2, B2,
+          launch_chained(k_fft_z_influence<R, LL, false, SH>, grd, SH::template block<LL>(sm, blocks_of(grd), 1024), sm, st, A2, B2,
                          n3, g.K1, g.K2, g.K3, nz, ia, mp.fft[2]);
       });
     });
@@ -688,7 +714,7 @@ void inverse_impl(const MeshPlan& mp, const void* B2v, void* B1v, void* out, int
     with_lines(L, [&](auto lc) {
       constexpr int LL = decltype(lc)::value;
       with_shape<R, LL>(mp.fft[1], [&](auto sh) {
-        launch_chained(k_fft_y_inv<R, LL, decltype(sh)>, grd, decltype(sh)::template threads<LL>(), sm, st, B2, B1, n2,
+        launch_chained(k_fft_y_inv<R, LL, decltype(sh)>, grd, decltype(sh)::template block<LL>(sm, blocks_of(grd)), sm, st, B2, B1, n2,
                        n3, g.K1, g.K2, H2, mp.fft[1]);
       });
     });
@@ -709,7 +735,7 @@ void inverse_impl(const MeshPlan& mp, const void* B2v, void* B1v, void* out, int
         constexpr int LL = decltype(lc)::value;
         if constexpr (LL >= 4)
           with_shape<R, LL>(mp.fft[0], [&](auto sh) {
-            launch_chained(k_fft_x_c2r<R, LL, 4, decltype(sh)>, grd, decltype(sh)::template threads<LL>(), sm, st, B1,
+            launch_chained(k_fft_x_c2r<R, LL, 4, decltype(sh)>, grd, decltype(sh)::template block<LL>(sm, blocks_of(grd)), sm, st, B1,
                            o, n1, nrows, g.K1, nc, mp.fft[0]);
           });
       });
@@ -718,7 +744,7 @@ void inverse_impl(const MeshPlan& mp, const void* B2v, void* B1v, void* out, int
       with_lines(L, [&](auto lc) {
         constexpr int LL = decltype(lc)::value;
         with_shape<R, LL>(mp.fft[0], [&](auto sh) {
-          launch_chained(k_fft_x_c2r<R, LL, 1, decltype(sh)>, grd, decltype(sh)::template threads<LL>(), sm, st, B1, o,
+          launch_chained(k_fft_x_c2r<R, LL, 1, decltype(sh)>, grd, decltype(sh)::template block<LL>(sm, blocks_of(grd)), sm, st, B1, o,
                          n1, nrows, g.K1, nc, mp.fft[0]);
         });
       });
@@ -808,7 +834,8 @@ void forward_seg_impl(const BatchLaunch& b, cudaStream_t st) {
     if (b.n_r2c)
       with_seg_shape<R, LL>(b, 0, [&](auto sh) {
         using SH = decltype(sh);
-        launch_chained(k_fft_x_r2c_seg<R, LL, SH>, b.n_r2c, SH::template threads<LL>(), b.smem[0],
+        launch_chained(k_fft_x_r2c_seg<R, LL, SH>, b.n_r2c,
+                       SH::template block<LL>(b.smem[0], b.n_r2c), b.smem[0],
                        st, b.cells, b.p_r2c, b.ncells);
         ++g_launches;
       });
@@ -816,7 +843,8 @@ void forward_seg_impl(const BatchLaunch& b, cudaStream_t st) {
     if (b.n_yfwd)
       with_seg_shape<R, LL>(b, 1, [&](auto sh) {
         using SH = decltype(sh);
-        launch_chained(k_fft_y_fwd_seg<R, LL, SH>, b.n_yfwd, SH::template threads<LL>(), b.smem[1],
+        launch_chained(k_fft_y_fwd_seg<R, LL, SH>, b.n_yfwd,
+                       SH::template block<LL>(b.smem[1], b.n_yfwd), b.smem[1],
                        st, b.cells, b.p_yfwd, b.ncells);
         ++g_launches;
       });
@@ -824,7 +852,8 @@ void forward_seg_impl(const BatchLaunch& b, cudaStream_t st) {
     if (b.n_z)
       with_seg_shape<R, LL>(b, 2, [&](auto sh) {
         using SH = decltype(sh);
-        launch_chained(k_fft_z_influence_seg<R, LL, SH>, b.n_z, SH::template threads<LL>(),
+        launch_chained(k_fft_z_influence_seg<R, LL, SH>, b.n_z,
+                       SH::template block<LL>(b.smem_z, b.n_z, 1024),
                        b.smem_z, st, b.cells, b.p_z, b.ncells, nz);
         ++g_launches;
       });
@@ -839,7 +868,8 @@ void inverse_seg_impl(const BatchLaunch& b, cudaStream_t st) {
     if (b.n_yinv)
       with_seg_shape<R, LL>(b, 1, [&](auto sh) {
         using SH = decltype(sh);
-        launch_chained(k_fft_y_inv_seg<R, LL, SH>, b.n_yinv, SH::template threads<LL>(), b.smem[1],
+        launch_chained(k_fft_y_inv_seg<R, LL, SH>, b.n_yinv,
+                       SH::template block<LL>(b.smem[1], b.n_yinv), b.smem[1],
                        st, b.cells, b.p_yinv, b.ncells);
         ++g_launches;
       });
@@ -850,12 +880,14 @@ void inverse_seg_impl(const BatchLaunch& b, cudaStream_t st) {
         ++g_launches;
         if constexpr (LL >= 4) {
           if (b.nc == 4) {
-            launch_chained(k_fft_x_c2r_seg<R, LL, 4, SH>, b.n_c2r, SH::template threads<LL>(),
+            launch_chained(k_fft_x_c2r_seg<R, LL, 4, SH>, b.n_c2r,
+                       SH::template block<LL>(b.smem[0], b.n_c2r),
                            b.smem[0], st, b.cells, b.p_c2r, b.ncells, b.nc);
             return;
           }
         }
-        launch_chained(k_fft_x_c2r_seg<R, LL, 1, SH>, b.n_c2r, SH::template threads<LL>(),
+        launch_chained(k_fft_x_c2r_seg<R, LL, 1, SH>, b.n_c2r,
+                       SH::template block<LL>(b.smem[0], b.n_c2r),
                        b.smem[0], st, b.cells, b.p_c2r, b.ncells, b.nc);
       });
   });
