@@ -8,7 +8,7 @@ parameters re-derived from the charges, real-space pair sum, adjoint NFFT, four
 forward NFFTs (potential and ik force), self term.
 
 Our arm (default):
-  value   plain FP64 form at tol 1e-10 (the reference chain: 280^3 grid, m=12),
+  value   plain FP64 form at tol 1e-10 (the reference chain: 140^3 modes, m=12),
           inputs and outputs resident in HBM, device-timed with CUDA events on
           the launching stream; L2 flushed between steps (flush not timed).
   e2e     the same through the C ABI with pinned host buffers: every step copies
@@ -139,9 +139,35 @@ class ClockSampler:
 # ---------------------------------------------------------------------------
 # algorithmic bytes per stage launch (one evaluation), for the roofline
 # ---------------------------------------------------------------------------
+def kaiser_bessel(params, real_bytes):
+    """The plain form evaluates half-widths 11 and 12 with the Kaiser-Bessel window."""
+    return real_bytes == 8 and params["window_cutoff"] in (11, 12)
+
+
+def fine_grid(params, real_bytes):
+    """Fine grid lengths: two points per mode, or for the Kaiser-Bessel window the
+    next multiple of 8 of factors up to 7 from 1.28 per mode."""
+    if not kaiser_bessel(params, real_bytes):
+        return [2 * m for m in params["n_modes"]]
+
+    def smooth(k):
+        for p in (2, 3, 5, 7):
+            while k % p == 0:
+                k //= p
+        return k == 1
+
+    out = []
+    for m in params["n_modes"]:
+        k = max(16, (128 * m + 99) // 100)
+        while k % 8 or not smooth(k):
+            k += 1
+        out.append(k)
+    return out
+
+
 def stage_bytes(params, natoms, real_bytes, nc=4):
     M = params["n_modes"]
-    n = [2 * m for m in M]
+    n = fine_grid(params, real_bytes)
     H = [m - m // 2 for m in M]
     K1, K2, K3 = H[0] + 1, 2 * H[1] + 1, 2 * H[2] + 1
     s, c = real_bytes, 2 * real_bytes
@@ -163,7 +189,7 @@ def stage_bytes(params, natoms, real_bytes, nc=4):
 def stage_flops(params, natoms, nc=4):
     """Algorithmic FP64 flops of the tensor-core stages: one multiply-add per
     stencil point and component (gather: nc components; spread: one)."""
-    w = (2 * params["window_cutoff"] + 1) ** 3
+    w = 14 ** 3 if kaiser_bessel(params, 8) else (2 * params["window_cutoff"] + 1) ** 3
     return {"spread": 2 * natoms * w, "gather": 2 * natoms * w * nc}
 
 
@@ -172,7 +198,7 @@ def stage_flops(params, natoms, nc=4):
 # bytes, grids through the inverse passes and the gather, stage); other
 # workloads report null.
 DRAM_TRAFFIC = {
-    ("c3", 8, 4, "gather"): 746.37e6 + 62.96e6,
+    ("c3", 8, 4, "gather"): 251.5e6 + 16.0e6,
 }
 
 
@@ -464,12 +490,12 @@ def run_scc(args, eb, torch, device, dist, ws, rank):
         pos, q, lat = workloads.c5_rock_salt_216k()
         charges = [workloads.c5_charge_update(q, k) for k in range(30)]
         label, metric = "c5_rock_salt_216000_scc30", "C5 SCC: shift evals/s at 216,000 sites, fixed geometry, 30 charge updates"
-        grids = "working set (512^3 grids) > L2"
+        grids = "working set (336^3 grids) > L2"
     else:
         pos, q, lat = workloads.c3_water_32k()
         charges = [workloads.charge_update(q, k, seed=3) for k in range(30)]
         label, metric = "c3_water_32769_scc30", "C3 SCC: shift evals/s at 32,769 atoms, fixed geometry, 30 charge updates"
-        grids = "working set (280^3 grids) > L2"
+        grids = "working set (192^3 grids) > L2"
 
     def maxrank(x):
         if not dist:
@@ -752,8 +778,8 @@ def run_ours(args):
         b = sum(stage_bytes(params, natoms, real_bytes, nc).values())
         return {"bytes": b, "achieved_gbs": b / t_step / 1e9, "frac": b / t_step / 1e9 / peak}
 
-    def grid_of(params):
-        return "x".join(str(2 * m) for m in params["n_modes"])
+    def grid_of(params, real_bytes):
+        return "x".join(str(k) for k in fine_grid(params, real_bytes))
 
     top64, per64, roof64 = roofline(stages, params64, 8, args.steps, tensor_peak)
     _, perad, roofad = roofline(stagesad, params64, 8, args.steps, tensor_peak, nc=1)
@@ -769,7 +795,7 @@ def run_ours(args):
         "warmup": args.warmup, "ms_per_step": 1e3 * t64 / args.steps, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
         "config": {"workload": label, "natoms": natoms,
-                   "tol": TOL_FP64, "grid": grid_of(params64),
+                   "tol": TOL_FP64, "grid": grid_of(params64, 8),
                    "window_cutoff": params64["window_cutoff"], "alpha": params64["alpha"],
                    "r_cut_bohr": params64["r_cut"], "forces": "ik (the reference's scheme)",
                    "kernel_shape": fp64.shape,
@@ -794,7 +820,7 @@ def run_ours(args):
                                  f"{MIXED_TARGET / 2:g} vs the FP64 form)",
                        "forces": scheme_name[tuned_scheme], "alpha": params32["alpha"],
                        "r_cut_bohr": params32["r_cut"], "k_cut": params32["k_cut"],
-                       "grid": grid_of(params32), "window_cutoff": params32["window_cutoff"],
+                       "grid": grid_of(params32, 4), "window_cutoff": params32["window_cutoff"],
                        "tuner_report": tune_report, "kernel_shape": mixed.shape},
             "speedup_vs_fp64": (ws * args.steps / t32) / value,
             "e2e": dict(value=ws * args.steps / te32, unit="evals/s", **e2e_io),
