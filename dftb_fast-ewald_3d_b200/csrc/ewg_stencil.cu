@@ -620,7 +620,7 @@ __device__ __forceinline__ void dmma_m8n8k4(double& c0, double& c1, double a, do
                : "d"(a), "d"(b));
 }
 
-constexpr int kGatherWarps = 4;   // tensor-core i k gather: warps per tile
+constexpr int kGatherWarps = 4;   // tensor-core i k gather: warps per tile (batch, short lists)
 constexpr int kGatherMB = 2;      // tensor-core i k gather: M blocks of 8 atoms per warp and round
 constexpr int kGatherAdWarps = 2;  // tensor-core gather with window derivatives: warps per tile
 // FP32 CUDA-core gather with window derivatives: one atom per lane (74 registers, so

@@ -242,7 +242,8 @@ typedef struct {
                        2 odd radices, then radix 4 in place of 8 */
   int gather_warps; /* FP64-contraction i k gather: warps per tile, 2, 4 or 8,
                        each with 64 / (8 warps) blocks of 8 atoms per round
-                       (default 4) */
+                       (default: 8 in the plain form where the tiles'
+                       lists are long, else 4) */
   int stencil;      /* mixed form's spread and gathers: 1 the FP64 tensor cores
                        on its FP32 weights and grids (default), 2 FP32 CUDA cores */
 } ewg_kernel_shape;

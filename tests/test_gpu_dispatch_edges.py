@@ -143,3 +143,24 @@ def test_unblurred_points(ewald_lib, oracle, edges, targets):
                        oracle.potential_gradient_at(folded, src, q, lat.T, 1e-10)) < TOL_POINTS
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("n", [5, 20, 40, 90])
+def test_gather_warps_by_list_length(ewald_lib, n):
+    """Lists below and above the length from which the gather takes eight warps (48
+    slots a tile; 3 x 3 x 3 tiles, of which each atom has a slot or more); the partials
+    do not depend on it, so every shape agrees bitwise."""
+    rng = np.random.default_rng(n)
+    lat = np.diag([9.5, 9.0, 10.0])
+    pos, q = rng.uniform(size=(n, 3)) @ lat, charges(rng, n)
+    ov = dict(alpha_in=0.8, r_cut_in=4.0, k_cut_in=3.0, windowCutoff_in=12)
+    c = ewald_lib.Context(0, ewald_lib.FP64)
+    try:
+        results = [c.potential_force(pos, q, lat, 1e-8, **ov)]
+        for warps in (2, 4, 8):
+            c.set_kernel_shape({"gather_warps": warps})
+            results.append(c.potential_force(pos, q, lat, 1e-8, **ov))
+        for p, f in results[1:]:
+            assert np.array_equal(p, results[0][0]) and np.array_equal(f, results[0][1])
+    finally:
+        c.close()
