@@ -6,8 +6,9 @@
 // line went three times through registers and twice through shared memory, each
 // thread with 5 to 8 loads outstanding between barriers.  Here a line goes
 // through registers twice (32,769 atoms, 192 points per axis, in us: x R2C 23, y
-// forward 16, z 43, y inverse 41, x C2R 82; 216,000 sites, 336 points: 146, 88, 425,
-// 262, 561, the last two at 4.0 and 3.4 TB/s): a thread loads R0 elements of its line at once, does
+// forward 16, z 41, y inverse 41, x C2R 81; 216,000 sites, 336 points: 146, 88, 265,
+// 262, 560, the last two at 4.0 and 3.4 TB/s; a batch of 128 cells: forward 425, inverse
+// 598): a thread loads R0 elements of its line at once, does
 // an R0-point transform in registers, leaves them in one shared buffer, and after
 // one barrier takes R1 of them through the second transform and out.  A CTA
 // holds 8 lines (128-byte rows: global and shared accesses are coalesced and

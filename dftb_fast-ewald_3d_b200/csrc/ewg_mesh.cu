@@ -1,8 +1,10 @@
-// ewg_mesh.cu -- the Gaussian-window NFFT of the reciprocal sum on the GPU.
+// ewg_mesh.cu -- the NFFT of the reciprocal sum on the GPU: the passes with a
+// runtime radix schedule, and the choice between them and the FP64 passes of two
+// register radices (ewg_fft64.cuh).
 //
 // Pipeline for one evaluation (reference: fft/ewald_fft_3d_fourier.f90:28-153
 // and nfft/nfft.f90:196-404):
-//   weights   per-atom 3 x (2m+1) window weights      (stencil_weights :122-159)
+//   weights   per-atom window weights, 3 axes         (stencil_weights :122-159)
 //   spread    tile-owned, deterministic, no atomics   (adjoint step 1 :253-278)
 //   R2C x     real rows -> k1 in [0, M1/2]            (adjoint step 2 :282, pruned)
 //   C2C y     -> k2 in [-M2/2, M2/2]

@@ -2,18 +2,20 @@
 // gather (nfft/nfft.f90:122-159, :253-278, :380-402).
 //
 // Tiling.  The fine grid is cut into tiles of 8 x 8 x 8 points.  Along each
-// axis an atom's stencil [c-m, c+m] (mod n) runs through at most S_d
-// consecutive tiles starting at tile f_d; the atom meets every tile of that
-// S_x x S_y x S_z block once ("slots").
+// axis an atom's stencil (2m + 1 points with the Gaussian window, 14 with the
+// Kaiser-Bessel window; mod n) runs through at most S_d consecutive tiles
+// starting at tile f_d; the atom meets every tile of that S_x x S_y x S_z block
+// once ("slots").
 //
 // Weights.  Per atom and axis the window weights are stored already laid out
 // per touched tile (S_d * 8 values; zero outside the stencil and beyond the
 // grid end; points a wrapping stencil reaches twice carry the sum).  A kernel
 // then reads an atom's weights for a tile with no index arithmetic.
 //
-// Pairs.  Once per geometry, every (atom, tile) pair is binned by tile with a
-// counting sort whose buckets are ordered by atom index, so each tile owns an
-// exact, deterministic list of the atoms that reach it.
+// Pairs.  Once per geometry, every (atom, tile) pair is binned by tile, and the
+// spread puts its tile's bucket in atom order and writes it back (a kernel of its
+// own does so where the lists are long), so each tile owns an exact,
+// deterministic list of the atoms that reach it.
 //
 // Spread: a CTA owns a tile and writes it once (no atomics, no zeroing, fixed
 // order).  Both precision forms contract on the FP64 tensor cores (DMMA); the

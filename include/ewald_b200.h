@@ -3,9 +3,12 @@
  *
  * This library replaces the engine behind DFTB+'s TCoulomb call surface for
  * three-dimensionally periodic, charge-neutral SCC calculations: the real-space
- * erfc pair sum over a linked-cell list, the Gaussian-window NFFT reciprocal
- * sum (spread, FFT, influence weights, gather) and the stock electrostatic
- * stress.  Every function returns an int status (EWG_OK == 0); see
+ * erfc pair sum over a linked-cell list, the NFFT reciprocal sum (spread, FFT,
+ * influence weights, gather) and the stock electrostatic stress.  The NFFT's
+ * window is the reference's Gaussian; the plain form at half-widths 11 and 12
+ * (tolerances of about 1e-9 and 1e-10), where the modes at the edge of the box
+ * are damped, takes a Kaiser-Bessel window of the same accuracy on a smaller
+ * grid.  Every function returns an int status (EWG_OK == 0); see
  * ewg_status_string().  All pointers are host memory unless a name ends in
  * _device.  Outputs are overwritten, never accumulated into.
  *
@@ -131,7 +134,7 @@ int ewg_set_background(ewg_context* ctx, int on);
  * (EWG_FORCE_IK or EWG_FORCE_AD).  Default: IK, the reference's own scheme,
  * in both precision forms.  AD computes the
  * reciprocal force as -q sum_d b_d sum_l g_l dW/ds_d, with g the potential grid
- * and W the product of the three Gaussian windows; it spends one inverse
+ * and W the product of the three windows; it spends one inverse
  * transform where IK spends four.  Both converge to the same Ewald force; at
  * the reference's parameters for tol = 1e-10 they differ by about 1e-12
  * relative.  Potentials, energies and stresses do not depend on the scheme.
@@ -237,9 +240,12 @@ typedef struct {
                        (box_count_3d, common/ewald_cell_list.f90:56-73) along
                        each axis, 1, 2 or 3 (default 2: 5 x 5 x 5 neighbourhoods) */
   int fft_lines;    /* most FFT lines per CTA: 1, 2, 4 or 8 (default: the most
-                       whose buffers fit the CTA's shared-memory budget) */
+                       whose buffers fit the CTA's shared-memory budget).  The
+                       FP64 passes of two register radices have 8 */
   int fft_sched;    /* FFT radix schedule: 1 odd radices, then radix 8 (default);
-                       2 odd radices, then radix 4 in place of 8 */
+                       2 odd radices, then radix 4 in place of 8.  With 1 the
+                       FP64 lengths that are a product of two radices of at
+                       most 24 (whole tiles of 8) take passes of their own */
   int gather_warps; /* FP64-contraction i k gather: warps per tile, 2, 4 or 8,
                        each with 64 / (8 warps) blocks of 8 atoms per round
                        (default: 8 in the plain form where the tiles'
