@@ -579,7 +579,7 @@ int evaluate(ewg_context* c, int n, const double* pos, long sa, long sd, const d
       launch_real_stress(s4s, x32s, boxstart, n, rg, p.alpha, p.r_cut, p6, stress12, err, rs);
     if (concurrent) cudaEventRecord(c->join, rs);
     prof_mark(mp.prof, st, ST_SPREAD);
-    launch_spread(mp, bins, slot, n, reuse, wtab, qk, grid, st);
+    launch_spread(mp, bins, slot, n, reuse, resident, wtab, qk, grid, st);
     launch_forward_and_weight(mp, grid, A1, A2, B2, nc, st, zpart);
     if (stress12) launch_sum_partials(zpart, mp.g.K1 * mp.g.K2, 6, stress12 + 6, st);
     launch_inverse(mp, B2, B1, outg, nc, st);
@@ -600,7 +600,7 @@ int evaluate(ewg_context* c, int n, const double* pos, long sa, long sd, const d
       key.push_back(u);
     };
     put(n), put(sa), put(sd), put(pos), put(q), put(pot), put(want_force ? force : nullptr);
-    put(err), put(err_flag), put(stress12), put(reuse), put(mixed), put(mp.sd.ad), put(nc), put(ad);
+    put(err), put(err_flag), put(stress12), put(resident), put(reuse), put(mixed), put(mp.sd.ad), put(nc), put(ad);
     put(p.alpha), put(p.r_cut), put(p.k_cut), put(p.window_cutoff);
     for (int d = 0; d < 3; ++d) put(p.n_modes[d]);
     for (int i = 0; i < 3; ++i)
@@ -2252,7 +2252,7 @@ int points_mesh(ewg_context* c, const Cell& cell, double tol, int nt, const doub
                    SortBufs{s4, skey, bcnt, btmp, sbox, sperm, s4s, x32}, kcnt, ntiles, st);
   // Fourier sum: spread the sources, transform, weight, invert, gather.
   launch_weights_bins(src, s4s, ns, swt, sqk, sslot, sbins, st);
-  launch_spread(src, sbins, sslot, ns, false, swt, sqk, grid, st);
+  launch_spread(src, sbins, sslot, ns, false, false, swt, sqk, grid, st);
   launch_forward_and_weight(src, grid, A1, A2, B2, 1, st, nullptr);
   launch_inverse(src, B2, B1, outg, 1, st);
   // Targets: the same box order, for locality in the gather, which takes the pairs

@@ -166,7 +166,8 @@ struct MeshPlan {
 
 // (atom, tile) pairs: entry (atom, packed slot) of tile t in [starts[t],
 // starts[t+1]).  counts (one per tile) and arrival (one per atom and slot) are
-// scratch; pairs is the ordered copy that long lists and the FP32 spread use.
+// scratch; pairs is the ordered copy: every list where the geometry is kept for later
+// calls and for the FP32 CUDA-core spread, else the long lists.
 struct PairBins {
   int *counts, *arrival, *starts;
   int2 *unordered, *pairs;
@@ -314,10 +315,10 @@ void launch_weights_bins(const MeshPlan& mp, const double4* s4s, int n, void* wt
                          int4* slot, const PairBins& b, cudaStream_t st);
 
 // Tile-owned deterministic spread (adjoint_nfft_3d step 1, nfft/nfft.f90:253-278).
-// It takes each tile's list in order of the atoms; ordered: an earlier call with the
-// same bins has put the lists that need it into b.pairs.
+// It takes each tile's list in order of the atoms.  keep: it leaves every list in order
+// in b.pairs; ordered: an earlier call with the same bins has done so.
 void launch_spread(const MeshPlan& mp, const PairBins& b, const int4* slot, int n, bool ordered,
-                   const void* wtab, const void* qk, void* grid, cudaStream_t st);
+                   bool keep, const void* wtab, const void* qk, void* grid, cudaStream_t st);
 
 // Pruned forward transform of the real grid to the compact spectrum, fused with
 // the influence weights and the first inverse pass: grid -> A1 -> A2 -> B2.

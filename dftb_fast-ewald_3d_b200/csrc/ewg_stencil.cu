@@ -13,9 +13,11 @@
 // then reads an atom's weights for a tile with no index arithmetic.
 //
 // Pairs.  Once per geometry, every (atom, tile) pair is binned by tile, and the
-// spread puts its tile's bucket in atom order and writes it back (a kernel of its
-// own does so where the lists are long), so each tile owns an exact,
-// deterministic list of the atoms that reach it.
+// spread puts its tile's bucket in atom order (a kernel of its own does so where the
+// lists are long, and for the FP32 CUDA-core spread), so each tile owns an exact,
+// deterministic list of the atoms that reach it.  Where the geometry stays for later
+// calls every bucket is also written out in order, whichever spread comes first: a
+// later call takes it as it is, with its own choice of spread.
 //
 // Spread: a CTA owns a tile and writes it once (no atomics, no zeroing, fixed
 // order).  Both precision forms contract on the FP64 tensor cores (DMMA); the
@@ -662,11 +664,15 @@ __device__ __forceinline__ void stage2(double* dst, const float* src) {
 // took 55.6 us at 32,769 atoms and 281 at 216,000 sites, this 43.7 and 203), and
 // the entries of a round are read before its first copy, which the compiler moves
 // no load across.
+//
+// unordered: the tile lists in no fixed order, or null when pairs holds them in order;
+// keep: the ordered lists go to pairs, all of them (else only the long ones do).
 template <typename R, int ATOMS>
 __device__ __forceinline__ void spread_tiles_dmma_body(int tx, int ty, int tz,
                                                        const int* __restrict__ tile_start,
                                                        const int2* __restrict__ unordered,
-                                                       int2* pairs, const R* __restrict__ wtab,
+                                                       int2* pairs, bool keep,
+                                                       const R* __restrict__ wtab,
                                                        const R* __restrict__ qk,
                                                        const StencilDims& sd,
                                                        R* __restrict__ grid) {
@@ -707,7 +713,10 @@ __device__ __forceinline__ void spread_tiles_dmma_body(int tx, int ty, int tz,
     }
 #pragma unroll
     for (int h = 0; h < kSpreadList / 32; ++h)
-      if (h * 32 + lane < m) sList[place[h]] = v[h];
+      if (h * 32 + lane < m) {
+        sList[place[h]] = v[h];
+        if (keep) pairs[p0 + place[h]] = v[h];
+      }
     __syncwarp();
   } else if (unordered) {  // a long list goes through its ordered copy
     for (int e = p0 + lane; e < p1; e += 32) {
@@ -1492,11 +1501,12 @@ __global__ void __launch_bounds__(kSpreadLanes) k_spread_tiles(const int* __rest
 template <typename R, int ATOMS>
 __global__ void __launch_bounds__(32) k_spread_tiles_dmma(const int* __restrict__ tile_start,
                                                           const int2* __restrict__ unordered,
-                                                          int2* pairs, const R* __restrict__ wtab,
+                                                          int2* pairs, bool keep,
+                                                          const R* __restrict__ wtab,
                                                           const R* __restrict__ qk,
                                                           StencilDims sd, R* __restrict__ grid) {
-  spread_tiles_dmma_body<R, ATOMS>(blockIdx.x, blockIdx.y, blockIdx.z, tile_start, unordered, pairs, wtab,
-                            qk, sd, grid);
+  spread_tiles_dmma_body<R, ATOMS>(blockIdx.x, blockIdx.y, blockIdx.z, tile_start, unordered, pairs,
+                                   keep, wtab, qk, sd, grid);
 }
 template <typename R, int ATOMS>
 __global__ void __launch_bounds__(32) k_spread_tiles_dmma_seg(
@@ -1505,8 +1515,8 @@ __global__ void __launch_bounds__(32) k_spread_tiles_dmma_seg(
     const R* __restrict__ wtab, const R* __restrict__ qk) {
   int tx, ty, tz;
   const BatchCell& bc = tile_of_block(cells, prefix, ncells, &tx, &ty, &tz);
-  spread_tiles_dmma_body<R, ATOMS>(tx, ty, tz, tile_start + bc.tile0, unordered, pairs, wtab, qk, bc.sd,
-                            static_cast<R*>(bc.grid));
+  spread_tiles_dmma_body<R, ATOMS>(tx, ty, tz, tile_start + bc.tile0, unordered, pairs, false, wtab, qk,
+                                   bc.sd, static_cast<R*>(bc.grid));
 }
 
 template <typename R, int NC, int A, int WARPS>
@@ -1620,19 +1630,17 @@ void launch_weights_bins(const MeshPlan& mp, const double4* s4s, int n, void* wt
 }
 
 void launch_spread(const MeshPlan& mp, const PairBins& b, const int4* slot, int n, bool ordered,
-                   const void* wtab, const void* qk, void* grid, cudaStream_t st) {
+                   bool keep, const void* wtab, const void* qk, void* grid, cudaStream_t st) {
   const int ntiles = mp.sd.ntiles[0] * mp.sd.ntiles[1] * mp.sd.ntiles[2];
   const size_t items = static_cast<size_t>(n) * mp.sd.S[0] * mp.sd.S[1] * mp.sd.S[2];
   const bool cores = mp.mixed && mp.stencil == 2;
   const int* tile_start = b.starts;
   int2* pairs = b.pairs;
-  const int2* unordered = b.unordered;
-  if (n > 0 && (cores || own_rank(items, ntiles))) {
-    if (!ordered) {
-      launch_chained(k_pair_rank, blocks_for(items, 256), 256, 0, st, unordered, tile_start, ntiles,
-                     slot, mp.sd, pairs);
-      ++g_launches;
-    }
+  const int2* unordered = ordered ? nullptr : b.unordered;
+  if (n > 0 && !ordered && (cores || own_rank(items, ntiles))) {
+    launch_chained(k_pair_rank, blocks_for(items, 256), 256, 0, st, unordered, tile_start, ntiles,
+                   slot, mp.sd, pairs);
+    ++g_launches;
     unordered = nullptr;
   }
   dim3 grd(mp.sd.ntiles[0], mp.sd.ntiles[1], mp.sd.ntiles[2]);
@@ -1642,12 +1650,14 @@ void launch_spread(const MeshPlan& mp, const PairBins& b, const int4* slot, int 
                    static_cast<float*>(grid));
   else if (mp.mixed)  // FP32 weights and grid, FP64 products on the tensor cores
     launch_chained(ntiles > kSpreadFull ? k_spread_tiles_dmma<float, kSpreadFew>
-                                        : k_spread_tiles_dmma<float, kSpreadMany>, grd, 32, 0, st, tile_start, unordered, pairs,
+                                        : k_spread_tiles_dmma<float, kSpreadMany>,
+                   grd, 32, 0, st, tile_start, unordered, pairs, keep,
                    static_cast<const float*>(wtab), static_cast<const float*>(qk), mp.sd,
                    static_cast<float*>(grid));
   else
     launch_chained(ntiles > kSpreadFull ? k_spread_tiles_dmma<double, kSpreadFew>
-                                        : k_spread_tiles_dmma<double, kSpreadMany>, grd, 32, 0, st, tile_start, unordered, pairs,
+                                        : k_spread_tiles_dmma<double, kSpreadMany>,
+                   grd, 32, 0, st, tile_start, unordered, pairs, keep,
                    static_cast<const double*>(wtab), static_cast<const double*>(qk), mp.sd,
                    static_cast<double*>(grid));
   ++g_launches;
