@@ -106,9 +106,27 @@ __device__ __forceinline__ void stencil_tiles(int c, const StencilDims& sd, int 
   *count = min(m, nt);
 }
 
+// The Kaiser-Bessel weights of the stencil points as polynomials in t = 2 frac - 1.
+constexpr int kKbCoefs = kKbDegree + 1;
+__constant__ double c_kb[kKbWidth * kKbCoefs];
+
+// Point j's weight and, with ad, its derivative with respect to t.
+__device__ __forceinline__ void kb_weight(int j, double t, int ad, double* v, double* dv) {
+  const double* cf = c_kb + j * kKbCoefs;
+  double w = cf[kKbDegree], dw = 0.0;
+#pragma unroll
+  for (int e = kKbDegree - 1; e >= 0; --e) {
+    if (ad) dw = fma(dw, t, w);
+    w = fma(w, t, cf[e]);
+  }
+  *v = w;
+  *dv = dw;
+}
+
 // ---------------------------------------------------------------------------
 // Tiled window weights of wide windows (rows beyond kAxisRow values per atom),
-// one thread per (atom, axis, tile slot), eight points each.
+// one thread per (atom, axis, tile slot), eight points each.  A batch comes here
+// when one of its cells is that wide; the others may have the Kaiser-Bessel window.
 // ---------------------------------------------------------------------------
 // Row r (axis and slot) of sorted atom k.
 template <typename R>
@@ -132,7 +150,18 @@ __device__ __forceinline__ void weights_row(const double4* __restrict__ s4s, int
   const int origin = ((first + s) % nt) * T;
   R wv[TX], dv[TX];
   static_assert(TX == TY && TY == TZ, "one row length for all axes");
-  if (W < nd) {
+  if (sd.kb) {  // more points than the window is wide, in whole tiles
+    const int o0 = pmod(origin - c, nd);
+    for (int p = 0; p < TX; ++p) {
+      int o = o0 + p;
+      if (o >= nd) o -= nd;
+      if (o > hi) o -= nd;  // largest offset <= hi congruent to P - c
+      double e = 0.0, de = 0.0;
+      if (s < count && o >= lo) kb_weight(o - lo, 2.0 * frac - 1.0, sd.ad, &e, &de);
+      wv[p] = static_cast<R>(e);
+      dv[p] = static_cast<R>(2.0 * static_cast<double>(nd) * de);  // dt/ds_d = 2 n
+    }
+  } else if (W < nd) {
     // Every point has at most one image in [lo, hi]: the offsets of the row are
     // consecutive (one wrap at most) and the eight terms are independent.
     const int o0 = pmod(origin - c, nd);
@@ -240,10 +269,9 @@ __device__ __forceinline__ bool pair_of(const int4& si, int s, const StencilDims
 // and keeps each pair's arrival number in its tile, which saves a launch and the
 // scatter its own round of atomics.
 // ---------------------------------------------------------------------------
-constexpr int kKbCoefs = kKbDegree + 1;
 constexpr int kAxisAtoms = 32;    // atoms per CTA
-constexpr int kAxisRow = 200;     // most values per atom (windows up to m = 12, ad): 52 KB of rows
-__constant__ double c_kb[kKbWidth * kKbCoefs];
+constexpr int kAxisRow = 200;     // most values per atom: 52 KB of rows (half-width 12 with
+                                  // derivatives and a part tile on an axis has up to 240)
 
 // Shared values per atom: the rows (and, for ad, derivative rows) plus padding
 // that spreads the lanes over the banks and keeps rows 16-byte aligned.
@@ -268,13 +296,8 @@ __device__ __forceinline__ int axis_weights(double s, int d, const StencilDims& 
     const double dscale = 2.0 * static_cast<double>(nd);  // dt/ds_d
 #pragma unroll
     for (int j = 0; j < kKbWidth; ++j) {
-      const double* cf = c_kb + j * kKbCoefs;
-      double v = cf[kKbDegree], dv = 0.0;
-#pragma unroll
-      for (int e = kKbDegree - 1; e >= 0; --e) {
-        if (sd.ad) dv = fma(dv, t, v);
-        v = fma(v, t, cf[e]);
-      }
+      double v, dv;
+      kb_weight(j, t, sd.ad, &v, &dv);
       int r = row0 + j;
       if (r >= nd) r -= nd;  // back in the first tile (nt = 2)
       out[r] = v;
