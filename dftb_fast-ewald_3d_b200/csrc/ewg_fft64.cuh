@@ -21,6 +21,7 @@
 // (kClass64), its blocks ordered from the longest line to the shortest.
 #pragma once
 
+#include <atomic>
 #include <initializer_list>
 
 #include "ewg_dft.cuh"
@@ -453,43 +454,67 @@ constexpr int pass64_axis(int pass) {
   return pass == P64_R2C || pass == P64_C2R ? 0 : pass == P64_Z ? 2 : 1;
 }
 
-template <class SH, class K, class... A>
-void go64(K kernel, const Launch64& l, size_t sm, A... args) {
-  if (sm > 48 * 1024)
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
-  launch_chained(kernel, l.blocks, SH::threads, sm, l.st, args...);
+// The largest dynamic shared memory of a pass at length n: one transform's buffer and,
+// in the z pass, the modes, of which a line has fewer than points (K3 < n).
+constexpr int most_smem64(int pass, int n, int elems) {
+  return static_cast<int>(sizeof(cx<double>)) * (elems + (pass == P64_Z ? 8 * n : 0));
+}
+
+// Launches KERNEL with sm <= MOST bytes of dynamic shared memory.  The limit of a kernel
+// is shared by the host threads that use the device, each with its own context: it is
+// set once per device, to the most that any launch takes, and never to one launch's
+// size, which could fall short of another thread's launch.
+template <auto KERNEL, int MOST, class... A>
+void go64(const Launch64& l, int threads, size_t sm, const A&... args) {
+  if constexpr (MOST > 48 * 1024) {
+    static std::atomic<unsigned long long> done{0};  // a bit per device
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (dev > 63 || !(done.load(std::memory_order_acquire) & bit)) {
+      cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST);
+      done.fetch_or(bit, std::memory_order_release);
+    }
+  }
+  launch_chained(KERNEL, l.blocks, threads, sm, l.st, args...);
   ++g_launches;
 }
 
 // A single cell's pass at the length of SH.
+template <class SH, int PASS, int VAR, class... A>
+void go64_one(const Launch64& l, const A&... args) {
+  constexpr int elems = SH::elems(PASS == P64_R2C || PASS == P64_C2R ? 1 : 8);
+  const size_t sm = sizeof(cx<double>) *
+                    (elems + (PASS == P64_Z ? SH::L * static_cast<size_t>(l.K3) : 0));
+  go64<k64_pass<SH, PASS, VAR>, most_smem64(PASS, SH::length, elems)>(l, SH::threads, sm, args...);
+}
+
 template <class SH>
 void launch64(const Launch64& l) {
-  const size_t sm = sizeof(cx<double>) * SH::elems(l.pass == P64_R2C || l.pass == P64_C2R ? 1 : 8);
-  const size_t smz = sm + sizeof(cx<double>) * SH::L * static_cast<size_t>(l.K3);
   switch (l.pass) {
-    case P64_R2C: go64<SH>(k64_pass<SH, P64_R2C, 0>, l, sm, *l.one, 1, l.stress); break;
-    case P64_YFWD: go64<SH>(k64_pass<SH, P64_YFWD, 0>, l, sm, *l.one, 1, l.stress); break;
+    case P64_R2C: go64_one<SH, P64_R2C, 0>(l, *l.one, 1, l.stress); break;
+    case P64_YFWD: go64_one<SH, P64_YFWD, 0>(l, *l.one, 1, l.stress); break;
     case P64_Z:
       if (l.stress)
-        go64<SH>(k64_pass<SH, P64_Z, 1>, l, smz, *l.one, l.nz, l.stress);
+        go64_one<SH, P64_Z, 1>(l, *l.one, l.nz, l.stress);
       else
-        go64<SH>(k64_pass<SH, P64_Z, 0>, l, smz, *l.one, l.nz, l.stress);
+        go64_one<SH, P64_Z, 0>(l, *l.one, l.nz, l.stress);
       break;
-    case P64_YINV: go64<SH>(k64_pass<SH, P64_YINV, 0>, l, sm, *l.one, 1, l.stress); break;
+    case P64_YINV: go64_one<SH, P64_YINV, 0>(l, *l.one, 1, l.stress); break;
     default:
       if (l.nc == 4)
-        go64<SH>(k64_pass<SH, P64_C2R, 4>, l, sm, *l.one, 1, l.stress);
+        go64_one<SH, P64_C2R, 4>(l, *l.one, 1, l.stress);
       else
-        go64<SH>(k64_pass<SH, P64_C2R, 1>, l, sm, *l.one, 1, l.stress);
+        go64_one<SH, P64_C2R, 1>(l, *l.one, 1, l.stress);
   }
 }
 
-// A batch's pass over the cells whose length lies in SHS (all of one class).
-// The same for a batch, whose kernel holds the lengths of a class.
+// The bound of a batch's kernel, which holds the lengths of a class.
 constexpr int min_blocks_seg(int pass, int threads) {
   return pass != P64_Z ? 0 : threads <= 64 ? 14 : threads <= 96 ? 8 : threads <= 128 ? 4 : 2;
 }
 
+// A batch's pass over the cells whose length lies in SHS (all of one class).
 template <int THREADS, int PASS, int VAR, class... SHS>
 __global__ void __launch_bounds__(THREADS, min_blocks_seg(PASS, THREADS)) k64_pass_seg(const BatchCell* __restrict__ cells,
                                                         PassGroup g, int nz) {
@@ -511,10 +536,11 @@ struct Seg64 {
   static constexpr int threads = most({SHS::threads...});
   template <int PASS, int VAR>
   static void go(const Launch64& l) {
-    const int x = PASS == P64_R2C || PASS == P64_C2R ? 1 : 8;
+    constexpr int x = PASS == P64_R2C || PASS == P64_C2R ? 1 : 8;
+    constexpr int bound = most({most_smem64(PASS, SHS::length, SHS::elems(x))...});
     size_t sm = sizeof(cx<double>) * most({(SHS::length <= l.nmax ? SHS::elems(x) : 0)...});
     if (PASS == P64_Z) sm += sizeof(cx<double>) * 8 * static_cast<size_t>(l.K3);
-    go64<Seg64>(k64_pass_seg<threads, PASS, VAR, SHS...>, l, sm, l.cells, l.group, l.nz);
+    go64<k64_pass_seg<threads, PASS, VAR, SHS...>, bound>(l, threads, sm, l.cells, l.group, l.nz);
   }
   static void launch(const Launch64& l) {
     switch (l.pass) {
