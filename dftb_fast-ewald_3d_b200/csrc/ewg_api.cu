@@ -2581,6 +2581,7 @@ int ewg_batch_potential_force_ov(ewg_context* c, int n_cells, const int* offsets
                                  int* cell_status, const ewg_overrides* ov) {
   if (!c || n_cells < 0 || !offsets || !coords || !charges || !lat_rows || !pot) return EWG_ERR_ARG;
   LaunchScope scope(c);
+  cudaGetLastError();  // an earlier call's error of the caller's is not this batch's
   c->uploaded_charges = -1;
   c->resident.coords_version = -1;
   int first = EWG_OK;
@@ -2760,6 +2761,9 @@ int ewg_batch_potential_force_ov(ewg_context* c, int n_cells, const int* offsets
   } else {
     launch_batch();
   }
+  // A launch that was refused leaves stale buffers: no results then.
+  const cudaError_t refused = cudaGetLastError();
+  if (refused != cudaSuccess) return fail(cuda_status(refused));
   std::vector<int> herr(std::max(n_cells, 1), 0);
   cudaError_t e = cudaMemcpyAsync(pot, dpot, sizeof(double) * total, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess && force)
