@@ -1,4 +1,4 @@
-// ewg_fft64.cuh -- the five FP64 transform passes at the lengths of fft64_lengths,
+// ewg_fft64.cuh -- the five FP64 transform passes at the lengths of kLengths64,
 // each a product of two radices of at most 24.
 //
 // What bounds a pass is the traffic of its grids through L2 and HBM and, before
@@ -23,11 +23,59 @@
 
 #include <atomic>
 #include <initializer_list>
+#include <type_traits>
+#include <utility>
 
 #include "ewg_dft.cuh"
 #include "ewg_kernels.h"
 
 namespace ewg {
+
+// The lengths that have these passes, each with its two radices, its class and the
+// source file (a single cell's kernels; they build in parallel) that instantiates it:
+// whole tiles of 8 points, the products of two radices of at most 24 that the grids
+// of either window reach most often.  504 = 24 x 21 and the lengths above 576 are left
+// to the runtime schedule.  The class bounds the registers, threads (64, 96, 128, 192) and shared
+// memory that a batch's launch gives every block.
+struct Length64 {
+  int n, r0, r1, klass, unit;
+};
+constexpr int kUnits64 = 7;
+constexpr Length64 kLengths64[] = {
+    {16, 4, 4, 0, 0},
+    {24, 6, 4, 0, 1},
+    {32, 8, 4, 0, 2},
+    {40, 8, 5, 0, 4},
+    {48, 8, 6, 0, 0},
+    {56, 8, 7, 0, 5},
+    {64, 8, 8, 0, 4},
+    {72, 9, 8, 1, 2},
+    {80, 10, 8, 1, 1},
+    {96, 12, 8, 1, 6},
+    {112, 14, 8, 2, 0},
+    {120, 12, 10, 2, 3},
+    {128, 16, 8, 2, 3},
+    {144, 12, 12, 2, 1},
+    {160, 16, 10, 2, 6},
+    {168, 14, 12, 2, 2},
+    {192, 16, 12, 2, 4},
+    {200, 20, 10, 3, 1},
+    {216, 18, 12, 3, 0},
+    {224, 16, 14, 2, 5},
+    {240, 16, 15, 2, 2},
+    {256, 16, 16, 2, 4},
+    {280, 20, 14, 3, 5},
+    {288, 18, 16, 3, 3},
+    {320, 20, 16, 3, 6},
+    {336, 21, 16, 3, 6},
+    {360, 20, 18, 3, 5},
+    {384, 24, 16, 3, 3},
+    {400, 20, 20, 3, 4},
+    {432, 24, 18, 3, 2},
+    {480, 24, 20, 3, 1},
+    {576, 24, 24, 3, 0},
+};
+constexpr int kCount64 = sizeof(kLengths64) / sizeof(kLengths64[0]);
 
 // LF: lines that are neighbours in the thread index (and in shared memory), 8 for
 // the strided axes, whose memory holds neighbouring lines side by side, 4 or 1 for
@@ -526,6 +574,25 @@ __global__ void __launch_bounds__(THREADS, min_blocks_seg(PASS, THREADS)) k64_pa
   ((n == SHS::length ? pass64_body<SHS, PASS, VAR>(pc, local, nz, nullptr) : void()), ...);
 }
 
+// Launches a single cell's pass if length n belongs to source file U.
+template <int U, int I>
+bool launch64_entry(int n, const Launch64& l) {
+  if constexpr (kLengths64[I].unit == U) {
+    if (n != kLengths64[I].n) return false;
+    launch64<TwoPass<kLengths64[I].n, kLengths64[I].r0, kLengths64[I].r1>>(l);
+    return true;
+  }
+  return false;
+}
+template <int U, int... I>
+bool launch64_unit(int n, const Launch64& l, std::integer_sequence<int, I...>) {
+  return (launch64_entry<U, I>(n, l) || ...);
+}
+template <int U>
+bool launch64_unit(int n, const Launch64& l) {
+  return launch64_unit<U>(n, l, std::make_integer_sequence<int, kCount64>{});
+}
+
 template <class... SHS>
 struct Seg64 {
   static constexpr int most(std::initializer_list<int> v) {
@@ -556,5 +623,26 @@ struct Seg64 {
     }
   }
 };
+
+// The lengths of class K as a Seg64.
+template <class... SHS>
+struct List64 {
+  using Seg = Seg64<SHS...>;
+};
+template <class... A, class... B>
+constexpr List64<A..., B...> operator+(List64<A...>, List64<B...>) {
+  return {};
+}
+template <int K, int I>
+using Entry64 = std::conditional_t<
+    kLengths64[I].klass == K,
+    List64<TwoPass<kLengths64[I].n, kLengths64[I].r0, kLengths64[I].r1>>, List64<>>;
+template <int K, int... I>
+constexpr auto class64(std::integer_sequence<int, I...>) {
+  return (List64<>{} + ... + Entry64<K, I>{});
+}
+template <int K>
+using Class64 =
+    typename decltype(class64<K>(std::make_integer_sequence<int, kCount64>{}))::Seg;
 
 }  // namespace ewg

@@ -3,10 +3,6 @@
 
 namespace ewg {
 
-void launch64_seg1(const Launch64& l) {
-  Seg64<TwoPass<72, 9, 8>,
-        TwoPass<80, 10, 8>,
-        TwoPass<96, 12, 8>>::launch(l);
-}
+void launch64_seg1(const Launch64& l) { Class64<1>::launch(l); }
 
 }  // namespace ewg

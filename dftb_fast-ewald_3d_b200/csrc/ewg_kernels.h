@@ -238,7 +238,7 @@ struct Launch64 {
   double* stress = nullptr;
   cudaStream_t st = nullptr;
 };
-void fft64_launch(int n, const Launch64& l);           // a single cell at length n
+bool fft64_launch(int n, const Launch64& l);           // a single cell; false: no such length
 void fft64_launch_seg(int klass, const Launch64& l);   // a batch's group of a class
 
 // One class's launches of a batch along one axis (two passes along x and y).

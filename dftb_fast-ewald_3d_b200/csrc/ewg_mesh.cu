@@ -613,8 +613,7 @@ bool pass64(const MeshPlan& mp, int pass, int d, const void* grid, const void* A
   l.nc = nc;
   l.stress = stress;
   l.st = st;
-  fft64_launch(mp.g.n[d], l);
-  return true;
+  return fft64_launch(mp.g.n[d], l);
 }
 
 long blocks_of(dim3 g) { return static_cast<long>(g.x) * g.y * g.z; }
