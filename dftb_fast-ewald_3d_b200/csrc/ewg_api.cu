@@ -1001,7 +1001,7 @@ void seg_kernels(ewg_context* c, const SegPlan& sp, const SegBufs& sb, const dou
   prof_mark(prof, st, ST_WEIGHTS);
   launch_weights_bins_seg(b, sb.sort.s4s, sb.wtab, sb.qk, sb.slot, sb.bins, st);
   prof_mark(prof, st, ST_SPREAD);
-  launch_spread_seg(b, sb.bins, sb.slot, sb.wtab, sb.qk, st);
+  launch_spread_seg(b, sb.bins, sb.wtab, sb.qk, st);
   prof_mark(prof, st, ST_FFT_X_R2C);  // the three forward passes together
   launch_forward_and_weight_seg(b, st);
   prof_mark(prof, st, ST_FFT_Y_INV);  // both inverse passes together

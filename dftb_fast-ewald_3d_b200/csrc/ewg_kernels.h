@@ -286,8 +286,8 @@ void launch_real_space_seg(const BatchLaunch& b, const double4* s4s, const float
                            int* cell_err, cudaStream_t st);
 void launch_weights_bins_seg(const BatchLaunch& b, const double4* s4s, void* wtab, void* qk,
                              int4* slot, const PairBins& pb, cudaStream_t st);
-void launch_spread_seg(const BatchLaunch& b, const PairBins& pb, const int4* slot,
-                       const void* wtab, const void* qk, cudaStream_t st);
+void launch_spread_seg(const BatchLaunch& b, const PairBins& pb, const void* wtab, const void* qk,
+                       cudaStream_t st);
 void launch_forward_and_weight_seg(const BatchLaunch& b, cudaStream_t st);
 void launch_inverse_seg(const BatchLaunch& b, cudaStream_t st);
 void launch_gather_seg(const BatchLaunch& b, const int* tile_start, const int2* pairs,

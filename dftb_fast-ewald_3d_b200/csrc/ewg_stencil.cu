@@ -13,8 +13,8 @@
 // then reads an atom's weights for a tile with no index arithmetic.
 //
 // Pairs.  Once per geometry, every (atom, tile) pair is binned by tile, and the
-// spread puts its tile's bucket in atom order (a kernel of its own does so where the
-// lists are long, and for the FP32 CUDA-core spread), so each tile owns an exact,
+// spread puts its tile's bucket in atom order (for the FP32 CUDA-core spread a kernel
+// of its own does so), so each tile owns an exact,
 // deterministic list of the atoms that reach it.  Where the geometry stays for later
 // calls every bucket is also written out in order, whichever spread comes first: a
 // later call takes it as it is, with its own choice of spread.
@@ -462,29 +462,6 @@ __global__ void k_pair_scatter_seg(const BatchCell* __restrict__ cells,
     tmp[starts[tile] + arrival[idx]] = make_int2(k, packed);
 }
 
-// As k_pair_rank, the entry's cell found from its atom (sorted ranges follow
-// the cells' atom ranges).
-__global__ void k_pair_rank_seg(const BatchCell* __restrict__ cells,
-                                const int* __restrict__ atom_prefix, int ncells,
-                                const int2* __restrict__ tmp, const int* __restrict__ starts,
-                                int ntiles, const int4* __restrict__ slot,
-                                int2* __restrict__ pairs) {
-  chain_enter();
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= starts[ntiles]) return;
-  const int2 v = tmp[e];
-  const BatchCell& bc = cells[seg_cell(atom_prefix, ncells, v.x)];
-  const int4 si = slot[v.x];
-  const int tx = (slot_first(si.x) + (v.y & 0xff)) % bc.sd.ntiles[0];
-  const int ty = (slot_first(si.y) + ((v.y >> 8) & 0xff)) % bc.sd.ntiles[1];
-  const int tz = (slot_first(si.z) + (v.y >> 16)) % bc.sd.ntiles[2];
-  const int tile = bc.tile0 + (tz * bc.sd.ntiles[1] + ty) * bc.sd.ntiles[0] + tx;
-  const int b = starts[tile], end = starts[tile + 1];
-  int r = 0;
-  for (int j = b; j < end; ++j) r += tmp[j].x < v.x;
-  pairs[b + r] = v;
-}
-
 __device__ __forceinline__ bool pair_of_thread(const int4* __restrict__ slot, int n,
                                                const StencilDims& sd, int* tile, int* k,
                                                int* packed) {
@@ -513,9 +490,9 @@ __global__ void k_pair_scatter(const int4* __restrict__ slot, int n, StencilDims
         make_int2(k, packed);
 }
 
-// One thread per entry: orders each tile's bucket by atom index (atoms are
-// unique within a bucket) by counting the bucket's entries with a smaller atom.
-// The entry's tile follows from its atom's slot record and its packed slot.
+// For the FP32 CUDA-core spread, one thread per entry: orders each tile's bucket by
+// atom index (atoms are unique within a bucket) by counting the bucket's entries with
+// a smaller atom.  The entry's tile follows from its atom's slot record and its packed slot.
 __global__ void k_pair_rank(const int2* __restrict__ tmp, const int* __restrict__ starts,
                             int ntiles, const int4* __restrict__ slot, StencilDims sd,
                             int2* __restrict__ pairs) {
@@ -680,6 +657,73 @@ __device__ __forceinline__ void stage2(double* dst, const float* src) {
   dst[1] = v.y;
 }
 
+// Puts the list [p0, p1) into pairs in order of its atoms (unique within a tile), a warp
+// to a list: the atoms of a window of kOrderWindow consecutive indices are marked in a
+// bitmap, an entry's place is the number of marks below its own, and the next window
+// starts at the smallest atom left, so a list takes two passes for each window that
+// holds some of it, whatever its length.  (Counting the smaller entries of every entry
+// costs the square of the length: with 5,000 charges in a ball of 0.02 of their cell,
+// lists of some thousand, the spread took 2.2 ms that way and 0.16 so, in the mixed
+// form 14.8 and 0.41.  A launch of its own with a thread per entry took 147 us with the
+// spread at 32,769 atoms of the mixed form and lists of 500, this 93.)
+constexpr int kOrderWords = 512, kOrderWindow = 32 * kOrderWords;
+constexpr int kOrderInts = 2 * (kOrderWords + kOrderWords / 16);  // scratch
+__device__ __forceinline__ void order_list(const int2* __restrict__ unordered, int2* pairs, int p0,
+                                           int p1, int* scratch) {
+  const int lane = threadIdx.x & 31;
+  // Word w of the bitmap and the place of its first mark, at w + w / 16: a lane sums 16
+  // consecutive words without bank conflicts.
+  unsigned* bits = reinterpret_cast<unsigned*>(scratch);
+  int* first = scratch + kOrderInts / 2;
+  int lo = INT_MAX;
+#pragma unroll 4
+  for (int e = p0 + lane; e < p1; e += 32) lo = min(lo, unordered[e].x);
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  int placed = p0;
+  while (lo != INT_MAX) {  // each window starts at an atom past the last one's end
+    for (int w = lane; w < kOrderInts / 2; w += 32) bits[w] = 0;
+    __syncwarp();
+    int next = INT_MAX;
+#pragma unroll 4
+    for (int e = p0 + lane; e < p1; e += 32) {
+      const int id = unordered[e].x, r = id - lo;
+      if (r >= 0 && r < kOrderWindow)
+        atomicOr(&bits[(r >> 5) + (r >> 9)], 1u << (r & 31));
+      else if (r > 0)
+        next = min(next, id);
+    }
+    __syncwarp();
+    int sum = 0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) sum += __popc(bits[17 * lane + j]);
+    int x = sum;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, off);
+      if (lane >= off) x += y;
+    }
+    int run = placed + x - sum;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      first[17 * lane + j] = run;
+      run += __popc(bits[17 * lane + j]);
+    }
+    __syncwarp();
+#pragma unroll 4
+    for (int e = p0 + lane; e < p1; e += 32) {
+      const int2 v = unordered[e];
+      const int r = v.x - lo;
+      if (r >= 0 && r < kOrderWindow) {
+        const int w = (r >> 5) + (r >> 9);
+        pairs[first[w] + __popc(bits[w] & ((1u << (r & 31)) - 1u))] = v;
+      }
+    }
+    placed += __shfl_sync(0xffffffffu, x, 31);
+    lo = __reduce_min_sync(0xffffffffu, next);
+    __syncwarp();
+  }
+}
+
 // One warp per tile owning all eight z-planes, so each step's x and y weights
 // are read from shared memory once for the eight planes.  Bound by the latency of
 // staging the weight rows, so the warps that fit an SM and the sectors per access
@@ -742,14 +786,8 @@ __device__ __forceinline__ void spread_tiles_dmma_body(int tx, int ty, int tz,
       }
     __syncwarp();
   } else if (unordered) {  // a long list goes through its ordered copy
-    for (int e = p0 + lane; e < p1; e += 32) {
-      const int2 v = unordered[e];
-      int place = p0;
-#pragma unroll 8
-      for (int j = p0; j < p1; ++j) place += unordered[j].x < v.x;
-      pairs[place] = v;
-    }
-    __syncwarp();
+    static_assert(sizeof(sW) >= kOrderInts * sizeof(int), "scratch");
+    order_list(unordered, pairs, p0, p1, reinterpret_cast<int*>(&sW[0][0][0]));
   }
   for (int b0 = p0; b0 < p1; b0 += ATOMS) {
     const int nb = min(ATOMS, p1 - b0);
@@ -1609,12 +1647,6 @@ inline int blocks_for(long n, int threads) { return static_cast<int>((n + thread
 namespace {
 size_t axis_smem(int row) { return sizeof(double) * kAxisAtoms * axis_pitch(row); }
 
-// Lists this long on average are ordered by a launch of their own, one thread per
-// entry, instead of by the spread's one warp per tile (both grow with the square
-// of the length; the tolerances in use give lists of 30 to 70).
-constexpr int kOwnRank = 256;
-bool own_rank(size_t npairs, size_t ntiles) { return npairs > kOwnRank * ntiles; }
-
 template <typename R>
 void weights_bins(const MeshPlan& mp, const double4* s4s, int n, R* wtab, R* qk, int4* slot,
                   const PairBins& b, cudaStream_t st) {
@@ -1660,7 +1692,7 @@ void launch_spread(const MeshPlan& mp, const PairBins& b, const int4* slot, int 
   const int* tile_start = b.starts;
   int2* pairs = b.pairs;
   const int2* unordered = ordered ? nullptr : b.unordered;
-  if (n > 0 && !ordered && (cores || own_rank(items, ntiles))) {
+  if (n > 0 && !ordered && cores) {
     launch_chained(k_pair_rank, blocks_for(items, 256), 256, 0, st, unordered, tile_start, ntiles,
                    slot, mp.sd, pairs);
     ++g_launches;
@@ -1811,18 +1843,12 @@ void launch_weights_bins_seg(const BatchLaunch& b, const double4* s4s, void* wta
     weights_bins_seg(b, s4s, static_cast<double*>(wtab), static_cast<double*>(qk), slot, pb, st);
 }
 
-void launch_spread_seg(const BatchLaunch& b, const PairBins& pb, const int4* slot,
-                       const void* wtab, const void* qk, cudaStream_t st) {
+void launch_spread_seg(const BatchLaunch& b, const PairBins& pb, const void* wtab, const void* qk,
+                       cudaStream_t st) {
   if (b.n_tiles == 0) return;
   const int* tile_start = pb.starts;
   int2* pairs = pb.pairs;
   const int2* unordered = pb.unordered;
-  if (b.n_slots > 0 && own_rank(b.n_slots, b.n_tiles)) {
-    launch_chained(k_pair_rank_seg, blocks_for(b.n_slots, 256), 256, 0, st, b.cells, b.p_atoms,
-                   b.ncells, unordered, tile_start, b.n_tiles, slot, pairs);
-    ++g_launches;
-    unordered = nullptr;
-  }
   if (b.mixed)
     launch_chained(k_spread_tiles_dmma_seg<float, kSpreadFew>, b.n_tiles, 32, 0, st, b.cells, b.p_tiles,
                    b.ncells, tile_start, unordered, pairs, static_cast<const float*>(wtab),
