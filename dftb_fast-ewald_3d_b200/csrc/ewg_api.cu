@@ -102,7 +102,7 @@ struct ewg_context {
   cudaEvent_t fork = nullptr, join = nullptr;
   DevBuf buf[B_COUNT];
   std::map<int, FftEntry> ffts;
-  std::map<std::tuple<int, int, int>, CorrEntry> corrs;  // (n, H, half-width or -1)
+  std::map<std::tuple<int, int, int>, CorrEntry> corrs;  // (n, H, half-width or -kb)
   long long launches = 0;
   ewg_params last{};
   // TCoulomb state
@@ -278,14 +278,14 @@ int get_fft(ewg_context* c, int n, FftPlan& out, int sched = 1) {
 // transform at k / n for the Kaiser-Bessel window.
 int get_corr(ewg_context* c, const MeshGeom& g, int d, const double** out) {
   const int n = g.n[d], H = g.M[d] - g.M[d] / 2;
-  auto key = std::make_tuple(n, H, g.kb ? -1 : g.m);
+  auto key = std::make_tuple(n, H, g.kb ? -g.kb : g.m);
   auto it = c->corrs.find(key);
   if (it == c->corrs.end()) {
     std::vector<double> host(2 * H + 1);
     for (int k = -H; k <= H; ++k) {
       double f;
       if (g.kb) {
-        f = 1.0 / kb_transform(static_cast<double>(k) / static_cast<double>(n));
+        f = 1.0 / kb_transform(g.kb, static_cast<double>(k) / static_cast<double>(n));
       } else {
         const double x = kPi * static_cast<double>(k) / static_cast<double>(n);
         f = std::exp(g.b * (x * x));
@@ -382,7 +382,7 @@ ewg_kernel_shape shape_for(const ewg_context* c, const std::array<int, 7>& bucke
 int mesh_geometry(const Cell& cell, const ewg_params& p, bool mixed, MeshGeom& g) {
   for (int d = 0; d < 3; ++d)
     if (p.n_modes[d] < 2) return EWG_ERR_ARG;
-  g.kb = mesh_window(cell, p, mixed) ? 1 : 0;
+  g.kb = mesh_window(cell, p, mixed);
   for (int d = 0; d < 3; ++d) {
     g.M[d] = p.n_modes[d];
     g.n[d] = kOversampling * p.n_modes[d];
@@ -390,7 +390,7 @@ int mesh_geometry(const Cell& cell, const ewg_params& p, bool mixed, MeshGeom& g
     // The mode counts that are accepted do not depend on the window.
     FftPlan twice;
     if (g.n[d] > kMaxFftLength || !factor_length(g.n[d], twice)) return EWG_ERR_GRID_TOO_LARGE;
-    g.n[d] = kb_length(p.n_modes[d]);
+    g.n[d] = kb_length(g.kb, p.n_modes[d], edge_damping(cell, p, d));
   }
   if (p.window_cutoff < 0) return EWG_ERR_ARG;
   // Closed box |k| <= H covering the mode set S = [M/2 - M, M/2 - 1] and -S.

@@ -121,17 +121,29 @@ double window_shape(int m) {
 // The reference's Gaussian at m = 11 or 12 (tolerances of about 1e-9 and 1e-10)
 // spends 23 or 25 points per axis on a twice oversampled grid.  The
 // Kaiser-Bessel window (Kaiser 1974; as an NFFT window: Jackson, Meyer,
-// Nishimura and Macovski 1991; Potts and Steidl 2003) concentrates better: with
-// 14 points on 1.28 points per mode the reciprocal sum of a one-dimensional
-// model with the same mode weights (150 random charges, modes damped to 1e-9 .. 1e-7
-// at the edge of the box as the parameter chain leaves them) is off by
-//   potential   2e-14 .. 7e-14   (Gaussian 1.1e-13 at m = 12, 8e-13 at m = 11)
-//   i k force   4e-14 .. 7e-13   (Gaussian 8e-14, 8e-13)
-//   window-derivative force 7e-12 .. 1e-11   (Gaussian 9e-12, 8e-11)
-// so the results keep the accuracy of the Gaussian's while the grid has 0.26 of
-// its points at best and the stencil 0.18 (m = 12).  beta above pi W (1 - 1/(2 sigma)),
-// the value for unweighted modes, trades error at the edge of the mode box,
-// where the Ewald factor has damped the modes, for error at its centre.
+// Nishimura and Macovski 1991; Potts and Steidl 2003) concentrates better and takes
+// 14 points on some 1.28 to 1.45 points per mode: at best 0.26 of the grid's points and 0.18
+// of the stencil's.
+//
+// Its error has two parts.  One does not depend on the modes: w ends with a jump
+// of 1/I0(beta) that its transform does not know, and the window-derivative force
+// feels it most.  The other is the alias of the modes at the edge of the box,
+// eps = what((n - H)/n) / what(H/n) with H the highest mode, of what the Ewald factor
+// has left of them there.  beta above pi W (1 - 1/(2 sigma)), the value for
+// undamped modes, trades the second for the first.  Against the same sums with a
+// Gaussian of half-width 20 (1,500 charges, skew cell, 10 to 256 modes per axis with
+// all three axes at the same damping of 2e-7 to 1e-11), relative to the Gaussian's own error
+// at the same half-width, which does not depend on the damping:
+//   first part      beta 31, m = 11: potential and i k force 0.06 to 0.13, window-derivative
+//                   force 0.34 to 0.85; beta 33.75, m = 12: 0.04 to 0.1 and 0.3 to 0.65
+//                   (0.94 on 216 points, with which the charges' lattice resonates)
+//   second part     i k force, the most sensitive: at most damping eps times 3e11
+//                   (m = 11), 4.5e12 or, if that is less, 1.8e14 / modes (m = 12);
+//                   window-derivative force at m = 12: 1.1e12
+// (One beta of 32 for both gave the window-derivative force 2.1 times the Gaussian's
+// error at m = 12.)  The grid grows, by a multiple of 8 points at a time, until damping times
+// eps is within kb_alias_limit, and the error is no larger than the Gaussian's in any
+// of them.
 namespace {
 long double bessel_i0(long double x) {  // power series; x <= beta
   const long double h = 0.25L * x * x;
@@ -144,10 +156,10 @@ long double bessel_i0(long double x) {  // power series; x <= beta
 }
 }  // namespace
 
-void kb_polynomials(double* coef) {
+void kb_polynomials(int kb, double* coef) {
   constexpr int N = kKbDegree + 1;
   const long double pi = 3.141592653589793238462643383279502884L;
-  const long double norm = bessel_i0(kKbBeta);
+  const long double beta = kKbBeta[kb - 1], norm = bessel_i0(beta);
   for (int j = 0; j < kKbWidth; ++j) {
     // Chebyshev interpolation of the piece on t in [-1, 1] (error 3e-18 of the
     // window's peak at degree 15), then its monomial coefficients.
@@ -156,7 +168,7 @@ void kb_polynomials(double* coef) {
       const long double t = cosl(pi * (i + 0.5L) / N);
       const long double u = (kKbLow + j) - 0.5L * (t + 1.0L);
       const long double r = 2.0L * u / kKbWidth;
-      f[i] = bessel_i0(kKbBeta * sqrtl(std::max(0.0L, 1.0L - r * r))) / norm;
+      f[i] = bessel_i0(beta * sqrtl(std::max(0.0L, 1.0L - r * r))) / norm;
     }
     for (int k = 0; k < N; ++k) {
       c[k] = 0.0L;
@@ -179,15 +191,37 @@ void kb_polynomials(double* coef) {
   }
 }
 
-double kb_transform(double x) {
+double kb_transform(int kb, double x) {
   // Integral of w(u) exp(-2 pi i u x) du; |pi W x| < beta for every retained
   // mode (|x| <= 1/2.56).
+  const long double beta = kKbBeta[kb - 1];
   const long double y = 3.141592653589793238462643383279502884L * kKbWidth * x;
-  const long double a = sqrtl(static_cast<long double>(kKbBeta) * kKbBeta - y * y);
-  return static_cast<double>(kKbWidth * (sinhl(a) / a) / bessel_i0(kKbBeta));
+  const long double a = sqrtl(beta * beta - y * y);
+  return static_cast<double>(kKbWidth * (sinhl(a) / a) / bessel_i0(beta));
 }
 
-int kb_length(int modes) {
+namespace {
+// what((n - H) / n) / what(H / n): what is W sinh(a) / a / I0(beta), a^2 = beta^2 -
+// (pi W x)^2, or for a^2 < 0 at most its value at a = 0.
+double kb_alias(int kb, int modes, int n) {
+  const double beta = kKbBeta[kb - 1], H = modes - modes / 2;
+  auto root = [&](double x) {
+    const double y = kPi * kKbWidth * x;
+    return std::sqrt(std::max(0.0, beta * beta - y * y));
+  };
+  auto scaled = [](double a) { return a > 1e-6 ? -std::expm1(-2.0 * a) / (2.0 * a) : 1.0; };
+  const double a1 = root((n - H) / n), a0 = root(H / n);
+  return std::exp(a1 - a0) * scaled(a1) / scaled(a0);
+}
+
+// The most of damping times alias: the second part of the error above, below 0.9 of
+// the Gaussian's in the i k force and 0.65 in the window-derivative force.
+double kb_alias_limit(int kb, int modes) {
+  return kb == 1 ? 3.0e-12 : std::min(std::max(1.9e-13, 4.2e-15 * modes), 5.0e-13);
+}
+}  // namespace
+
+int kb_length(int kb, int modes, double damping) {
   // At least 1.28 points per mode and more points than the window is wide (every
   // grid point then meets one image of a stencil), in whole tiles of 8: with a
   // part tile at the end of the axis a stencil would cross four tiles there
@@ -197,23 +231,28 @@ int kb_length(int modes) {
     int r = n;
     for (int p : {2, 3, 5, 7})
       while (r % p == 0) r /= p;
-    if (r == 1) return n;
+    if (r == 1 && (n >= kOversampling * modes ||
+                   damping * kb_alias(kb, modes, n) <= kb_alias_limit(kb, modes)))
+      return n;
   }
 }
 
-bool mesh_window(const Cell& cell, const ewg_params& p, bool mixed) {
-  // Only where the Gaussian is as accurate as the Kaiser-Bessel window: half-widths
-  // 11 and 12 in the plain form.  Narrower Gaussians are the caller's choice of a
-  // looser result, wider ones of a tighter one, and the mixed form's FP32 weights
+double edge_damping(const Cell& cell, const ewg_params& p, int d) {
+  const double edge = kPi * p.n_modes[d] / cell.latLen[d];
+  return std::exp(-edge * edge / (4.0 * p.alpha * p.alpha));
+}
+
+int mesh_window(const Cell& cell, const ewg_params& p, bool mixed) {
+  // Half-widths 11 and 12 in the plain form.  Narrower Gaussians are the caller's choice
+  // of a looser result, wider ones of a tighter one, and the mixed form's FP32 weights
   // keep their values.  The modes at the edge of the box must be damped to
   // 2e-7 (the chain leaves 1e-10 .. 1e-7): overrides of alpha, k_cut or the modes
-  // that leave them undamped keep the Gaussian, whose error there is smaller.
-  if (mixed || p.window_cutoff < 11 || p.window_cutoff > 12) return false;
-  for (int d = 0; d < 3; ++d) {
-    const double edge = kPi * p.n_modes[d] / cell.latLen[d];
-    if (!(std::exp(-edge * edge / (4.0 * p.alpha * p.alpha)) <= 2.0e-7)) return false;
-  }
-  return true;
+  // that leave them undamped keep the Gaussian, whose error there is smaller than on any
+  // smaller grid.
+  if (mixed || p.window_cutoff < 11 || p.window_cutoff > 12) return 0;
+  for (int d = 0; d < 3; ++d)
+    if (!(edge_damping(cell, p, d) <= 2.0e-7)) return 0;
+  return p.window_cutoff - 10;
 }
 
 int box_count(double r_cut, double recLen) { return floor_int(1.0 / (r_cut * recLen)); }

@@ -48,18 +48,23 @@ double window_shape(int m);       // nfft/nfft.f90:82-92
 // The Kaiser-Bessel window that stands in for the reference's Gaussian in the
 // plain form (see mesh_window in ewg_chain.cpp for the rule and the errors):
 // w(u) = I0(beta sqrt(1 - (2u/W)^2)) / I0(beta) on |u| <= W/2, u in grid units,
-// on a fine grid of at least 1.28 points per retained mode instead of two.
+// on a fine grid of at least 1.28 points per retained mode instead of two.  kb: 1 for
+// the Gaussian's half-width 11, 2 for 12, each with its own beta.
 constexpr int kKbWidth = 14;     // W: grid points per axis
 constexpr int kKbDegree = 15;    // polynomial degree of the evaluated window
-constexpr double kKbBeta = 32.0;
+constexpr int kKbKinds = 2;
+constexpr double kKbBeta[kKbKinds] = {31.0, 33.75};
 // w at the W points o = kb_low + j - frac, j = 0..W-1, as polynomials in
 // t = 2 frac - 1: coef[j * (kKbDegree + 1) + k] multiplies t^k.
 constexpr int kKbLow = -(kKbWidth / 2 - 1);
-void kb_polynomials(double* coef);
-double kb_transform(double x);   // Fourier transform of w at x cycles per grid unit
-int kb_length(int modes);        // fine grid length for that many modes
-// True when the Kaiser-Bessel window serves these parameters.
-bool mesh_window(const Cell& cell, const ewg_params& p, bool mixed);
+void kb_polynomials(int kb, double* coef);
+double kb_transform(int kb, double x);  // Fourier transform of w at x cycles per grid unit
+// Fine grid length for that many modes, the outermost damped to `damping`.
+int kb_length(int kb, int modes, double damping);
+// exp(-(k/2 alpha)^2) at the edge of the modes along axis d.
+double edge_damping(const Cell& cell, const ewg_params& p, int d);
+// The window of these parameters: kb, or 0 for the Gaussian.
+int mesh_window(const Cell& cell, const ewg_params& p, bool mixed);
 int box_count(double r_cut, double recLen);  // common/ewald_cell_list.f90:56-73
 
 // Balanced splitting of the direct engine (direct/ewald_direct_3d.f90:319-347).
@@ -98,7 +103,7 @@ struct MeshGeom {
   int M[3];        // retained modes
   int K1, K2, K3;  // compact spectrum extents: M1/2+1, M2+1, M3+1
   int m;           // window half-width of the parameter set
-  int kb;          // 1: Kaiser-Bessel window
+  int kb;          // kind of the Kaiser-Bessel window, 0: Gaussian
   int lo;          // lowest stencil offset from the lowest grid point: -m, or kKbLow
   int W;           // stencil points per axis: 2m+1, or kKbWidth
   double b;        // window shape

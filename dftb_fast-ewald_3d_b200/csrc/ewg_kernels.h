@@ -139,7 +139,7 @@ struct StencilDims {
   int wstride;     // per-atom weight count: sum S_d T_d
   int lo;          // lowest stencil offset from the atom's lowest grid point
   int W;           // stencil points per axis
-  int kb;          // 1: Kaiser-Bessel window
+  int kb;          // kind of the Kaiser-Bessel window, 0: Gaussian
   double b;        // Gaussian window shape
   double pref;     // 1/sqrt(pi b)
   int ad;          // 1: window derivatives stored after the weights (forces by

@@ -108,11 +108,12 @@ __device__ __forceinline__ void stencil_tiles(int c, const StencilDims& sd, int 
 
 // The Kaiser-Bessel weights of the stencil points as polynomials in t = 2 frac - 1.
 constexpr int kKbCoefs = kKbDegree + 1;
-__constant__ double c_kb[kKbWidth * kKbCoefs];
+__constant__ double c_kb[kKbKinds * kKbWidth * kKbCoefs];
 
-// Point j's weight and, with ad, its derivative with respect to t.
-__device__ __forceinline__ void kb_weight(int j, double t, int ad, double* v, double* dv) {
-  const double* cf = c_kb + j * kKbCoefs;
+// Point j's weight under the window of kind kb and, with ad, its derivative with
+// respect to t.
+__device__ __forceinline__ void kb_weight(int kb, int j, double t, int ad, double* v, double* dv) {
+  const double* cf = c_kb + ((kb - 1) * kKbWidth + j) * kKbCoefs;
   double w = cf[kKbDegree], dw = 0.0;
 #pragma unroll
   for (int e = kKbDegree - 1; e >= 0; --e) {
@@ -157,7 +158,7 @@ __device__ __forceinline__ void weights_row(const double4* __restrict__ s4s, int
       if (o >= nd) o -= nd;
       if (o > hi) o -= nd;  // largest offset <= hi congruent to P - c
       double e = 0.0, de = 0.0;
-      if (s < count && o >= lo) kb_weight(o - lo, 2.0 * frac - 1.0, sd.ad, &e, &de);
+      if (s < count && o >= lo) kb_weight(sd.kb, o - lo, 2.0 * frac - 1.0, sd.ad, &e, &de);
       wv[p] = static_cast<R>(e);
       dv[p] = static_cast<R>(2.0 * static_cast<double>(nd) * de);  // dt/ds_d = 2 n
     }
@@ -277,6 +278,24 @@ constexpr int kAxisRow = 200;     // most values per atom: 52 KB of rows (half-w
 // that spreads the lanes over the banks and keeps rows 16-byte aligned.
 __host__ __device__ constexpr int axis_pitch(int row) { return row + 2; }
 
+// The Kaiser-Bessel weights of an axis into the shared row `out` (row0: the first
+// point's place in it).  The kind is fixed at compile time for constant operands.
+template <int KB>
+__device__ __forceinline__ void axis_kaiser_bessel(double frac, int row0, const StencilDims& sd,
+                                                   int nd, double* __restrict__ out) {
+  const double t = 2.0 * frac - 1.0;
+  const double dscale = 2.0 * static_cast<double>(nd);  // dt/ds_d
+#pragma unroll
+  for (int j = 0; j < kKbWidth; ++j) {
+    double v, dv;
+    kb_weight(KB, j, t, sd.ad, &v, &dv);
+    int r = row0 + j;
+    if (r >= nd) r -= nd;  // back in the first tile (nt = 2)
+    out[r] = v;
+    if (sd.ad) out[sd.dwoff + r] = dscale * dv;
+  }
+}
+
 // The weights of an atom with fractional coordinate s along axis d into its shared
 // row w, zeroed before (with sd.ad the derivatives dwoff further on); returns the
 // slot record.
@@ -292,17 +311,11 @@ __device__ __forceinline__ int axis_weights(double s, int d, const StencilDims& 
     int p0 = c + kKbLow;
     if (p0 < 0) p0 += nd;
     const int row0 = p0 - first * kTileX;
-    const double t = 2.0 * frac - 1.0;
-    const double dscale = 2.0 * static_cast<double>(nd);  // dt/ds_d
-#pragma unroll
-    for (int j = 0; j < kKbWidth; ++j) {
-      double v, dv;
-      kb_weight(j, t, sd.ad, &v, &dv);
-      int r = row0 + j;
-      if (r >= nd) r -= nd;  // back in the first tile (nt = 2)
-      out[r] = v;
-      if (sd.ad) out[sd.dwoff + r] = dscale * dv;
-    }
+    static_assert(kKbKinds == 2, "a call per kind");
+    if (sd.kb == 1)
+      axis_kaiser_bessel<1>(frac, row0, sd, nd, out);
+    else
+      axis_kaiser_bessel<2>(frac, row0, sd, nd, out);
   } else {
     // d/ds_d [pref exp(-u^2 / b)] = n_d (2 u / b) pref exp(-u^2 / b) at u = o - frac.
     const double dscale = -2.0 * static_cast<double>(nd) / sd.b;
@@ -1925,8 +1938,11 @@ void launch_gather_final_seg(const BatchLaunch& b, const int4* slot, const int* 
 int stencil_configure_kernels() {
   // The window's polynomials, computed once (0.5 ms) and put on the context's device.
   struct Table {
-    double coef[kKbWidth * kKbCoefs];
-    Table() { kb_polynomials(coef); }
+    double coef[kKbKinds * kKbWidth * kKbCoefs];
+    Table() {
+      for (int kb = 1; kb <= kKbKinds; ++kb)
+        kb_polynomials(kb, coef + (kb - 1) * kKbWidth * kKbCoefs);
+    }
   };
   static const Table t;
   const int rows = static_cast<int>(axis_smem(kAxisRow));
