@@ -282,7 +282,7 @@ int get_corr(ewg_context* c, const MeshGeom& g, int d, const double** out) {
   auto it = c->corrs.find(key);
   if (it == c->corrs.end()) {
     std::vector<double> host(2 * H + 1);
-    for (int k = -H; k <= H; ++k) {
+    for (int k = 0; k <= H; ++k) {
       double f;
       if (g.kb) {
         f = 1.0 / kb_transform(g.kb, static_cast<double>(k) / static_cast<double>(n));
@@ -290,7 +290,7 @@ int get_corr(ewg_context* c, const MeshGeom& g, int d, const double** out) {
         const double x = kPi * static_cast<double>(k) / static_cast<double>(n);
         f = std::exp(g.b * (x * x));
       }
-      host[k + H] = f * f;
+      host[H + k] = host[H - k] = f * f;
     }
     CorrEntry e;
     if (cudaMalloc(&e.dev, sizeof(double) * host.size()) != cudaSuccess) {

@@ -154,25 +154,34 @@ long double bessel_i0(long double x) {  // power series; x <= beta
   }
   return s;
 }
+
+// I0(beta) of a kind, summed once.
+long double bessel_norm(int kb) {
+  static const long double norm[kKbKinds] = {bessel_i0(kKbBeta[0]), bessel_i0(kKbBeta[1])};
+  return norm[kb - 1];
+}
 }  // namespace
 
 void kb_polynomials(int kb, double* coef) {
   constexpr int N = kKbDegree + 1;
   const long double pi = 3.141592653589793238462643383279502884L;
-  const long double beta = kKbBeta[kb - 1], norm = bessel_i0(beta);
+  const long double beta = kKbBeta[kb - 1], norm = bessel_norm(kb);
+  long double cosine[N][N];  // T_k at the Chebyshev nodes
+  for (int k = 0; k < N; ++k)
+    for (int i = 0; i < N; ++i) cosine[k][i] = cosl(pi * k * (i + 0.5L) / N);
   for (int j = 0; j < kKbWidth; ++j) {
     // Chebyshev interpolation of the piece on t in [-1, 1] (error 3e-18 of the
     // window's peak at degree 15), then its monomial coefficients.
     long double f[N], c[N], mono[N] = {0.0L}, t0[N] = {0.0L}, t1[N] = {0.0L};
     for (int i = 0; i < N; ++i) {
-      const long double t = cosl(pi * (i + 0.5L) / N);
+      const long double t = cosine[1][i];
       const long double u = (kKbLow + j) - 0.5L * (t + 1.0L);
       const long double r = 2.0L * u / kKbWidth;
       f[i] = bessel_i0(beta * sqrtl(std::max(0.0L, 1.0L - r * r))) / norm;
     }
     for (int k = 0; k < N; ++k) {
       c[k] = 0.0L;
-      for (int i = 0; i < N; ++i) c[k] += f[i] * cosl(pi * k * (i + 0.5L) / N);
+      for (int i = 0; i < N; ++i) c[k] += f[i] * cosine[k][i];
       c[k] *= (k == 0 ? 1.0L : 2.0L) / N;
     }
     t0[0] = 1.0L;  // T_0
@@ -197,7 +206,7 @@ double kb_transform(int kb, double x) {
   const long double beta = kKbBeta[kb - 1];
   const long double y = 3.141592653589793238462643383279502884L * kKbWidth * x;
   const long double a = sqrtl(beta * beta - y * y);
-  return static_cast<double>(kKbWidth * (sinhl(a) / a) / bessel_i0(beta));
+  return static_cast<double>(kKbWidth * (sinhl(a) / a) / bessel_norm(kb));
 }
 
 namespace {

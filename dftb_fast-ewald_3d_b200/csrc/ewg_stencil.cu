@@ -36,7 +36,9 @@
 #include <cuda_runtime.h>
 
 #include <climits>
+#include <mutex>
 #include <type_traits>
+#include <vector>
 
 #include "ewg_kernels.h"
 
@@ -1936,22 +1938,27 @@ void launch_gather_final_seg(const BatchLaunch& b, const int4* slot, const int* 
 }
 
 int stencil_configure_kernels() {
-  // The window's polynomials, computed once (0.5 ms) and put on the context's device.
-  struct Table {
-    double coef[kKbKinds * kKbWidth * kKbCoefs];
-    Table() {
-      for (int kb = 1; kb <= kKbKinds; ++kb)
-        kb_polynomials(kb, coef + (kb - 1) * kKbWidth * kKbCoefs);
-    }
-  };
-  static const Table t;
   const int rows = static_cast<int>(axis_smem(kAxisRow));
   for (const void* k : {reinterpret_cast<const void*>(k_weights_axis<double>),
                         reinterpret_cast<const void*>(k_weights_axis<float>),
                         reinterpret_cast<const void*>(k_weights_axis_seg<double>),
                         reinterpret_cast<const void*>(k_weights_axis_seg<float>)})
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, rows);
-  return cudaMemcpyToSymbol(c_kb, t.coef, sizeof(t.coef)) == cudaSuccess ? EWG_OK : EWG_ERR_CUDA;
+  // The windows' polynomials, once per device: other contexts' kernels may be reading
+  // them later.
+  static std::mutex lock;
+  static std::vector<bool> done;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return EWG_ERR_CUDA;
+  const std::lock_guard<std::mutex> hold(lock);
+  if (dev < static_cast<int>(done.size()) && done[dev]) return EWG_OK;
+  double coef[kKbKinds * kKbWidth * kKbCoefs];
+  for (int kb = 1; kb <= kKbKinds; ++kb)
+    kb_polynomials(kb, coef + (kb - 1) * kKbWidth * kKbCoefs);
+  if (cudaMemcpyToSymbol(c_kb, coef, sizeof(coef)) != cudaSuccess) return EWG_ERR_CUDA;
+  if (dev >= static_cast<int>(done.size())) done.resize(dev + 1, false);
+  done[dev] = true;
+  return EWG_OK;
 }
 
 int measure_dmma_peak(cudaStream_t st, double* tflops) {
