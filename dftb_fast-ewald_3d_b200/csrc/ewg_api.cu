@@ -330,18 +330,14 @@ void real_geometry(const Cell& cell, double r_cut, int natoms, RealGeom& g, int 
   set_scan_mode(g);
 }
 
-void stencil_dims(const MeshGeom& g, bool ad, StencilDims& sd);
-
 // Warps per tile of the i k gather: 8 of one block of 8 atoms where a tile's list fills
 // most of a round of 64, 4 of two blocks where the lists are short and half the warps
 // would have no atom.  By slots per tile: 64 (32,769 atoms) 156 -> 143 us, 79
 // (216,000 sites) 741 -> 716; 31 (128 small cells) 471 with 4 warps, 505 with 8.
 // The mixed form's rows are widened on their way and its gather stays at 4 (60,000
 // atoms 358 us, 386 with 8).
-int default_gather_warps(int n, const MeshGeom& g, bool mixed) {
+int default_gather_warps(int n, const StencilDims& sd, bool mixed) {
   if (mixed) return 4;
-  StencilDims sd;
-  stencil_dims(g, false, sd);
   long slots = n, tiles = 1;
   for (int d = 0; d < 3; ++d) {
     slots *= sd.S[d];
@@ -350,14 +346,14 @@ int default_gather_warps(int n, const MeshGeom& g, bool mixed) {
   return slots > 48 * tiles ? 8 : 4;
 }
 
-// Kernel shapes: the zero (or out-of-range) fields of s take the defaults.
-ewg_kernel_shape resolve_shape(ewg_kernel_shape s, int gather_warps) {
+// Kernel shapes: the zero (or out-of-range) fields of s take the defaults.  (That of
+// gather_warps depends on the stencil: 0 here.)
+ewg_kernel_shape resolve_shape(ewg_kernel_shape s) {
   if (s.box_div < 1 || s.box_div > 3) s.box_div = 2;
   if (s.fft_lines != 1 && s.fft_lines != 2 && s.fft_lines != 4 && s.fft_lines != 8)
     s.fft_lines = 0;  // the most that fit
   if (s.fft_sched != 2) s.fft_sched = 1;
-  if (s.gather_warps != 2 && s.gather_warps != 4 && s.gather_warps != 8)
-    s.gather_warps = gather_warps;
+  if (s.gather_warps != 2 && s.gather_warps != 4 && s.gather_warps != 8) s.gather_warps = 0;
   if (s.stencil != 2) s.stencil = 1;
   return s;
 }
@@ -371,12 +367,10 @@ std::array<int, 7> shape_bucket(int precision, int grids, int n, const MeshGeom&
   return {precision, grids, oct, g.n[0], g.n[1], g.n[2], g.kb ? -g.m : g.m};
 }
 
-ewg_kernel_shape shape_for(const ewg_context* c, const std::array<int, 7>& bucket, int n,
-                           const MeshGeom& g) {
-  const int warps = default_gather_warps(n, g, c->precision == EWG_PRECISION_MIXED);
-  if (c->shape_pinned) return resolve_shape(c->pinned, warps);
+ewg_kernel_shape shape_for(const ewg_context* c, const std::array<int, 7>& bucket) {
+  if (c->shape_pinned) return resolve_shape(c->pinned);
   auto it = c->shapes.find(bucket);
-  return resolve_shape(it == c->shapes.end() ? ewg_kernel_shape{} : it->second, warps);
+  return resolve_shape(it == c->shapes.end() ? ewg_kernel_shape{} : it->second);
 }
 
 int mesh_geometry(const Cell& cell, const ewg_params& p, bool mixed, MeshGeom& g) {
@@ -475,15 +469,14 @@ int evaluate(ewg_context* c, int n, const double* pos, long sa, long sd, const d
   MeshPlan mp;
   rc = mesh_geometry(cell, p, mixed, mp.g);
   if (rc) return rc;
-  const ewg_kernel_shape ks =
-      shape_for(c, shape_bucket(c->precision, want_force ? (ad ? 2 : 1) : 0, n, mp.g), n, mp.g);
+  ewg_kernel_shape ks =
+      shape_for(c, shape_bucket(c->precision, want_force ? (ad ? 2 : 1) : 0, n, mp.g));
   RealGeom rg;
   real_geometry(cell, p.r_cut, n, rg, ks.box_div);
   mp.mixed = mixed;
   mp.prof = &c->prof;
   mp.lines_cap = ks.fft_lines;
   mp.two_pass = ks.fft_sched != 2;
-  mp.gather_warps = ks.gather_warps;
   mp.stencil = ks.stencil;
   for (int d = 0; d < 3; ++d) {
     if ((rc = get_fft(c, mp.g.n[d], mp.fft[d], ks.fft_sched))) return rc;
@@ -491,6 +484,8 @@ int evaluate(ewg_context* c, int n, const double* pos, long sa, long sd, const d
   }
   if ((rc = mesh_check_lengths(mp.g, mixed))) return rc;
   stencil_dims(mp.g, ad, mp.sd);
+  if (!ks.gather_warps) ks.gather_warps = default_gather_warps(n, mp.sd, mixed);
+  mp.gather_warps = ks.gather_warps;
   const int nboxes = rg.nb[0] * rg.nb[1] * rg.nb[2];
   const int ntiles = mp.sd.ntiles[0] * mp.sd.ntiles[1] * mp.sd.ntiles[2];
   const MeshSizes ms = mesh_sizes(mp.g, mp.sd, mixed, nc, n, nparts);
@@ -1485,10 +1480,14 @@ int tune_shapes(ewg_context* c, int n, const double* dpos, const double* dq, con
     cudaGetLastError();
     return EWG_ERR_CUDA;
   }
-  ewg_kernel_shape best = resolve_shape(
-      ewg_kernel_shape{}, default_gather_warps(n, g, c->precision == EWG_PRECISION_MIXED));
+  ewg_kernel_shape best = resolve_shape(ewg_kernel_shape{});
   double best_ms = 0.0;
   rc = time_shape(c, n, dpos, dq, cell, p, dpot, dforce, shift, best, e0, e1, &best_ms);
+  if (!rc) {
+    StencilDims sd;
+    stencil_dims(g, ad, sd);
+    best.gather_warps = default_gather_warps(n, sd, c->precision == EWG_PRECISION_MIXED);
+  }
   const double ms_default = best_ms;
   auto consider = [&](const ewg_kernel_shape& cand) {
     if (rc) return;
