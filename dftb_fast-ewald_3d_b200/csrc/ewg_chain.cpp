@@ -138,7 +138,7 @@ double window_shape(int m) {
 //                   force 0.34 to 0.85; beta 33.75, m = 12: 0.04 to 0.1 and 0.3 to 0.65
 //                   (0.94 on 216 points, with which the charges' lattice resonates)
 //   second part     i k force, the most sensitive: at most damping eps times 3e11
-//                   (m = 11), 4.5e12 or, if that is less, 1.8e14 / modes (m = 12);
+//                   (m = 11), 4.6e12 at 24 modes falling to 1.2e12 at 150 (m = 12);
 //                   window-derivative force at m = 12: 1.1e12
 // (One beta of 32 for both gave the window-derivative force 2.1 times the Gaussian's
 // error at m = 12.)  The grid grows, by a multiple of 8 points at a time, until damping times
@@ -226,7 +226,7 @@ double kb_alias(int kb, int modes, int n) {
 // The most of damping times alias: the second part of the error above, below 0.9 of
 // the Gaussian's in the i k force and 0.65 in the window-derivative force.
 double kb_alias_limit(int kb, int modes) {
-  return kb == 1 ? 3.0e-12 : std::min(std::max(1.9e-13, 4.2e-15 * modes), 5.0e-13);
+  return kb == 1 ? 3.0e-12 : std::min(1.9e-13 * std::sqrt(std::max(1.0, modes / 24.0)), 5.0e-13);
 }
 }  // namespace
 
