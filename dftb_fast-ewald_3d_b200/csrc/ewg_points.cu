@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(256) k_points_real(
   for (int d = 0; d < 3; ++d) {
     const double u = g.rec[d][0] * x[0] + g.rec[d][1] * x[1] + g.rec[d][2] * x[2];
     st[d] = u - floor(u);
-    bt[d] = min(static_cast<int>(st[d] * g.nb[d]), g.nb[d] - 1);
+    bt[d] = max(0, min(static_cast<int>(st[d] * g.nb[d]), g.nb[d] - 1));  // NaN: the first
   }
   const double wt = tblur ? tblur[t] : 0.0;
   const int sx = 2 * g.R[0] + 1, sy = 2 * g.R[1] + 1;

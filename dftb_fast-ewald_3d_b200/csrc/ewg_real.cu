@@ -50,6 +50,12 @@ __device__ __forceinline__ int floor_div(int a, int n) {
 // sorted atoms themselves.  (They were eight, with two memsets, at 27 us for 4,096
 // atoms.)  Up to kSmallAtoms atoms one CTA does all four steps in shared memory.
 // ---------------------------------------------------------------------------
+// Box of the wrapped coordinate s.  A coordinate that is not a number converts to the lowest
+// int; it goes to the first box, and its NaN through the sums.
+__device__ __forceinline__ int box_index(double s, int nb) {
+  return max(0, min(static_cast<int>(s * nb), nb - 1));
+}
+
 struct PrepArgs {
   double rec[3][3];
   int nb[3];
@@ -65,7 +71,7 @@ __device__ __forceinline__ int atom_box(const double (&x)[3], const PrepArgs& a,
   for (int d = 0; d < 3; ++d) {
     const double t = a.rec[d][0] * x[0] + a.rec[d][1] * x[1] + a.rec[d][2] * x[2];
     s[d] = t - floor(t);
-    bx[d] = min(static_cast<int>(s[d] * a.nb[d]), a.nb[d] - 1);
+    bx[d] = box_index(s[d], a.nb[d]);
   }
   return (bx[2] * a.nb[1] + bx[1]) * a.nb[0] + bx[0];
 }
@@ -504,7 +510,7 @@ __device__ __forceinline__ void for_each_candidate(const float4* __restrict__ x3
   double xi[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    b[d] = min(static_cast<int>(sv[d] * g.nb[d]), g.nb[d] - 1);
+    b[d] = box_index(sv[d], g.nb[d]);
     xi[d] = sv[0] * g.lat[0][d] + sv[1] * g.lat[1][d] + sv[2] * g.lat[2][d];
   }
   for (int dz = -g.R[2]; dz <= g.R[2]; ++dz) {
@@ -589,7 +595,7 @@ __device__ __forceinline__ void for_each_candidate_flat(const float4* __restrict
   double xi[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    b[d] = min(static_cast<int>(sv[d] * g.nb[d]), g.nb[d] - 1);
+    b[d] = box_index(sv[d], g.nb[d]);
     xi[d] = sv[0] * g.lat[0][d] + sv[1] * g.lat[1][d] + sv[2] * g.lat[2][d];
   }
   const int wdy = 2 * g.R[1] + 1;

@@ -77,12 +77,13 @@ __device__ __forceinline__ int slot_first(int packed) { return packed & 0xffff; 
 __device__ __forceinline__ int slot_count(int packed) { return packed >> 16; }
 
 // Mesh stencil origin of a wrapped fractional coordinate: lowest grid point
-// floor(s n) (mod n) and the fraction s n - lowest (nfft/nfft.f90:148-152).
+// floor(s n) (mod n) and the fraction s n - lowest (nfft/nfft.f90:148-152).  A coordinate
+// that is not a number, which converts to the lowest int, goes to point 0.
 __device__ __forceinline__ int lowest_point(double s, int n, double* frac) {
   const double scaled = s * n;
   const int lowest = static_cast<int>(floor(scaled));
   *frac = scaled - static_cast<double>(lowest);
-  return lowest >= n ? lowest - n : lowest;
+  return lowest > 0 && lowest < n ? lowest : 0;
 }
 
 // Tiles the stencil [c + lo, c + lo + W - 1] (mod n) runs through, starting at
