@@ -2580,8 +2580,8 @@ int ewg_batch_potential_force(ewg_context* c, int n_cells, const int* offsets, c
                                       force, cell_status, nullptr);
 }
 
-// Mean real-grid bytes per cell above which a batch runs cell by cell (about
-// half the B200's 126 MB L2).
+// Mean bytes per cell, of a real grid with two points per mode, above which a batch runs
+// cell by cell (about half the B200's 126 MB L2; on the Kaiser-Bessel window's grids some 17 MB).
 constexpr double kSegGridBytes = 64.0 * 1024 * 1024;
 
 int ewg_batch_potential_force_ov(ewg_context* c, int n_cells, const int* offsets,
@@ -2631,8 +2631,8 @@ int ewg_batch_potential_force_ov(ewg_context* c, int n_cells, const int* offsets
     all_ok = all_ok && st == EWG_OK;
   }
   // Segmented launches (one per stage over every cell) unless lanes were asked
-  // for, a cell failed its checks, or the cells are large: when the cells' real
-  // grids average more than kSegGridBytes, one cell alone fills the GPU and its
+  // for, a cell failed its checks, or the cells are large: when the cells' grids
+  // of two points per mode average more than kSegGridBytes, one cell alone fills the GPU and its
   // middle FFT passes run from L2, which interleaving the cells would give up;
   // such a batch runs cell by cell on the context's stream.
   double grid_bytes = 0.0;

@@ -492,8 +492,8 @@ constexpr int min_blocks64(int pass, int threads) {
 }
 
 template <class SH, int PASS, int VAR>
-__global__ void __launch_bounds__(SH::threads, min_blocks64(PASS, SH::threads)) k64_pass(const __grid_constant__ PassCell pc, int nz,
-                                                        double* __restrict__ stress) {
+__global__ void __launch_bounds__(SH::threads, min_blocks64(PASS, SH::threads))
+    k64_pass(const __grid_constant__ PassCell pc, int nz, double* __restrict__ stress) {
   chain_enter();
   pass64_body<SH, PASS, VAR>(pc, blockIdx.x, nz, stress);
 }
@@ -564,8 +564,8 @@ constexpr int min_blocks_seg(int pass, int threads) {
 
 // A batch's pass over the cells whose length lies in SHS (all of one class).
 template <int THREADS, int PASS, int VAR, class... SHS>
-__global__ void __launch_bounds__(THREADS, min_blocks_seg(PASS, THREADS)) k64_pass_seg(const BatchCell* __restrict__ cells,
-                                                        PassGroup g, int nz) {
+__global__ void __launch_bounds__(THREADS, min_blocks_seg(PASS, THREADS))
+    k64_pass_seg(const BatchCell* __restrict__ cells, PassGroup g, int nz) {
   chain_enter();
   const int m = seg_cell(g.prefix, g.n, blockIdx.x);
   const PassCell& pc = cells[g.cell[m]];

@@ -630,36 +630,37 @@ void forward_impl(const MeshPlan& mp, const void* grid, void* A1v, void* A2v, vo
   {  // x, real to complex
     prof_mark(mp.prof, st, ST_FFT_X_R2C);
     if (!pass64<R>(mp, P64_R2C, 0, grid, A1, A2, B2, nullptr, nullptr, nc, nullptr, st)) {
-    const int npairs = n2 * n3 / 2;
-    const int L = plan_lines(mp, n1, cb);
-    const size_t sm = pass_smem(n1, L, cb, 0);
-    const int blocks = (npairs + L - 1) / L;
-    with_lines(L, [&](auto lc) {
-      constexpr int LL = decltype(lc)::value;
-      with_shape<R, LL>(mp.fft[0], [&](auto sh) {
-        launch_chained(k_fft_x_r2c<R, LL, decltype(sh)>, blocks, decltype(sh)::template block<LL>(sm, blocks), sm, st,
-                       static_cast<const R*>(grid), A1, n1, npairs, g.K1, mp.fft[0]);
+      const int npairs = n2 * n3 / 2;
+      const int L = plan_lines(mp, n1, cb);
+      const size_t sm = pass_smem(n1, L, cb, 0);
+      const int blocks = (npairs + L - 1) / L;
+      with_lines(L, [&](auto lc) {
+        constexpr int LL = decltype(lc)::value;
+        with_shape<R, LL>(mp.fft[0], [&](auto sh) {
+          using SH = decltype(sh);
+          launch_chained(k_fft_x_r2c<R, LL, SH>, blocks, SH::template block<LL>(sm, blocks), sm,
+                         st, static_cast<const R*>(grid), A1, n1, npairs, g.K1, mp.fft[0]);
+        });
       });
-    });
-    ++g_launches;
+      ++g_launches;
     }
   }
   {  // y forward
     prof_mark(mp.prof, st, ST_FFT_Y_FWD);
     if (!pass64<R>(mp, P64_YFWD, 1, grid, A1, A2, B2, nullptr, nullptr, nc, nullptr, st)) {
-    const int L = plan_lines(mp, n2, cb);
-    const size_t sm = pass_smem(n2, L, cb, 0);
-    dim3 grd((g.K1 + L - 1) / L, n3);
-    const int H2 = (g.K2 - 1) / 2;
-    with_lines(L, [&](auto lc) {
-      constexpr int LL = decltype(lc)::value;
-      with_shape<R, LL>(mp.fft[1], [&](auto sh) {
-        launch_chained(k_fft_y_fwd<R, LL, decltype(sh)>, grd, decltype(sh)::template block<LL>(sm, blocks_of(grd)), sm, st,
-                       A1, A2, n2,
-                       g.K1, g.K2, H2, mp.fft[1]);
+      const int L = plan_lines(mp, n2, cb);
+      const size_t sm = pass_smem(n2, L, cb, 0);
+      dim3 grd((g.K1 + L - 1) / L, n3);
+      const int H2 = (g.K2 - 1) / 2;
+      with_lines(L, [&](auto lc) {
+        constexpr int LL = decltype(lc)::value;
+        with_shape<R, LL>(mp.fft[1], [&](auto sh) {
+          using SH = decltype(sh);
+          launch_chained(k_fft_y_fwd<R, LL, SH>, grd, SH::template block<LL>(sm, blocks_of(grd)),
+                         sm, st, A1, A2, n2, g.K1, g.K2, H2, mp.fft[1]);
+        });
       });
-    });
-    ++g_launches;
+      ++g_launches;
     }
   }
   {  // z forward + influence + z inverse
@@ -686,11 +687,13 @@ void forward_impl(const MeshPlan& mp, const void* grid, void* A1v, void* A2v, vo
       with_shape<R, LL>(mp.fft[2], [&](auto sh) {
         using SH = decltype(sh);
         if (stress_part)
-          launch_chained(k_fft_z_influence<R, LL, true, SH>, grd, SH::template block<LL>(sm, blocks_of(grd), 1024), sm, st, A2, B2,
-                         n3, g.K1, g.K2, g.K3, nz, ia, mp.fft[2]);
+          launch_chained(k_fft_z_influence<R, LL, true, SH>, grd,
+                         SH::template block<LL>(sm, blocks_of(grd), 1024), sm, st, A2, B2, n3, g.K1,
+                         g.K2, g.K3, nz, ia, mp.fft[2]);
         else
-          launch_chained(k_fft_z_influence<R, LL, false, SH>, grd, SH::template block<LL>(sm, blocks_of(grd), 1024), sm, st, A2, B2,
-                         n3, g.K1, g.K2, g.K3, nz, ia, mp.fft[2]);
+          launch_chained(k_fft_z_influence<R, LL, false, SH>, grd,
+                         SH::template block<LL>(sm, blocks_of(grd), 1024), sm, st, A2, B2, n3, g.K1,
+                         g.K2, g.K3, nz, ia, mp.fft[2]);
       });
     });
     ++g_launches;
@@ -708,18 +711,19 @@ void inverse_impl(const MeshPlan& mp, const void* B2v, void* B1v, void* out, int
   {
     prof_mark(mp.prof, st, ST_FFT_Y_INV);
     if (!pass64<R>(mp, P64_YINV, 1, nullptr, nullptr, nullptr, B2, B1, out, nc, nullptr, st)) {
-    const int L = plan_lines(mp, n2, cb);
-    const size_t sm = pass_smem(n2, L, cb, 0);
-    dim3 grd((g.K1 + L - 1) / L, n3, nc == 4 ? 3 : 1);
-    const int H2 = (g.K2 - 1) / 2;
-    with_lines(L, [&](auto lc) {
-      constexpr int LL = decltype(lc)::value;
-      with_shape<R, LL>(mp.fft[1], [&](auto sh) {
-        launch_chained(k_fft_y_inv<R, LL, decltype(sh)>, grd, decltype(sh)::template block<LL>(sm, blocks_of(grd)), sm, st, B2, B1, n2,
-                       n3, g.K1, g.K2, H2, mp.fft[1]);
+      const int L = plan_lines(mp, n2, cb);
+      const size_t sm = pass_smem(n2, L, cb, 0);
+      dim3 grd((g.K1 + L - 1) / L, n3, nc == 4 ? 3 : 1);
+      const int H2 = (g.K2 - 1) / 2;
+      with_lines(L, [&](auto lc) {
+        constexpr int LL = decltype(lc)::value;
+        with_shape<R, LL>(mp.fft[1], [&](auto sh) {
+          using SH = decltype(sh);
+          launch_chained(k_fft_y_inv<R, LL, SH>, grd, SH::template block<LL>(sm, blocks_of(grd)),
+                         sm, st, B2, B1, n2, n3, g.K1, g.K2, H2, mp.fft[1]);
+        });
       });
-    });
-    ++g_launches;
+      ++g_launches;
     }
   }
   {
@@ -736,8 +740,10 @@ void inverse_impl(const MeshPlan& mp, const void* B2v, void* B1v, void* out, int
         constexpr int LL = decltype(lc)::value;
         if constexpr (LL >= 4)
           with_shape<R, LL>(mp.fft[0], [&](auto sh) {
-            launch_chained(k_fft_x_c2r<R, LL, 4, decltype(sh)>, grd, decltype(sh)::template block<LL>(sm, blocks_of(grd)), sm, st, B1,
-                           o, n1, nrows, g.K1, nc, mp.fft[0]);
+            using SH = decltype(sh);
+            launch_chained(k_fft_x_c2r<R, LL, 4, SH>, grd,
+                           SH::template block<LL>(sm, blocks_of(grd)), sm, st, B1, o, n1, nrows,
+                           g.K1, nc, mp.fft[0]);
           });
       });
     } else {  // one component per CTA row (grid.y = component)
@@ -745,8 +751,10 @@ void inverse_impl(const MeshPlan& mp, const void* B2v, void* B1v, void* out, int
       with_lines(L, [&](auto lc) {
         constexpr int LL = decltype(lc)::value;
         with_shape<R, LL>(mp.fft[0], [&](auto sh) {
-          launch_chained(k_fft_x_c2r<R, LL, 1, decltype(sh)>, grd, decltype(sh)::template block<LL>(sm, blocks_of(grd)), sm, st, B1, o,
-                         n1, nrows, g.K1, nc, mp.fft[0]);
+          using SH = decltype(sh);
+          launch_chained(k_fft_x_c2r<R, LL, 1, SH>, grd,
+                         SH::template block<LL>(sm, blocks_of(grd)), sm, st, B1, o, n1, nrows, g.K1,
+                         nc, mp.fft[0]);
         });
       });
     }

@@ -1866,12 +1866,12 @@ void launch_spread_seg(const BatchLaunch& b, const PairBins& pb, const void* wta
   int2* pairs = pb.pairs;
   const int2* unordered = pb.unordered;
   if (b.mixed)
-    launch_chained(k_spread_tiles_dmma_seg<float, kSpreadFew>, b.n_tiles, 32, 0, st, b.cells, b.p_tiles,
-                   b.ncells, tile_start, unordered, pairs, static_cast<const float*>(wtab),
+    launch_chained(k_spread_tiles_dmma_seg<float, kSpreadFew>, b.n_tiles, 32, 0, st, b.cells,
+                   b.p_tiles, b.ncells, tile_start, unordered, pairs, static_cast<const float*>(wtab),
                    static_cast<const float*>(qk));
   else
-    launch_chained(k_spread_tiles_dmma_seg<double, kSpreadFew>, b.n_tiles, 32, 0, st, b.cells, b.p_tiles,
-                   b.ncells, tile_start, unordered, pairs, static_cast<const double*>(wtab),
+    launch_chained(k_spread_tiles_dmma_seg<double, kSpreadFew>, b.n_tiles, 32, 0, st, b.cells,
+                   b.p_tiles, b.ncells, tile_start, unordered, pairs, static_cast<const double*>(wtab),
                    static_cast<const double*>(qk));
   ++g_launches;
 }

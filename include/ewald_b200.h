@@ -243,9 +243,9 @@ typedef struct {
                        whose buffers fit the CTA's shared-memory budget).  The
                        FP64 passes of two register radices have 8 */
   int fft_sched;    /* FFT radix schedule: 1 odd radices, then radix 8 (default);
-                       2 odd radices, then radix 4 in place of 8.  With 1 the
-                       FP64 lengths that are a product of two radices of at
-                       most 24 (whole tiles of 8) take passes of their own */
+                       2 odd radices, then radix 4 in place of 8.  With 1, 32
+                       FP64 lengths from 16 to 576 (whole tiles of 8, products of
+                       two radices of at most 24) take passes of their own */
   int gather_warps; /* FP64-contraction i k gather: warps per tile, 2, 4 or 8,
                        each with 64 / (8 warps) blocks of 8 atoms per round
                        (default: 8 in the plain form where the tiles'
