@@ -384,8 +384,8 @@ int mesh_geometry(const Cell& cell, const ewg_params& p, bool mixed, MeshGeom& g
     // The mode counts that are accepted do not depend on the window.
     FftPlan twice;
     if (g.n[d] > kMaxFftLength || !factor_length(g.n[d], twice)) return EWG_ERR_GRID_TOO_LARGE;
-    g.n[d] = kb_length(g.kb, p.n_modes[d], edge_damping(cell, p, d));
   }
+  if (g.kb) kb_lengths(g.kb, cell, p, g.n);
   if (p.window_cutoff < 0) return EWG_ERR_ARG;
   // Closed box |k| <= H covering the mode set S = [M/2 - M, M/2 - 1] and -S.
   int H[3];

@@ -141,9 +141,8 @@ double window_shape(int m) {
 //                   (m = 11), 4.6e12 at 24 modes falling to 1.2e12 at 150 (m = 12);
 //                   window-derivative force at m = 12: 1.1e12
 // (One beta of 32 for both gave the window-derivative force 2.1 times the Gaussian's
-// error at m = 12.)  The grid grows, by a multiple of 8 points at a time, until damping times
-// eps is within kb_alias_limit, and the error is no larger than the Gaussian's in any
-// of them.
+// error at m = 12.)  The grid grows until damping times eps is small enough (kb_lengths), and
+// the error is no larger than the Gaussian's in any of them.
 namespace {
 long double bessel_i0(long double x) {  // power series; x <= beta
   const long double h = 0.25L * x * x;
@@ -210,45 +209,80 @@ double kb_transform(int kb, double x) {
 }
 
 namespace {
-// what((n - H) / n) / what(H / n): what is W sinh(a) / a / I0(beta), a^2 = beta^2 -
+// ln(what((n - H) / n) / what(H / n)): what is W sinh(a) / a / I0(beta), a^2 = beta^2 -
 // (pi W x)^2, or for a^2 < 0 at most its value at a = 0.
-double kb_alias(int kb, int modes, int n) {
-  const double beta = kKbBeta[kb - 1], H = modes - modes / 2;
-  auto root = [&](double x) {
-    const double y = kPi * kKbWidth * x;
-    return std::sqrt(std::max(0.0, beta * beta - y * y));
-  };
-  auto scaled = [](double a) { return a > 1e-6 ? -std::expm1(-2.0 * a) / (2.0 * a) : 1.0; };
-  const double a1 = root((n - H) / n), a0 = root(H / n);
-  return std::exp(a1 - a0) * scaled(a1) / scaled(a0);
+double kb_log_alias(int kb, int modes, int n) {
+  const double beta = kKbBeta[kb - 1], y = kPi * kKbWidth / n, H = modes - modes / 2;
+  const double y1 = y * (n - H), y0 = y * H;
+  const double a1 = std::sqrt(std::max(0.0, beta * beta - y1 * y1));
+  const double a0 = std::sqrt(beta * beta - y0 * y0);  // y0 < beta, a0 > 10
+  // ln(sinh(a) / a) = a - ln(2 a), exact to 1e-8 at a0; at a1 an upper bound below 10.
+  return a1 - a0 + std::log(a0 / std::max(a1, 0.5));
 }
 
-// The most of damping times alias: the second part of the error above, below 0.9 of
+// ln of the most of damping times alias: the second part of the error above, below 0.9 of
 // the Gaussian's in the i k force and 0.65 in the window-derivative force.
-double kb_alias_limit(int kb, int modes) {
-  return kb == 1 ? 3.0e-12 : std::min(1.9e-13 * std::sqrt(std::max(1.0, modes / 24.0)), 5.0e-13);
+double kb_log_limit(int kb, int modes) {
+  static const double at11 = std::log(3.0e-12), at12 = std::log(1.9e-13), most = std::log(5.0e-13);
+  if (kb == 1) return at11;
+  return modes <= 24 ? at12 : std::min(at12 + 0.5 * std::log(modes / 24.0), most);
 }
 }  // namespace
 
-int kb_length(int kb, int modes, double damping) {
+namespace {
+// The next multiple of 8 with factors up to 7 from 8 i on (a batch asks for some
+// hundred).
+struct SmoothTable {
+  static constexpr int kCount = kMaxFftLength / 8 + 1;
+  short next[kCount] = {};
+};
+constexpr SmoothTable smooth_table() {
+  SmoothTable t{};
+  int from = SmoothTable::kCount - 1;  // 4096 is one
+  for (int i = from; i >= 0; --i) {
+    int r = i > 0 ? i : 11;
+    for (int p = 2; p <= 7; ++p)
+      while (r % p == 0) r /= p;
+    if (r == 1) from = i;
+    t.next[i] = static_cast<short>(8 * from);
+  }
+  return t;
+}
+constexpr SmoothTable kSmooth = smooth_table();
+}  // namespace
+
+void kb_lengths(int kb, const Cell& cell, const ewg_params& p, int n[3]) {
   // At least 1.28 points per mode and more points than the window is wide (every
   // grid point then meets one image of a stencil), in whole tiles of 8: with a
   // part tile at the end of the axis a stencil would cross four tiles there
   // instead of three and every per-atom table would grow by a third per axis.
-  int n = std::max((32 * modes + 24) / 25, kKbWidth + 2);
-  for (n = (n + 7) / 8 * 8;; n += 8) {
-    int r = n;
-    for (int p : {2, 3, 5, 7})
-      while (r % p == 0) r /= p;
-    if (r == 1 && (n >= kOversampling * modes ||
-                   damping * kb_alias(kb, modes, n) <= kb_alias_limit(kb, modes)))
-      return n;
+  // Then the axis whose outermost modes' alias is farthest above its limit grows until the
+  // axes' errors, which add in squares, are within what two axes at their limits would
+  // give (the limits were measured with three axes at the same damping; one axis alone
+  // at 1.7 times its limit gave 1.2 times the Gaussian's error at 50 modes).
+  double over[3];
+  auto weigh = [&](int d) {
+    const int M = p.n_modes[d];
+    over[d] = n[d] < kOversampling * M ? std::exp(2.0 * (kb_log_alias(kb, M, n[d]) -
+                                                         edge_exponent(cell, p, d) -
+                                                         kb_log_limit(kb, M)))
+                                       : 0.0;
+  };
+  for (int d = 0; d < 3; ++d) {
+    const int least = std::max((32 * p.n_modes[d] + 24) / 25, kKbWidth + 2);
+    n[d] = kSmooth.next[(least + 7) / 8];
+    weigh(d);
+  }
+  while (over[0] + over[1] + over[2] > 2.0) {
+    const int d = over[0] >= over[1] ? (over[0] >= over[2] ? 0 : 2) : (over[1] >= over[2] ? 1 : 2);
+    n[d] = kSmooth.next[n[d] / 8 + 1];
+    weigh(d);
   }
 }
 
-double edge_damping(const Cell& cell, const ewg_params& p, int d) {
+double edge_exponent(const Cell& cell, const ewg_params& p, int d) {
   const double edge = kPi * p.n_modes[d] / cell.latLen[d];
-  return std::exp(-edge * edge / (4.0 * p.alpha * p.alpha));
+  return edge * edge / (4.0 * p.alpha * p.alpha);
 }
 
 int mesh_window(const Cell& cell, const ewg_params& p, bool mixed) {
@@ -258,9 +292,10 @@ int mesh_window(const Cell& cell, const ewg_params& p, bool mixed) {
   // 2e-7 (the chain leaves 1e-10 .. 1e-7): overrides of alpha, k_cut or the modes
   // that leave them undamped keep the Gaussian, whose error there is smaller than on any
   // smaller grid.
+  constexpr double kDamped = 15.4249484703983730;  // -ln 2e-7
   if (mixed || p.window_cutoff < 11 || p.window_cutoff > 12) return 0;
   for (int d = 0; d < 3; ++d)
-    if (!(edge_damping(cell, p, d) <= 2.0e-7)) return 0;
+    if (!(edge_exponent(cell, p, d) >= kDamped)) return 0;
   return p.window_cutoff - 10;
 }
 

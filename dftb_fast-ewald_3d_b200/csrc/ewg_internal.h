@@ -59,10 +59,10 @@ constexpr double kKbBeta[kKbKinds] = {31.0, 33.75};
 constexpr int kKbLow = -(kKbWidth / 2 - 1);
 void kb_polynomials(int kb, double* coef);
 double kb_transform(int kb, double x);  // Fourier transform of w at x cycles per grid unit
-// Fine grid length for that many modes, the outermost damped to `damping`.
-int kb_length(int kb, int modes, double damping);
-// exp(-(k/2 alpha)^2) at the edge of the modes along axis d.
-double edge_damping(const Cell& cell, const ewg_params& p, int d);
+// Fine grid lengths for these parameters' modes.
+void kb_lengths(int kb, const Cell& cell, const ewg_params& p, int n[3]);
+// (k / 2 alpha)^2 at the edge of the modes along axis d.
+double edge_exponent(const Cell& cell, const ewg_params& p, int d);
 // The window of these parameters: kb, or 0 for the Gaussian.
 int mesh_window(const Cell& cell, const ewg_params& p, bool mixed);
 int box_count(double r_cut, double recLen);  // common/ewald_cell_list.f90:56-73
@@ -99,7 +99,7 @@ struct FftPlan {
 
 // Everything the mesh kernels need about one evaluation.
 struct MeshGeom {
-  int n[3];        // fine grid: 2 * modes (Gaussian), kb_length(modes) (Kaiser-Bessel)
+  int n[3];        // fine grid: 2 * modes (Gaussian), kb_lengths (Kaiser-Bessel)
   int M[3];        // retained modes
   int K1, K2, K3;  // compact spectrum extents: M1/2+1, M2+1, M3+1
   int m;           // window half-width of the parameter set
