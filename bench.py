@@ -32,6 +32,7 @@ from __future__ import annotations
 import argparse
 import ctypes as C
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -146,9 +147,12 @@ def kaiser_bessel(params, real_bytes):
 
 def fine_grid(params, real_bytes):
     """Fine grid lengths: two points per mode, or for the Kaiser-Bessel window the
-    next multiple of 8 of factors up to 7 from 1.28 per mode."""
+    next multiple of 8 of factors up to 7 from 1.28 per mode, the axis with the largest
+    window error growing until the three axes' are small enough (the library's rule;
+    params["edges"]: the lattice vectors' lengths)."""
+    M = params["n_modes"]
     if not kaiser_bessel(params, real_bytes):
-        return [2 * m for m in params["n_modes"]]
+        return [2 * m for m in M]
 
     def smooth(k):
         for p in (2, 3, 5, 7):
@@ -156,13 +160,29 @@ def fine_grid(params, real_bytes):
                 k //= p
         return k == 1
 
-    out = []
-    for m in params["n_modes"]:
-        k = max(16, (128 * m + 99) // 100)
+    def grid_from(k):
         while k % 8 or not smooth(k):
             k += 1
-        out.append(k)
-    return out
+        return k
+
+    m11 = params["window_cutoff"] == 11
+    beta = 31.0 if m11 else 33.75
+
+    def over(d, k):
+        """Square of (damping times alias of the outermost modes) over its limit."""
+        h, y = M[d] - M[d] // 2, math.pi * 14 / k
+        a1 = math.sqrt(max(0.0, beta * beta - (y * (k - h)) ** 2))
+        a0 = math.sqrt(beta * beta - (y * h) ** 2)
+        alias = a1 - a0 + math.log(a0 / max(a1, 0.5))
+        exponent = (math.pi * M[d] / params["edges"][d] / (2 * params["alpha"])) ** 2
+        limit = 3e-12 if m11 else min(1.9e-13 * math.sqrt(max(1.0, M[d] / 24)), 5e-13)
+        return 0.0 if k >= 2 * M[d] else math.exp(2 * (alias - exponent - math.log(limit)))
+
+    n = [grid_from(max(16, (128 * m + 99) // 100)) for m in M]
+    while sum(over(d, n[d]) for d in range(3)) > 2.0:
+        d = max(range(3), key=lambda i: over(i, n[i]))
+        n[d] = grid_from(n[d] + 1)
+    return n
 
 
 def stage_bytes(params, natoms, real_bytes, nc=4):
@@ -490,7 +510,7 @@ def run_scc(args, eb, torch, device, dist, ws, rank):
         pos, q, lat = workloads.c5_rock_salt_216k()
         charges = [workloads.c5_charge_update(q, k) for k in range(30)]
         label, metric = "c5_rock_salt_216000_scc30", "C5 SCC: shift evals/s at 216,000 sites, fixed geometry, 30 charge updates"
-        grids = "working set (336^3 grids) > L2"
+        grids = "working set (360 x 336 x 336 grids) > L2"
     else:
         pos, q, lat = workloads.c3_water_32k()
         charges = [workloads.charge_update(q, k, seed=3) for k in range(30)]
@@ -661,6 +681,8 @@ def run_ours(args):
     err64_direct = {"potential": rel(p64, pd), "force": rel(f64, fd)}
     params64 = fp64.ctx.last_params()
     params32 = mixed.ctx.last_params()
+    for p in (params64, params32):
+        p["edges"] = [float(np.linalg.norm(a)) for a in lat]
 
     def barrier():
         if dist:
