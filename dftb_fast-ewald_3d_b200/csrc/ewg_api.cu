@@ -2272,7 +2272,7 @@ int points_mesh(ewg_context* c, const Cell& cell, double tol, int nt, const doub
                       st);
   launch_gather(tgt, tpstart, tpairs_d, twt, outg, 1, part, st);
   // Real-space sum over the source cell list.
-  if (!sblur && !tblur) {
+  if (!sblur && !tblur && rg.flat) {
     launch_points_flat(nt, t4s, tperm, dt, s4s, x32, sperm, ds, sbox, rg, p.alpha, r_pair, potsr,
                        want_grad ? gradsr : nullptr, st);
   } else {

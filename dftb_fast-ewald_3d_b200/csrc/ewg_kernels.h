@@ -400,8 +400,8 @@ void launch_points_real(int nt, const double* tc, const double* tblur, int ns, c
                         const int* sperm, const double* sc, const double* sblur,
                         const int* box_start, const PointsReal& g, double* pot, double* grad,
                         cudaStream_t st);
-// The same without blur (targets in box order: t4s, tperm; sources s4s, x32, sperm):
-// pot and, unless null, grad.
+// The same without blur where the neighbourhood is flat (g.flat; targets in box order:
+// t4s, tperm; sources s4s, x32, sperm): pot and, unless null, grad.
 void launch_points_flat(int nt, const double4* t4s, const int* tperm, const double* tc,
                         const double4* s4s, const float4* x32, const int* sperm, const double* sc,
                         const int* box_start, const RealGeom& g, double alpha, double r_cut,
