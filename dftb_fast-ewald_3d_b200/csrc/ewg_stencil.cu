@@ -259,10 +259,10 @@ __device__ __forceinline__ bool pair_of(const int4& si, int s, const StencilDims
 }
 
 // ---------------------------------------------------------------------------
-// Tiled window weights, a warp per axis of 32 atoms, a lane per atom, and the
-// counts of the (atom, tile) pairs.
+// Tiled window weights, a warp per axis of 32 atoms, a lane per atom (or of 8 atoms, four
+// lanes to each), and the counts of the (atom, tile) pairs.
 //
-// A lane evaluates exactly the W points of its stencil: the Kaiser-Bessel
+// The lanes evaluate exactly the W points of their stencils: the Kaiser-Bessel
 // weights as polynomials in the atom's fraction with the same coefficients for
 // every lane, constant operands without a memory access; the Gaussian by its
 // exponential.  (One thread per row of 8 points evaluated 24 or 32 points for 13 to
@@ -273,7 +273,14 @@ __device__ __forceinline__ bool pair_of(const int4& si, int s, const StencilDims
 // and keeps each pair's arrival number in its tile, which saves a launch and the
 // scatter its own round of atomics.
 // ---------------------------------------------------------------------------
-constexpr int kAxisAtoms = 32;    // atoms per CTA
+// Atoms per CTA: 32, or 8 where 32 would leave SMs without a CTA.  Under the Gaussian four
+// lanes then share an atom's points: up to 32 atoms per SM the call is shorter (tolerance
+// 1e-8, half-width 9, us with 8 for 32: 300 atoms 103 for 119, 1,500 132 for 143, 4,500 196
+// for 206; from 9,000 atoms equal, and mixed precision at 32,769 348 for 337).  The
+// Kaiser-Bessel window has a lane per atom in both, and gains where each CTA of 8 has its
+// own SM (300 atoms 97 for 107, 1,500 122 for 121, 4,096 162 for 157).
+constexpr int kAxisMany = 32, kAxisFew = 8;
+constexpr int kAxisFewGaussian = 148 * kAxisMany, kAxisFewBessel = 148 * kAxisFew;
 constexpr int kAxisRow = 200;     // most values per atom: 52 KB of rows (half-width 12 with
                                   // derivatives and a part tile on an axis has up to 240)
 
@@ -301,8 +308,10 @@ __device__ __forceinline__ void axis_kaiser_bessel(double frac, int row0, const 
 
 // The weights of an atom with fractional coordinate s along axis d into its shared
 // row w, zeroed before (with sd.ad the derivatives dwoff further on); returns the
-// slot record.
-__device__ __forceinline__ int axis_weights(double s, int d, const StencilDims& sd,
+// slot record.  SUB lanes (sub: 0 .. SUB - 1) take the atom's points in turn, with the
+// Kaiser-Bessel window and where points are reached twice the first lane all of them.
+template <int SUB>
+__device__ __forceinline__ int axis_weights(double s, int d, int sub, const StencilDims& sd,
                                             double* __restrict__ w) {
   const int nd = sd.n[d], nt = sd.ntiles[d];
   double frac;
@@ -315,6 +324,7 @@ __device__ __forceinline__ int axis_weights(double s, int d, const StencilDims& 
     if (p0 < 0) p0 += nd;
     const int row0 = p0 - first * kTileX;
     static_assert(kKbKinds == 2, "a call per kind");
+    if (sub > 0) return first | (count << 16);
     if (sd.kb == 1)
       axis_kaiser_bessel<1>(frac, row0, sd, nd, out);
     else
@@ -322,9 +332,12 @@ __device__ __forceinline__ int axis_weights(double s, int d, const StencilDims& 
   } else {
     // d/ds_d [pref exp(-u^2 / b)] = n_d (2 u / b) pref exp(-u^2 / b) at u = o - frac.
     const double dscale = -2.0 * static_cast<double>(nd) / sd.b;
-    int o = sd.lo + sd.W - 1;
+    const bool alone = SUB == 1 || sd.W > nd;  // a lane for all points
+    if (alone && sub > 0) return first | (count << 16);
+    const int step = alone ? 1 : SUB;
+    int o = sd.lo + sd.W - 1 - sub;
     int p = pmod(c + o, nd);
-    for (; o >= sd.lo; --o) {
+    for (; o >= sd.lo; o -= step) {
       const double dd = frac - static_cast<double>(o);
       const double e = sd.pref * exp(-(dd * dd) / sd.b);
       const int t = p / kTileX;
@@ -333,7 +346,7 @@ __device__ __forceinline__ int axis_weights(double s, int d, const StencilDims& 
       const int r = sl * kTileX + (p - t * kTileX);
       out[r] += e;  // a point that the stencil reaches again carries the sum
       if (sd.ad) out[sd.dwoff + r] += dscale * dd * e;
-      p = p == 0 ? nd - 1 : p - 1;
+      p = p < step ? p - step + nd : p - step;  // a next point has step < W <= nd, or step 1
     }
   }
   return first | (count << 16);
@@ -353,7 +366,7 @@ __device__ __forceinline__ void copy_row(float* __restrict__ dst, const double* 
 
 // dims(k): the stencil geometry of atom k; pairs0(k): the atom's first place in
 // arrival; tile0(k): its cell's first tile.
-template <typename R, class Dims, class Pairs0, class Tile0>
+template <typename R, int ATOMS, class Dims, class Pairs0, class Tile0>
 __device__ __forceinline__ void weights_axis_body(double* __restrict__ sm, int row, int wstride,
                                                   int pstride, const double4* __restrict__ s4s,
                                                   int n, R* __restrict__ wtab,
@@ -361,17 +374,21 @@ __device__ __forceinline__ void weights_axis_body(double* __restrict__ sm, int r
                                                   int* __restrict__ tile_counts,
                                                   int* __restrict__ arrival, Dims dims,
                                                   Pairs0 pairs0, Tile0 tile0) {
-  __shared__ int sslot[3][kAxisAtoms];
-  const int lane = threadIdx.x & 31, d = threadIdx.x >> 5;
-  const int k0 = blockIdx.x * kAxisAtoms, na = min(kAxisAtoms, n - k0);
+  __shared__ int sslot[3][ATOMS];
+  constexpr int SUB = 32 / ATOMS;
+  const int atom = threadIdx.x % ATOMS, sub = threadIdx.x % 32 / ATOMS, d = threadIdx.x >> 5;
+  const int k0 = blockIdx.x * ATOMS, na = min(ATOMS, n - k0);
   const int pitch = axis_pitch(row);
-  for (int e = threadIdx.x; e < kAxisAtoms * pitch; e += 96) sm[e] = 0.0;
+  for (int e = threadIdx.x; e < ATOMS * pitch; e += 96) sm[e] = 0.0;
   __syncthreads();
-  if (lane < na) {
-    const double4 s4 = s4s[k0 + lane];
-    sslot[d][lane] = axis_weights(d == 0 ? s4.x : (d == 1 ? s4.y : s4.z), d, dims(k0 + lane),
-                                  sm + lane * pitch);
-    if (d == 0) qk[k0 + lane] = static_cast<R>(s4.w);
+  if (atom < na) {
+    const double4 s4 = s4s[k0 + atom];
+    const int record = axis_weights<SUB>(d == 0 ? s4.x : (d == 1 ? s4.y : s4.z), d, sub,
+                                         dims(k0 + atom), sm + atom * pitch);
+    if (sub == 0) {
+      sslot[d][atom] = record;
+      if (d == 0) qk[k0 + atom] = static_cast<R>(s4.w);
+    }
   }
   __syncthreads();
   constexpr int kVec = 16 / sizeof(R);
@@ -393,24 +410,26 @@ __device__ __forceinline__ void weights_axis_body(double* __restrict__ sm, int r
   }
 }
 
-template <typename R>
+template <typename R, int ATOMS>
 __global__ void __launch_bounds__(96) k_weights_axis(const double4* __restrict__ s4s, int n,
-                                                     StencilDims sd, R* __restrict__ wtab,
+                                                     const __grid_constant__ StencilDims sd,
+                                                     R* __restrict__ wtab,
                                                      R* __restrict__ qk, int4* __restrict__ slot,
                                                      int* __restrict__ tile_counts,
                                                      int* __restrict__ arrival) {
   chain_enter();
   extern __shared__ __align__(16) double sm_rows[];
   const int S = sd.S[0] * sd.S[1] * sd.S[2];
-  weights_axis_body(
+  const StencilDims* dims = &sd;  // the parameter itself, no copy per thread
+  weights_axis_body<R, ATOMS>(
       sm_rows, sd.wstride, sd.wstride, S, s4s, n, wtab, qk, slot, tile_counts, arrival,
-      [&](int) -> const StencilDims& { return sd; }, [&](int k) { return static_cast<size_t>(k) * S; },
-      [](int) { return 0; });
+      [dims](int) -> const StencilDims& { return *dims; },
+      [S](int k) { return static_cast<size_t>(k) * S; }, [](int) { return 0; });
 }
 
 // Every cell of a batch (atom_prefix: first atom of each cell, slot_prefix: first
 // (atom, slot) item).
-template <typename R>
+template <typename R, int ATOMS>
 __global__ void __launch_bounds__(96) k_weights_axis_seg(
     const BatchCell* __restrict__ cells, const int* __restrict__ atom_prefix,
     const int* __restrict__ slot_prefix, int ncells, int n, int wstride, int pstride,
@@ -418,12 +437,12 @@ __global__ void __launch_bounds__(96) k_weights_axis_seg(
     int4* __restrict__ slot, int* __restrict__ tile_counts, int* __restrict__ arrival) {
   chain_enter();
   extern __shared__ __align__(16) double sm_rows[];
-  __shared__ int cid[kAxisAtoms];
-  const int k0 = blockIdx.x * kAxisAtoms;
-  if (threadIdx.x < kAxisAtoms)
+  __shared__ int cid[ATOMS];
+  const int k0 = blockIdx.x * ATOMS;
+  if (threadIdx.x < ATOMS)
     cid[threadIdx.x] = seg_cell(atom_prefix, ncells, min(k0 + static_cast<int>(threadIdx.x), n - 1));
   __syncthreads();
-  weights_axis_body(
+  weights_axis_body<R, ATOMS>(
       sm_rows, wstride, wstride, pstride, s4s, n, wtab, qk, slot, tile_counts, arrival,
       [&](int k) -> const StencilDims& { return cells[cid[k - k0]].sd; },
       [&](int k) {
@@ -1661,7 +1680,7 @@ inline int blocks_for(long n, int threads) { return static_cast<int>((n + thread
 }  // namespace
 
 namespace {
-size_t axis_smem(int row) { return sizeof(double) * kAxisAtoms * axis_pitch(row); }
+size_t axis_smem(int row, int atoms) { return sizeof(double) * atoms * axis_pitch(row); }
 
 template <typename R>
 void weights_bins(const MeshPlan& mp, const double4* s4s, int n, R* wtab, R* qk, int4* slot,
@@ -1670,8 +1689,11 @@ void weights_bins(const MeshPlan& mp, const double4* s4s, int n, R* wtab, R* qk,
   const int ntiles = sd.ntiles[0] * sd.ntiles[1] * sd.ntiles[2];
   const long items = static_cast<long>(n) * sd.S[0] * sd.S[1] * sd.S[2];
   if (sd.wstride <= kAxisRow) {
-    launch_chained(k_weights_axis<R>, blocks_for(n, kAxisAtoms), 96, axis_smem(sd.wstride), st, s4s,
-                   n, sd, wtab, qk, slot, b.counts, b.arrival);
+    const bool few = n <= (sd.kb ? kAxisFewBessel : kAxisFewGaussian);
+    const int atoms = few ? kAxisFew : kAxisMany;
+    launch_chained(few ? k_weights_axis<R, kAxisFew> : k_weights_axis<R, kAxisMany>,
+                   blocks_for(n, atoms), 96, axis_smem(sd.wstride, atoms), st, s4s, n, sd, wtab, qk,
+                   slot, b.counts, b.arrival);
     ++g_launches;
   } else {
     const long threads = static_cast<long>(sd.S[0] + sd.S[1] + sd.S[2]) * n;
@@ -1829,9 +1851,12 @@ template <typename R>
 void weights_bins_seg(const BatchLaunch& b, const double4* s4s, R* wtab, R* qk, int4* slot,
                       const PairBins& pb, cudaStream_t st) {
   if (b.wstride <= kAxisRow) {
-    launch_chained(k_weights_axis_seg<R>, blocks_for(b.n_atoms, kAxisAtoms), 96,
-                   axis_smem(b.wstride), st, b.cells, b.p_atoms, b.p_slots, b.ncells, b.n_atoms,
-                   b.wstride, b.pstride, s4s, wtab, qk, slot, pb.counts, pb.arrival);
+    const bool few = b.n_atoms <= (b.mixed ? kAxisFewGaussian : kAxisFewBessel);
+    const int atoms = few ? kAxisFew : kAxisMany;
+    launch_chained(few ? k_weights_axis_seg<R, kAxisFew> : k_weights_axis_seg<R, kAxisMany>,
+                   blocks_for(b.n_atoms, atoms), 96, axis_smem(b.wstride, atoms), st, b.cells,
+                   b.p_atoms, b.p_slots, b.ncells, b.n_atoms, b.wstride, b.pstride, s4s, wtab, qk,
+                   slot, pb.counts, pb.arrival);
     ++g_launches;
   } else {
     launch_chained(k_weights_seg<R>, blocks_for(b.n_weights, 128), 128, 0, st, b.cells,
@@ -1939,11 +1964,12 @@ void launch_gather_final_seg(const BatchLaunch& b, const int4* slot, const int* 
 }
 
 int stencil_configure_kernels() {
-  const int rows = static_cast<int>(axis_smem(kAxisRow));
-  for (const void* k : {reinterpret_cast<const void*>(k_weights_axis<double>),
-                        reinterpret_cast<const void*>(k_weights_axis<float>),
-                        reinterpret_cast<const void*>(k_weights_axis_seg<double>),
-                        reinterpret_cast<const void*>(k_weights_axis_seg<float>)})
+  const int rows = static_cast<int>(axis_smem(kAxisRow, kAxisMany));
+  static_assert(8 * kAxisFew * axis_pitch(kAxisRow) <= 48 * 1024, "needs no larger limit");
+  for (const void* k : {reinterpret_cast<const void*>(k_weights_axis<double, kAxisMany>),
+                        reinterpret_cast<const void*>(k_weights_axis<float, kAxisMany>),
+                        reinterpret_cast<const void*>(k_weights_axis_seg<double, kAxisMany>),
+                        reinterpret_cast<const void*>(k_weights_axis_seg<float, kAxisMany>)})
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, rows);
   // The windows' polynomials, once per device: other contexts' kernels may be reading
   // them later.
